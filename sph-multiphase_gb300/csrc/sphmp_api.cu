@@ -31,6 +31,7 @@ struct sphmp_ctx {
     bool alpha_advanced = false;  // alpha4[cur] = advanced fractions, alpha4[cur^1] = start of step
     bool grid_valid = false;      // cell starts built for the current slot order
     bool nbr_valid = false;       // neighbour list built by the density pass for the current positions
+    bool ii_valid = false;        // the lists hold the IISPH neighbours (fluid, within h) of the current positions
     bool oct_built = false;       // the last grid list also built the next internal order (osrc)
     bool oct_valid = false;       // the internal order is octant-grouped for the current cell list
     bool pos_sorted = false;      // positions unchanged since the cell list was built from them
@@ -145,6 +146,14 @@ sphmp_status validate_params(const sphmp_params* p) {
     return SPHMP_OK;
 }
 
+// The smallest float whose square root, rounded to float, is not below r.
+float sqrt_cut(float r) {
+    float x = r * r;
+    while (sqrtf(x) >= r && x > 0.f) x = nextafterf(x, 0.f);
+    while (sqrtf(x) < r) x = nextafterf(x, INFINITY);
+    return x;
+}
+
 DevParams dev_params(const sphmp_ctx* c) {
     const sphmp_params& p = c->prm;
     DevParams P;
@@ -195,6 +204,16 @@ DevParams dev_params(const sphmp_ctx* c) {
     P.morton = p.cell_order == SPHMP_CELL_ORDER_MORTON;
     P.bwin = p.bucket_window > 0 ? p.bucket_window : (int)kBucketWindow;
     P.heavy = p.heavy_list > 0 ? (uint32_t)p.heavy_list : kHeavyList;
+    const double h = (double)P.h;
+    P.ii_c1 = 2.25 / h;
+    P.ii_k = (double)P.kspline / (h * h);
+    P.ii_ih[0] = (float)(1.0 / h);
+    P.ii_ih[1] = (float)(1.0 / h - (double)P.ii_ih[0]);
+    const double idt2 = 1.0 / ((double)P.dt * (double)P.dt);
+    P.ii_idt2[0] = (float)idt2;
+    P.ii_idt2[1] = (float)(idt2 - (double)P.ii_idt2[0]);
+    P.ii_cut[0] = sqrt_cut(P.h);
+    P.ii_cut[1] = sqrt_cut(2.0f * P.h);
     return P;
 }
 
@@ -211,7 +230,7 @@ void free_buffers(sphmp_ctx* c) {
         for (int b = 0; b < 2; b++) cudaFree(B.f4[f][b]);
     void* ptrs[] = {B.densp, B.accel4, B.drift4, B.velxcor, B.pmod, B.mgcell, B.midsort, B.mgndx, B.mgridoff, B.mgridcnt,
                     B.key, B.octk, B.arank, B.sidx, B.ccount, B.cstart, B.cend, B.corder, B.bsum, B.uchunk, B.big, B.color, B.bornid,
-                    B.mass_raw, B.err, B.red, B.vtmp, B.nbr, B.nbr_cnt, B.nmask, B.btab, B.dctr, B.wq, B.wq_n, B.hq, B.hq_n, B.hctr, B.iis_dii, B.iis_dijpj, B.iis_aii, B.iis_rho_adv, B.iis_pl, B.iis_pl1, B.iis_res, B.nrec, B.opos, B.oidx, B.osrc, B.oct_start,
+                    B.mass_raw, B.err, B.red, B.vtmp, B.nbr, B.nbr_cnt, B.nmask, B.btab, B.dctr, B.wq, B.wq_n, B.hq, B.hq_n, B.hctr, B.iis_dii, B.iis_dijpj, B.iis_aii, B.iis_rho_adv, B.iis_pl, B.iis_dsum, B.iis_pm, B.iis_ctl, B.iis_list, B.nrec, B.opos, B.oidx, B.osrc, B.oct_start,
                     B.act, B.act_n, B.nact, B.frame, c->stage};
     for (void* q : ptrs) cudaFree(q);
     memset(&c->B, 0, sizeof(c->B));
@@ -256,7 +275,7 @@ sphmp_status alloc_buffers(sphmp_ctx* c) {
     CK(dalloc(&B.mass_raw, N));
     CK(dalloc(&B.err, 1));
     CK(dalloc(&B.red, 16));
-    CK(dalloc(&B.vtmp, N));
+    CK(dalloc(&B.vtmp, N + 64));  // also three doubles per block of the IISPH walks (at most N / 64 + 1)
     CK(dalloc(&B.nbr, (size_t)kMaxNbr * N));
     CK(dalloc(&B.nbr_cnt, N));
     CK(dalloc(&B.nmask, (size_t)kMaskWords * N));
@@ -274,12 +293,13 @@ sphmp_status alloc_buffers(sphmp_ctx* c) {
     CK(dalloc(&B.iis_aii, N));
     CK(dalloc(&B.iis_rho_adv, N));
     CK(dalloc(&B.iis_pl, N));
-    CK(dalloc(&B.iis_pl1, N));
-    CK(dalloc(&B.iis_res, N));
+    CK(dalloc(&B.iis_dsum, N));
+    CK(dalloc(&B.iis_pm, N));
+    CK(dalloc(&B.iis_ctl, 4));
+    CK(dalloc(&B.iis_list, N));
     CK(cudaMemset(B.iis_dii, 0, sizeof(float4) * N));
     CK(cudaMemset(B.iis_dijpj, 0, sizeof(float4) * N));
     CK(cudaMemset(B.iis_pl, 0, sizeof(float) * N));
-    CK(cudaMemset(B.iis_res, 0, sizeof(float) * N));
     CK(dalloc(&B.nrec, (size_t)kNrecFloat4 * N));
     CK(dalloc(&B.opos, N));
     CK(dalloc(&B.oidx, N));
@@ -380,6 +400,7 @@ void run_density(sphmp_ctx* c, cudaStream_t s) {
     else launch_density(P, c->B, c->cur, s);
     c->list_mode = 1;
     c->nbr_valid = true;
+    c->ii_valid = false;  // one list storage
 }
 
 void run_force_drift(sphmp_ctx* c, bool force, bool drift, cudaStream_t s) {
@@ -448,7 +469,7 @@ sphmp_status enqueue_step(sphmp_ctx* c, int schedule, StageTimer* T = nullptr, c
         c->grid_valid = true;
         c->oct_valid = true;
         c->oct_built = false;
-        c->nbr_valid = false;
+        c->nbr_valid = c->ii_valid = false;
         c->pos_sorted = true;
         run_density(c, s);
         mark("density");
@@ -478,7 +499,7 @@ sphmp_status enqueue_step(sphmp_ctx* c, int schedule, StageTimer* T = nullptr, c
             c->lrows = PL.n;
             mark("correction");
         }
-        c->nbr_valid = false;  // positions moved
+        c->nbr_valid = c->ii_valid = false;  // positions moved
         c->oct_valid = false;
         c->pos_sorted = false;
     } else {
@@ -505,7 +526,7 @@ sphmp_status enqueue_step(sphmp_ctx* c, int schedule, StageTimer* T = nullptr, c
         }
         launch_advance(dev_params(c), c->B, c->cur, s);
         mark("advance");
-        c->nbr_valid = false;
+        c->nbr_valid = c->ii_valid = false;
         c->oct_valid = false;
         c->pos_sorted = false;
     }
@@ -645,7 +666,7 @@ sphmp_status sphmp_set_params(sphmp_ctx* c, const sphmp_params* p) {
     if (sphmp_status st = ensure_cell_order(c)) return st;
     if (grid_changed || order_changed) c->grid_valid = false;
     if (grid_changed || radius_changed || order_changed) {
-        c->nbr_valid = false;
+        c->nbr_valid = c->ii_valid = false;
         c->oct_valid = false;
     }
     drop_graph(c);
@@ -724,7 +745,7 @@ static sphmp_status upload_records(sphmp_ctx* c, const sphmp_display_pack* disp,
     CHECK_LAUNCH("unpack records");
     c->alpha_advanced = false;
     c->grid_valid = false;
-    c->nbr_valid = false;
+    c->nbr_valid = c->ii_valid = false;
     c->oct_valid = false;
     c->oct_built = false;
     c->pos_sorted = false;
@@ -885,7 +906,7 @@ static sphmp_status unpack_field_staged(sphmp_ctx* c, int field, const void* dev
     launch_unpack_field(P, c->B, c->cur, field, a_cur, a_pre, dev, n, c->stream);
     CHECK_LAUNCH("unpack field");
     if (field == SPHMP_F_POS) {
-        c->nbr_valid = false;
+        c->nbr_valid = c->ii_valid = false;
         c->oct_valid = false;
         c->oct_built = false;
         c->pos_sorted = false;
@@ -910,7 +931,7 @@ sphmp_status sphmp_upload_field(sphmp_ctx* c, int32_t field, const void* host, i
         if (n < 0 || (size_t)n > count) return fail(SPHMP_ERR_CAPACITY, "n %d exceeds %zu entries", n, count);
         if (sphmp_status st = check_sort_upload(c, field, host, n)) return st;
         CK(cudaMemcpyAsync(arr, host, sizeof(uint32_t) * (size_t)n, cudaMemcpyHostToDevice, c->stream));
-        c->nbr_valid = false;
+        c->nbr_valid = c->ii_valid = false;
         c->oct_valid = false;
         c->oct_built = false;
         c->pos_sorted = false;
@@ -947,7 +968,7 @@ sphmp_status sphmp_get_particle_index(sphmp_ctx* c) {
     CHECK_LAUNCH("GetParticleIndex");
     c->hash_n = c->n;
     c->grid_valid = false;
-    c->nbr_valid = false;
+    c->nbr_valid = c->ii_valid = false;
     c->oct_valid = false;
     c->oct_built = false;
     return SPHMP_OK;
@@ -974,7 +995,7 @@ sphmp_status sphmp_rearrange_data(sphmp_ctx* c) {
     swap_all(c);
     c->alpha_advanced = false;
     c->grid_valid = true;
-    c->nbr_valid = false;
+    c->nbr_valid = c->ii_valid = false;
     c->oct_valid = c->oct_built;
     c->oct_built = false;
     c->pos_sorted = true;
@@ -986,7 +1007,7 @@ sphmp_status sphmp_compute_boundary_density(sphmp_ctx* c) {
     if (sphmp_status st = need_grid(c)) return st;
     launch_boundary_volume(dev_params(c), c->B, c->cur, c->stream);
     CHECK_LAUNCH("ComputeBoundaryDensity");
-    c->nbr_valid = false;
+    c->nbr_valid = c->ii_valid = false;
     return SPHMP_OK;
 }
 
@@ -1099,7 +1120,7 @@ sphmp_status sphmp_advance(sphmp_ctx* c) {
     if (sphmp_status st = need_ctx(c)) return st;
     launch_advance(dev_params(c), c->B, c->cur, c->stream);
     CHECK_LAUNCH("MfAdvance");
-    c->nbr_valid = false;
+    c->nbr_valid = c->ii_valid = false;
     c->oct_valid = false;
     c->pos_sorted = false;
     return SPHMP_OK;
@@ -1187,19 +1208,62 @@ sphmp_status sphmp_autotune(sphmp_ctx* c, int32_t trial_steps, int32_t allow_reo
 
 // ---- IISPH (fluid_system_host.cu:504-557, kernels in sphmp_iisph.cu) ----
 
+// The IISPH list walks need the lists of the current positions and cells: the
+// density pass writes them with the density, every other caller gets them here.
+static void need_iisph_lists(sphmp_ctx* c) {
+    if (c->ii_valid) return;
+    launch_iisph_lists(dev_params(c), c->B, c->cur, c->stream);
+    c->nbr_valid = false;  // one list storage
+    c->ii_valid = true;
+}
+
 sphmp_status sphmp_iisph_density(sphmp_ctx* c) {
     if (sphmp_status st = need_ctx(c)) return st;
     if (sphmp_status st = need_grid(c)) return st;
     launch_iisph_density(dev_params(c), c->B, c->cur, c->stream);
     CHECK_LAUNCH("ComputeDensityIISPH");
+    c->nbr_valid = false;
+    c->ii_valid = true;
     return SPHMP_OK;
 }
 
 sphmp_status sphmp_iisph_predict_advection(sphmp_ctx* c) {
     if (sphmp_status st = need_ctx(c)) return st;
     if (sphmp_status st = need_grid(c)) return st;
+    need_iisph_lists(c);
     launch_iisph_predict(dev_params(c), c->B, c->cur, c->stream);
     CHECK_LAUNCH("PredictAdvection");
+    return SPHMP_OK;
+}
+
+// Pressure iterations until the mean |residue| is at most tol after min_iter of
+// them (decided on the device: iterations queued behind the last one return at
+// once), at most max_iter; the host waits once for every batch of them, the
+// first of 4, each of the others twice as long up to 32.
+static sphmp_status iisph_solve(sphmp_ctx* c, double tol, int min_iter, int max_iter, int* iters, double* residue) {
+    need_iisph_lists(c);
+    const DevParams P = dev_params(c);
+    launch_iisph_begin(P, c->B, c->cur, c->stream);
+    struct {
+        double red[3];
+        uint32_t ctl[3];
+    } h = {};
+    int queued = 0;
+    for (int batch = tol > 0.0 ? 4 : 32; queued < max_iter; batch = batch < 32 ? 2 * batch : 32) {
+        const int m = batch < max_iter - queued ? batch : max_iter - queued;
+        for (int k = 0; k < m; k++) launch_iisph_iteration(P, c->B, c->cur, tol, min_iter, c->stream);
+        CHECK_LAUNCH("Pressure_DP / Pressure_Iter");
+        queued += m;
+        CK(cudaMemcpyAsync(h.red, c->B.red + 11, sizeof(h.red), cudaMemcpyDeviceToHost, c->stream));
+        CK(cudaMemcpyAsync(h.ctl, c->B.iis_ctl, sizeof(h.ctl), cudaMemcpyDeviceToHost, c->stream));
+        CK(cudaStreamSynchronize(c->stream));
+        if (h.ctl[1]) break;
+    }
+    if (iters) *iters = P.n > 0 ? (int)h.ctl[2] : (0.0 <= tol && min_iter <= max_iter ? (min_iter > 1 ? min_iter : 1) : max_iter);
+    if (residue) {
+        residue[0] = c->n > 0 ? h.red[0] / c->n : 0.0;        // the reference's quantity: sum / pnum
+        residue[1] = h.red[2] > 0 ? h.red[1] / h.red[2] : 0.0;  // mean |residue| over in-grid fluid particles
+    }
     return SPHMP_OK;
 }
 
@@ -1207,16 +1271,7 @@ sphmp_status sphmp_iisph_pressure_iteration(sphmp_ctx* c, double* residue) {
     if (sphmp_status st = need_ctx(c)) return st;
     if (sphmp_status st = need_grid(c)) return st;
     if (sphmp_status st = refresh_n(c)) return st;
-    launch_iisph_iteration(dev_params(c), c->B, c->cur, c->stream);
-    CHECK_LAUNCH("Pressure_DP / Pressure_Iter");
-    double red[3];
-    CK(cudaMemcpyAsync(red, c->B.red + 8, sizeof(red), cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
-    if (residue) {
-        residue[0] = c->n > 0 ? red[0] / c->n : 0.0;      // the reference's quantity: sum / pnum
-        residue[1] = red[2] > 0 ? red[1] / red[2] : 0.0;  // mean |residue| over in-grid fluid particles
-    }
-    return SPHMP_OK;
+    return iisph_solve(c, -1.0, 1, 1, nullptr, residue);
 }
 
 sphmp_status sphmp_iisph_pressure_solve(sphmp_ctx* c, float tol, int32_t min_iter, int32_t max_iter,
@@ -1224,13 +1279,11 @@ sphmp_status sphmp_iisph_pressure_solve(sphmp_ctx* c, float tol, int32_t min_ite
     if (sphmp_status st = need_ctx(c)) return st;
     if (!(tol >= 0.f) || min_iter < 0 || max_iter < 1 || min_iter > max_iter)
         return fail(SPHMP_ERR_INVALID_ARG, "need tol >= 0 and 0 <= min_iter <= max_iter, max_iter >= 1");
+    if (sphmp_status st = need_grid(c)) return st;
+    if (sphmp_status st = refresh_n(c)) return st;
     double r[2] = {0.0, 0.0};
     int it = 0;
-    while (it < max_iter) {
-        if (sphmp_status st = sphmp_iisph_pressure_iteration(c, r)) return st;
-        it++;
-        if (it >= min_iter && r[1] <= (double)tol) break;
-    }
+    if (sphmp_status st = iisph_solve(c, (double)tol, min_iter, max_iter, &it, r)) return st;
     if (iters) *iters = it;
     if (residue) {
         residue[0] = r[0];
@@ -1244,7 +1297,7 @@ sphmp_status sphmp_iisph_integrate(sphmp_ctx* c) {
     if (sphmp_status st = need_grid(c)) return st;
     launch_iisph_integrate(dev_params(c), c->B, c->cur, c->stream);
     CHECK_LAUNCH("IntegrateIISPH");
-    c->nbr_valid = false;
+    c->nbr_valid = c->ii_valid = false;
     c->oct_valid = false;
     c->pos_sorted = false;
     return SPHMP_OK;
@@ -1322,7 +1375,7 @@ sphmp_status sphmp_step(sphmp_ctx* c, int32_t nsteps, int32_t schedule, int32_t 
         // the state a step leaves behind (as enqueue_step sets it)
         c->alpha_advanced = schedule != SPHMP_SCHEDULE_FUSED && c->prm.multiphase;
         c->grid_valid = true;
-        c->nbr_valid = false;
+        c->nbr_valid = c->ii_valid = false;
         c->oct_valid = false;
         c->oct_built = false;
         c->pos_sorted = false;
@@ -1522,7 +1575,7 @@ static sphmp_status clone_state(sphmp_ctx* dst, sphmp_ctx* src) {
     dst->pos_sorted = src->pos_sorted;
     dst->hash_n = src->hash_n;
     dst->list_mode = src->list_mode;
-    dst->nbr_valid = false;
+    dst->nbr_valid = dst->ii_valid = false;
     dst->n_stale = false;
     dst->emit_on = src->emit_on;
     dst->emitter = src->emitter;

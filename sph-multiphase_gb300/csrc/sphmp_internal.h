@@ -97,6 +97,11 @@ struct DevParams {
     int morton;      // 1: cells in Z-order in the sorted arrays (corder), 0: the reference's linear order
     int bwin;        // members per work item of the bucket density pass (8..32)
     uint32_t heavy;  // index lists longer than this are heavy (queued in hq)
+    // IISPH: 2.25 / h, kspline / h^2, 1 / h and 1 / dt^2 in two parts each, and the smallest
+    // floats whose square root is not below h and 2h (the cut-offs on squared distances)
+    double ii_c1, ii_k;
+    float ii_ih[2], ii_idt2[2];
+    float ii_cut[2];
 };
 
 struct DevBuffers {
@@ -128,7 +133,7 @@ struct DevBuffers {
     float* mass_raw;    // [cap] per origin
     uint32_t* err;      // device error word
     double* red;        // [16] FP64 reduction results
-    float* vtmp;        // [cap] scratch (boundary volumes)
+    float* vtmp;        // [cap + 64] scratch (boundary volumes; block sums of the IISPH residue)
     uint32_t* nbr;      // [kMaxNbr * cap] neighbour indices, groups of 4 column-major: entry k of s at ((k / 4) * cap + s) * 4 + k % 4
     uint32_t* nbr_cnt;  // [cap] list of particle s: kMaskList | bucket, index count (<= kMaxNbr) or kRescan
     uint32_t* nmask;    // [kMaskWords * cap] bucket mask lists, column-major: word k of particle s at k * cap + s
@@ -140,15 +145,18 @@ struct DevBuffers {
     uint32_t* hq;       // [cap] heavy particles (internal index), filled by the list expansion
     uint32_t* hq_n;     // [1] entries in hq (cleared by the scan)
     uint32_t* hctr;     // [2] work counters over hq of the force and the alpha pass
-    // IISPH step (sphmp_iisph.cu): d_ii, sum_j d_ij p_j (float4, w unused), a_ii, the
-    // predicted density, the pressure iterates p_l and p_l+1, the density residue
+    // IISPH step (sphmp_iisph.cu): d_ii, sum_j d_ij p_j, d_ii p_l + sum_j d_ij p_j (float4,
+    // w unused), a_ii, the predicted density, the pressure iterate p_l, p_l m / rho^2
     float4* iis_dii;
     float4* iis_dijpj;
+    float4* iis_dsum;
     float* iis_aii;
     float* iis_rho_adv;
     float* iis_pl;
-    float* iis_pl1;
-    float* iis_res;
+    float* iis_pm;
+    uint32_t* iis_ctl;  // [4] finished blocks of the running iteration, 1 when the solve has ended, iterations,
+                        // particles in iis_list
+    uint32_t* iis_list; // [cap] in-grid fluid particles with IISPH lists (any order)
     float4* nrec;       // [kNrecFloat4 * cap] neighbour records of the alpha pass (written by force + drift)
     // Internal order: inside every 2h cell, members grouped by the h-subcell
     // (octant) they occupy, octant index (oy * 2 + oz) * 2 + ox.
@@ -224,12 +232,17 @@ void launch_advance(const DevParams& P, const DevBuffers& B, const int* cur, cud
 // fused alpha + correction + advance: reads cur, writes cur^1 for all five float4 fields
 void launch_pass_c(const DevParams& P, const DevBuffers& B, const int* cur, cudaStream_t s);
 void launch_conservation(const DevParams& P, const DevBuffers& B, const int* cur, cudaStream_t s);
-// IISPH step (sphmp_iisph.cu): density (densp.x = rho), PredictAdvection (veleval,
-// d_ii, rho_adv, p_l = p / 2, a_ii), one pressure iteration (dijpj, p_l1, residue,
-// accel, pressure, then p_l = p_l1; FP64 residue sums in red[8..10]), integration
+// IISPH step (sphmp_iisph.cu): density (densp.x = rho, and the index lists in nbr /
+// nbr_cnt of the fluid neighbours within h, which the next two need; `lists` writes
+// only those), PredictAdvection (veleval, d_ii, rho_adv, p_l = p / 2, a_ii), the start
+// of a solve, one pressure iteration (accel, pressure = the next p_l; FP64 residue
+// sums in red[11..13], iis_ctl[1] set when the solve has ended), integration
 void launch_iisph_density(const DevParams& P, const DevBuffers& B, const int* cur, cudaStream_t s);
+void launch_iisph_lists(const DevParams& P, const DevBuffers& B, const int* cur, cudaStream_t s);
 void launch_iisph_predict(const DevParams& P, const DevBuffers& B, const int* cur, cudaStream_t s);
-void launch_iisph_iteration(const DevParams& P, const DevBuffers& B, const int* cur, cudaStream_t s);
+void launch_iisph_begin(const DevParams& P, const DevBuffers& B, const int* cur, cudaStream_t s);
+void launch_iisph_iteration(const DevParams& P, const DevBuffers& B, const int* cur, double tol, int min_iter,
+                            cudaStream_t s);
 void launch_iisph_integrate(const DevParams& P, const DevBuffers& B, const int* cur, cudaStream_t s);
 // set the device counter of active slots
 void launch_set_count(const DevBuffers& B, int n, cudaStream_t s);
