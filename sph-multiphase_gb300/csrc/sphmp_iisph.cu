@@ -74,13 +74,13 @@ constexpr uint32_t kIiSearch = 0xffffffffu;  // nbr_cnt: the lists overflowed
 constexpr int kScanThreads = 64;  // small blocks: warps with members (fluid) and without spread evenly over the SMs
 constexpr int kScanWarps = kScanThreads / 32;
 
-// The candidates of cell gc: its 27 cells' index ranges and their offsets in
-// the concatenated sequence (roff[27] = its length, returned).
-__device__ __forceinline__ uint32_t ii_ranges(const DevParams& P, const DevBuffers& B, uint32_t gc, unsigned lane,
-                                              uint32_t* rstart, uint32_t* roff) {
+// Up to 27 cells (`cell` of the lanes below 27, kUndef for none) as index ranges:
+// their starts and their offsets in the concatenated sequence go to the warp's
+// shared table (roff[27] = its length, returned).
+__device__ __forceinline__ uint32_t scan_ranges(const DevBuffers& B, uint32_t cell, unsigned lane, uint32_t* rstart,
+                                                uint32_t* roff) {
     uint32_t st = 0, len = 0;
-    if (lane < 27) {
-        const uint32_t cell = gc + (uint32_t)P.neighborid[lane];
+    if (lane < 27 && cell != kUndef) {
         st = __ldg(&B.cstart[cell]);
         len = __ldg(&B.cend[cell]) - st;
     }
@@ -101,15 +101,15 @@ __device__ __forceinline__ uint32_t ii_ranges(const DevParams& P, const DevBuffe
     return T;
 }
 
-// Visits the candidates of the particles s0 .. s0 + 7 that `mine` marks (lane i
-// holds particle s0 + i and its cell): for each of their cells, `cell_fn` with
-// the members in it (a bit mask), 32 candidates at a time, one a lane (j, its
-// position pj; lanes past the end get a far one). Eight particles share a
-// candidate's load and range lookup; particles of one cell follow each other in
-// the sorted arrays, so a warp has one or two cells.
-template <class F>
-__device__ __forceinline__ void ii_scan(const DevParams& P, const DevBuffers& B, const float4* __restrict__ pos4,
-                                        bool mine, uint32_t cell, uint32_t* rstart, uint32_t* roff, F&& chunk) {
+// Visits, with a whole warp, the candidates of the particles its first lanes
+// hold (`mine`; cell: the one each was sorted into): for each of their cells, the
+// cells around it (`around` gets that cell and the lanes whose particle lies in
+// it as a bit mask, and gives every lane below 27 a cell to search or kUndef),
+// `chunk` with that mask and 32 candidates at a time, one a lane (index j, position pj; far
+// away with w = 0 past the end), loaded one chunk ahead.
+template <class A, class F>
+__device__ __forceinline__ void scan_cells(const DevBuffers& B, const float4* __restrict__ pos4, bool mine,
+                                           uint32_t cell, uint32_t* rstart, uint32_t* roff, A&& around, F&& chunk) {
     const unsigned lane = lane_id();
     const float kFar = __int_as_float(0x7f800000);
     unsigned todo = __ballot_sync(0xffffffffu, mine);
@@ -117,11 +117,11 @@ __device__ __forceinline__ void ii_scan(const DevParams& P, const DevBuffers& B,
         const uint32_t gc = __shfl_sync(0xffffffffu, cell, __ffs(todo) - 1);
         const unsigned members = __ballot_sync(0xffffffffu, mine && cell == gc);
         todo &= ~members;
-        const uint32_t T = ii_ranges(P, B, gc, lane, rstart, roff);
+        const uint32_t T = scan_ranges(B, around(gc, members), lane, rstart, roff);
         int r = 0;
-        uint32_t j = 0, jn = 0;
-        float4 pj, pn;
-        auto load = [&](uint32_t e) {  // the candidate e of the sequence, one chunk ahead of its use
+        uint32_t jn = 0;
+        float4 pn;
+        auto load = [&](uint32_t e) {
             pn = make_float4(kFar, kFar, kFar, 0.f);
             if (e < T) {
                 while (roff[r + 1] <= e) r++;
@@ -131,8 +131,8 @@ __device__ __forceinline__ void ii_scan(const DevParams& P, const DevBuffers& B,
         };
         load(lane);
         for (uint32_t base = 0; base < T; base += 32) {
-            j = jn;
-            pj = pn;
+            const uint32_t j = jn;
+            const float4 pj = pn;
             load(base + 32 + lane);
             chunk(members, j, pj);
         }
@@ -187,7 +187,8 @@ __global__ void __launch_bounds__(kScanThreads) k_ii_density(const __grid_consta
         acc[i] = 0.f;
         cf[i] = cb[i] = 0;
     }
-    ii_scan(P, B, pos4, mine, cell, tab[w][0], tab[w][1], [&](unsigned members, uint32_t j, const float4 pj) {
+    scan_cells(B, pos4, mine, cell, tab[w][0], tab[w][1], [&](uint32_t gc, unsigned) { return gc + (uint32_t)P.neighborid[min(lane, 26u)]; },
+               [&](unsigned members, uint32_t j, const float4 pj) {
         const float2 NX = make_float2(-pj.x, -pj.x), NY = make_float2(-pj.y, -pj.y), NZ = make_float2(-pj.z, -pj.z);
         const float cm = fmaxf(pj.w, 0.f), cv = fmaxf(-pj.w, 0.f);  // mass, or boundary volume
         const bool any_b = __any_sync(0xffffffffu, cv > 0.f);
