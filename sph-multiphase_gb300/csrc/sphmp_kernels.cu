@@ -543,56 +543,55 @@ __global__ void __launch_bounds__(kThreads) k_boundary_volume_store(const __grid
 // Density + EOS pressure (MfComputePressureCUDA)
 // ---------------------------------------------------------------------------
 
-// Density + EOS, one warp per octant bucket (the members of one h-subcell).
-// Every member of a bucket has its neighbours within the 27 h-subcells around
-// it: a pair closer than h is at most one subcell apart per axis, up to the
-// rounding of the grid coordinate (a pair that rounding puts two subcells apart
-// is within 1e-4 h of the cutoff, where the kernels and their gradients vanish
-// to below 1e-7 of a typical term). The 27 subcells form 18 contiguous index
-// ranges (per (y, z) row: the x-neighbour bucket in the adjacent cell and the
-// two buckets of the same cell); their concatenation is the bucket's candidate
-// sequence, recorded in btab. A warp takes one window of up to P.bwin (<= 32)
-// members of a bucket (one member per lane, broadcast by shuffles) and the
-// bucket's candidates in blocks of 32 * kBucketChunks held in registers, one
-// per lane and chunk; for each block it walks the window's members, every lane
-// testing its candidates against the member. The neighbour list of a member is
-// the ballot of those tests, one mask word per 32 candidates, without the
-// member itself. The density terms are non-negative; each lane sums at most
-// kBucketChunks of them per block, the lanes are summed pairwise and the blocks
-// with Kahan compensation (in the member's lane), so the relative rounding
-// error of a member's sum stays below (kBucketChunks + 6) * 2^-24. Warps take
-// work items from a shared counter (their costs differ by orders of magnitude):
-// the first window of every bucket, then the further windows of large buckets,
-// which the cell sort queued in wq, so that no bucket serialises on one warp.
+// Density + EOS and the neighbour lists, one warp per octant bucket (the members of
+// one h-subcell). Every member of a bucket has its neighbours within the 27
+// h-subcells around it: a pair closer than h is at most one subcell apart per
+// axis, up to the rounding of the grid coordinate (a pair that rounding puts two
+// subcells apart is within 1e-4 h of the cutoff, where the kernels and their
+// gradients vanish to below 1e-7 of a typical term). The 27 subcells form 18
+// contiguous index ranges (per (y, z) row: the x-neighbour bucket in the adjacent
+// cell and the two buckets of the same cell); their concatenation is the bucket's
+// candidate sequence. A warp takes one window of up to P.bwin (<= 32) members of a
+// bucket and stages the bucket's candidates in shared memory, 256 at a time. The
+// window's n fluid members share the lanes out: 32 / n lanes a member, each
+// testing every 32 / n-th pair of candidates in packed FP32 arithmetic, adding its density terms and appending the hits to a
+// list of its own in shared memory. The lanes' lists of a member are then joined
+// and written as rows of four indices. Bound by shared-memory accesses (78 % of
+// the L1 data pipe) and the issue slots (64 %): about 14 instructions a candidate
+// and lane, none of them across lanes. (The kernel this replaces had the lanes
+// hold the candidates and walked the members, with ballots and selects per 32
+// candidates and a shuffle reduction per member, and left mask words that a
+// second kernel expanded: 174 M warp instructions at 442 K fluid particles
+// against 117 M here; 404 against 338 us at 1.05 M, 33 against 16 us at 4 K.) A lane adds at most 16
+// pairs of terms before they go to its Kahan-compensated sum, and the lanes of a
+// member are added pairwise (a scan). Warps take work items from a shared counter (their
+// costs differ by orders of magnitude): the first window of every bucket, then
+// the further windows of large buckets, which the cell sort queued in wq, so that
+// no bucket serialises on one warp. Members whose lists overflow their kMaxNbr
+// entries get mask lists instead (overflow_masks) or, where the sequence is too
+// long for those, are left to the cell search; they and members with more than
+// P.heavy neighbours are queued in hq for the force and alpha passes.
 // The candidate sequence of bucket (c, q): the 27 h-subcells around it as 18
-// contiguous index ranges, two per (y, z) subcell row (the x-neighbour bucket in
-// the adjacent cell, and both x buckets of the bucket's own cell column). Lane i
-// < 18 computes range i; the warp scans the lengths. Range starts and sequence
-// offsets go to the warp's shared table (offset[18] = length T); lane i < 18
-// returns its range start and offset in st / off.
-__device__ __forceinline__ uint32_t bucket_ranges(const DevParams& P, const DevBuffers& B, uint32_t c, uint32_t q,
-                                                  unsigned lane, uint32_t* rstart, uint32_t* roff, uint32_t& st,
-                                                  uint32_t& off) {
-    const int cx = (int)(c % (uint32_t)P.rx);
-    const int cyz = (int)(c / (uint32_t)P.rx);
-    const int cz = cyz % P.rz, cy = cyz / P.rz;
+// contiguous index ranges, two per (y, z) subcell row r = 0 .. 8 (the x-neighbour
+// bucket in the adjacent cell, and both x buckets of the bucket's own cell
+// column). Lane 2 r + part < 18 computes one range; the warp scans the lengths.
+// rows[r] = {sequence offset of row r, offset of its second range, index minus
+// offset in the first range, in the second}; rows[9].x = the sequence length T,
+// returned. Cells are found relative to c (a neighbour subcell lies 0 or 1 cells
+// away per axis), so nothing is divided.
+__device__ __forceinline__ uint32_t bucket_rows(const DevParams& P, const DevBuffers& B, uint32_t c, uint32_t q,
+                                                unsigned lane, uint4* rows) {
     const int ox = (int)(q & 1u), oz = (int)((q >> 1) & 1u), oy = (int)(q >> 2);
-    uint32_t len = 0;
-    st = 0;
+    uint32_t len = 0, st = 0;
     if (lane < 18) {
         const int r = (int)(lane >> 1), part = (int)(lane & 1u);
-        const int sy = 2 * cy + oy + r / 3 - 1, sz = 2 * cz + oz + r % 3 - 1;
+        const int sy = oy + r / 3 - 1, sz = oz + r % 3 - 1;  // subcell row relative to the cell's first
         const int oyz = ((sy & 1) * 2 + (sz & 1)) * 2;
-        int ccx, xlo, xhi;
-        if ((ox == 0) == (part == 0)) {  // the single x-neighbour bucket in the adjacent cell
-            ccx = ox == 0 ? cx - 1 : cx + 1;
-            xlo = xhi = ox == 0 ? 1 : 0;
-        } else {                         // both x buckets of the bucket's own cell column
-            ccx = cx;
-            xlo = 0;
-            xhi = 1;
-        }
-        const uint32_t cc = (uint32_t)(((sy >> 1) * P.rz + (sz >> 1)) * P.rx + ccx);
+        // the single x-neighbour bucket in the adjacent cell, or both of the bucket's own cell column
+        const bool single = (ox == 0) == (part == 0);
+        const int dx = single ? (ox == 0 ? -1 : 1) : 0;
+        const int xlo = single && ox == 0 ? 1 : 0, xhi = single ? xlo : 1;
+        const uint32_t cc = c + (uint32_t)(((sy >> 1) * P.rz + (sz >> 1)) * P.rx + dx);
         const uint32_t cs = __ldg(&B.cstart[cc]), ce = __ldg(&B.cend[cc]);
         if (cs < ce) {
             st = __ldg(&B.oct_start[(size_t)cc * 8 + oyz + xlo]);
@@ -606,25 +605,16 @@ __device__ __forceinline__ uint32_t bucket_ranges(const DevParams& P, const DevB
         const uint32_t v = __shfl_up_sync(0xffffffffu, inc, d);
         if ((int)lane >= d) inc += v;
     }
-    const uint32_t T = __shfl_sync(0xffffffffu, inc, 31);
-    off = inc - len;
-    if (lane < 18) {
-        rstart[lane] = st;
-        roff[lane] = off;
+    const uint32_t off = inc - len;
+    if (lane <= 18) {
+        uint32_t* d = &rows[lane >> 1].x + (lane & 1u);
+        d[0] = off;
+        d[2] = st - off;
     }
-    if (lane == 18) roff[18] = T;
     __syncwarp();
-    return T;
+    return __shfl_sync(0xffffffffu, inc, 31);
 }
 
-// Index of candidate e of the sequence; r is the caller's range cursor (e must
-// not decrease between calls with the same cursor).
-__device__ __forceinline__ uint32_t seq_index(const uint32_t* rstart, const uint32_t* roff, int& r, uint32_t e) {
-    while (roff[r + 1] <= e) r++;
-    return rstart[r] + (e - roff[r]);
-}
-
-constexpr int kBucketChunks = 8;
 
 __device__ __forceinline__ uint32_t next_bucket(uint32_t* ctr, unsigned lane) {
     uint32_t v = 0;
@@ -632,21 +622,76 @@ __device__ __forceinline__ uint32_t next_bucket(uint32_t* ctr, unsigned lane) {
     return __shfl_sync(0xffffffffu, v, 0);
 }
 
+// The mask lists of the members `over` (a bit mask over the lanes, which hold the
+// members' positions in pm) of window [w0, ...) of bucket bid: bit e of a
+// member's mask stands for candidate e of the bucket's sequence (length T <= 32 *
+// kMaskWords), whose index is e plus the offset of the sequence range holding e
+// (btab). With the packed arithmetic of the density pass, so the same tests.
 template <bool SS1>
-__global__ void __launch_bounds__(kThreads, 4) k_density_bucket(const __grid_constant__ DevParams P,
-                                                                const __grid_constant__ DevBuffers B,
-                                                                const float4* __restrict__ pos4,
-                                                                const float4* __restrict__ alpha4) {
-    constexpr int kWarps = kThreads / 32;
-    __shared__ uint32_t tab[kWarps][2][20];                 // range starts and sequence offsets
+__device__ __noinline__ void overflow_masks(const DevParams& P, const DevBuffers& B, const float4* __restrict__ pos4,
+                                            uint32_t over, const float4 pm, uint32_t w0, uint32_t bid, uint32_t T,
+                                            const uint4* rows) {
     const unsigned lane = lane_id();
-    const int w = threadIdx.x >> 5;
-    uint32_t* rstart = tab[w][0];
-    uint32_t* roff = tab[w][1];
+    uint32_t* __restrict__ bt = B.btab + (size_t)bid * kTabStride;
+    if (lane < 18) {
+        const uint32_t* d = &rows[lane >> 1].x + (lane & 1u);
+        bt[lane] = d[0];
+        bt[20 + lane] = d[2];
+    }
+    if (lane == 18) bt[18] = T;
+    int r = 0;  // the row holding e, which only grows
+    for (uint32_t base = 0; base < T; base += 32u) {
+        const uint32_t e = base + lane;
+        float4 c = make_float4(__int_as_float(0x7f800000), 0.f, 0.f, 0.f);
+        if (e < T) {
+            while (rows[r + 1].x <= e) r++;
+            const uint4 row = rows[r];
+            c = __ldg(&pos4[e + (e < row.y ? row.z : row.w)]);
+        }
+        for (uint32_t om = over; om != 0u; om &= om - 1u) {
+            const int i = __ffs(om) - 1;
+            float dx = __fadd_rn(__shfl_sync(0xffffffffu, pm.x, i), -c.x);
+            float dy = __fadd_rn(__shfl_sync(0xffffffffu, pm.y, i), -c.y);
+            float dz = __fadd_rn(__shfl_sync(0xffffffffu, pm.z, i), -c.z);
+            if (!SS1) {
+                dx = __fmul_rn(dx, P.ss);
+                dy = __fmul_rn(dy, P.ss);
+                dz = __fmul_rn(dz, P.ss);
+            }
+            const float dsq = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx)));
+            const uint32_t t = w0 + (uint32_t)i;
+            const uint32_t b = __ballot_sync(0xffffffffu, dsq < P.r2list && dsq > 0.f);
+            if (lane == 0) B.nmask[(size_t)(base >> 5) * (size_t)P.cap + t] = b;
+        }
+    }
+}
+
+constexpr int kDensThreads = 128;
+constexpr int kDensBlock = 256;  // candidates staged at a time
+constexpr int kDensList = 64;    // hits a lane keeps per block of candidates
+constexpr int kDensRow = kDensList + 4;  // bytes of its row (17 words: the lanes' rows start in different banks)
+
+struct DensityWarp {  // one warp's shared memory
+    float4 pxy[kDensBlock / 2];     // two candidates: {x0, x1, y0, y1}
+    float4 pzw[kDensBlock / 2];     // {z0, z1, w0, w1}
+    uint32_t cidx[kDensBlock];      // their indices
+    uint8_t list[32 * kDensRow];    // the lanes' hits as positions in the block
+    uint4 rows[10];                 // the candidate sequence (bucket_rows)
+};
+
+template <bool SS1>
+__global__ void __launch_bounds__(kDensThreads, 7) k_density_bucket(const __grid_constant__ DevParams P,
+                                                                    const __grid_constant__ DevBuffers B,
+                                                                    const float4* __restrict__ pos4,
+                                                                    const float4* __restrict__ alpha4) {
+    __shared__ DensityWarp shared[kDensThreads / 32];
+    const unsigned lane = lane_id();
+    DensityWarp& W = shared[threadIdx.x >> 5];
+    uint8_t* const row = W.list + lane * kDensRow;
     const uint32_t nb = *B.act_n * 8u;
     const uint32_t nitems = nb + *B.wq_n;  // the first window of every bucket, then the queued windows
     const size_t cap = (size_t)P.cap;
-    const float r2 = P.r2, r2list = P.r2list, ss = P.ss;
+    const float r2 = P.r2, r2list = P.r2list;
     const float kFar = __int_as_float(0x7f800000);  // +inf: never within range
     for (uint32_t it = next_bucket(B.dctr, lane); it < nitems; it = next_bucket(B.dctr, lane)) {
         uint32_t c, q, w0;
@@ -661,211 +706,205 @@ __global__ void __launch_bounds__(kThreads, 4) k_density_bucket(const __grid_con
             w0 = e.y;
         }
         const uint32_t bid = c * 8u + q;
-        const uint32_t m0 = __ldg(&B.oct_start[(size_t)bid]);
         const uint32_t m1 = q == 7 ? __ldg(&B.cend[c]) : __ldg(&B.oct_start[(size_t)bid + 1]);
         if (w0 >= m1) continue;
         const uint32_t w1 = min(m1, w0 + (uint32_t)P.bwin);
         // the window's members, one per lane; boundary members carry their volume and need no list
-        const uint32_t tl = w0 + lane;
-        float4 pm = make_float4(kFar, kFar, kFar, -1.f);
-        float rm = 0.f;
-        if (tl < w1) {
-            pm = __ldg(&pos4[tl]);
+        float4 pm = make_float4(0.f, 0.f, 0.f, -1.f);
+        float rho0 = 0.f;
+        if (w0 + lane < w1) {
+            pm = __ldg(&pos4[w0 + lane]);
             if (pm.w < 0.f) {
-                B.densp[tl] = make_float2(-pm.w, 0.f);
-                B.nbr_cnt[tl] = 0;
+                B.densp[w0 + lane] = make_float2(-pm.w, 0.f);
+                B.nbr_cnt[w0 + lane] = 0;
             } else {
-                rm = __ldg(&alpha4[tl]).w;
+                rho0 = __ldg(&alpha4[w0 + lane]).w;
             }
         }
-        const uint32_t fluid = __ballot_sync(0xffffffffu, tl < w1 && pm.w >= 0.f);
+        const uint32_t fluid = __ballot_sync(0xffffffffu, w0 + lane < w1 && pm.w >= 0.f);
         if (!fluid) continue;
-        uint32_t st, off;
-        const uint32_t T = bucket_ranges(P, B, c, q, lane, rstart, roff, st, off);
-        const bool masked = T <= 32u * kMaskWords;
-        if (masked && w0 == m0) {  // the bucket's range table, once per bucket
-            uint32_t* __restrict__ bt = B.btab + (size_t)bid * kTabStride;
-            if (lane < 18) {
-                bt[lane] = off;
-                bt[20 + lane] = st - off;
-            }
-            if (lane == 18) bt[18] = T;
+        // L lanes a fluid member: lane l takes share l % L of member `src` (lane L ord + share)
+        // (the quotients in float: half a unit away from the next whole number)
+        const uint32_t nf = (uint32_t)__popc(fluid);
+        const uint32_t L = (uint32_t)__fdividef(32.5f, (float)nf);
+        const uint32_t ord = (uint32_t)__fdividef((float)lane + 0.5f, (float)L), share = lane - ord * L;
+        uint32_t src = ord;
+        if (fluid != (nf == 32u ? 0xffffffffu : (1u << nf) - 1u)) {  // boundary members among them
+            if (fluid >> lane & 1u) W.list[__popc(fluid & lanemask_lt())] = (uint8_t)lane;
+            __syncwarp();
+            src = ord < nf ? W.list[ord] : 0u;
+            __syncwarp();
         }
-        const uint32_t lst = masked ? (kMaskList | bid) : kRescan;
-        // sequence position of member t = t + self_base: the bucket lies in the range of its own
-        // cell column on its own subcell row (range 8 + part, part = 1 for the low x half)
-        const int rs = 8 + ((q & 1u) == 0u ? 1 : 0);
-        const uint32_t self_base = __shfl_sync(0xffffffffu, off, rs) - __shfl_sync(0xffffffffu, st, rs);
-        Kahan msum;  // lane i: member w0 + i, summed over the candidate blocks
-        int r = 0;
-        const float2 R2 = make_float2(r2, r2), NEG1 = make_float2(-1.f, -1.f);
-        for (uint32_t base = 0; base < T; base += 32u * kBucketChunks) {
-            // chunks 2p and 2p + 1 side by side in float2 pairs (packed FP32 arithmetic):
-            // negated coordinates and w (fluid mass > 0, minus the boundary volume < 0; 0 for padding)
-            float2 NX[kBucketChunks / 2], NY[kBucketChunks / 2], NZ[kBucketChunks / 2], CW[kBucketChunks / 2];
-            bool bnd = false;
-#pragma unroll
-            for (int pr = 0; pr < kBucketChunks / 2; pr++) {
-                float4 c2[2];
-#pragma unroll
-                for (int h = 0; h < 2; h++) {
-                    const uint32_t e = base + lane + 32u * (2 * pr + h);
-                    c2[h] = make_float4(kFar, kFar, kFar, 0.f);
-                    if (e < T) c2[h] = __ldg(&pos4[seq_index(rstart, roff, r, e)]);
-                    bnd |= c2[h].w < 0.f;
+        const bool live = ord < nf;
+        const uint32_t t = w0 + src;
+        const float px = __shfl_sync(0xffffffffu, pm.x, (int)src), py = __shfl_sync(0xffffffffu, pm.y, (int)src),
+                    pz = __shfl_sync(0xffffffffu, pm.z, (int)src);
+        rho0 = __shfl_sync(0xffffffffu, rho0, (int)src);
+        const float2 PX = make_float2(px, px), PY = make_float2(py, py), PZ = make_float2(pz, pz);
+        const float2 SS = make_float2(P.ss, P.ss), R2 = make_float2(r2, r2), NEG1 = make_float2(-1.f, -1.f);
+        const uint32_t T = bucket_rows(P, B, c, q, lane, W.rows);
+        Kahan sum;
+        uint32_t count = 0;  // the member's neighbours in the blocks so far
+        for (uint32_t base = 0; base < T; base += kDensBlock) {
+            const uint32_t n = min(T - base, (uint32_t)kDensBlock);
+            // stage the candidates, a row of two ranges at a time
+            float wmin = 0.f;
+            uint4 rw = W.rows[0];
+#pragma unroll 3
+            for (int r = 0; r < 9; r++) {
+                const uint4 next = W.rows[r + 1];
+                uint32_t e = rw.x + lane, end = next.x;
+                if (T > (uint32_t)kDensBlock) {  // the part of the row in this block
+                    e = max(rw.x, base) + lane;
+                    end = min(end, base + (uint32_t)kDensBlock);
                 }
-                NX[pr] = make_float2(-c2[0].x, -c2[1].x);
-                NY[pr] = make_float2(-c2[0].y, -c2[1].y);
-                NZ[pr] = make_float2(-c2[0].z, -c2[1].z);
-                CW[pr] = make_float2(c2[0].w, c2[1].w);
+                for (; e < end; e += 32u) {
+                    const uint32_t j = e + (e < rw.y ? rw.z : rw.w);
+                    const float4 p = __ldg(&pos4[j]);
+                    wmin = fminf(wmin, p.w);
+                    const uint32_t l = e - base;
+                    float* a = &W.pxy[l >> 1].x + (l & 1u);
+                    float* b = &W.pzw[l >> 1].x + (l & 1u);
+                    a[0] = p.x;
+                    a[2] = p.y;
+                    b[0] = p.z;
+                    b[2] = p.w;
+                    W.cidx[l] = j;
+                }
+                rw = next;
             }
-            const int nch = (int)min((T - base + 31u) >> 5, (uint32_t)kBucketChunks);
-            const uint32_t word0 = base >> 5;
-            // The member loop, with boundary candidates in the block or without (the usual case:
-            // no volume weights and no rest density to broadcast, so fewer live registers).
-            // The weight of a candidate is its mass, or rho0 V for a boundary particle; without
-            // boundary candidates rho0 * 0 + m is m exactly, so both forms give the same sums.
-            auto members = [&](auto with_boundary) {
-                constexpr bool BND = decltype(with_boundary)::value;
-                float2 CM[kBucketChunks / 2], CV[kBucketChunks / 2];
-#pragma unroll
-                for (int pr = 0; pr < kBucketChunks / 2; pr++) {
-                    CM[pr] = CW[pr];
-                    CV[pr] = make_float2(0.f, 0.f);
-                    if (BND) {
-                        CM[pr] = make_float2(fmaxf(CW[pr].x, 0.f), fmaxf(CW[pr].y, 0.f));
-                        CV[pr] = make_float2(fmaxf(-CW[pr].x, 0.f), fmaxf(-CW[pr].y, 0.f));
-                    }
+            if (lane == 0 && (n & 1u)) {  // the odd last one's partner: out of range, no weight
+                float4& a = W.pxy[n >> 1];
+                float4& b = W.pzw[n >> 1];
+                a.y = a.w = b.y = kFar;
+                b.w = 0.f;
+            }
+            const bool any_bnd = __any_sync(0xffffffffu, wmin < 0.f);
+            __syncwarp();
+            const uint32_t npairs = (n + 1u) >> 1;
+            auto dist2 = [&](const float4 a, const float4 b) {
+                float2 dx = __ffma2_rn(make_float2(a.x, a.y), NEG1, PX), dy = __ffma2_rn(make_float2(a.z, a.w), NEG1, PY),
+                       dz = __ffma2_rn(make_float2(b.x, b.y), NEG1, PZ);
+                if (!SS1) {
+                    dx = __fmul2_rn(dx, SS);
+                    dy = __fmul2_rn(dy, SS);
+                    dz = __fmul2_rn(dz, SS);
                 }
-                for (uint32_t fm = fluid; fm != 0u; fm &= fm - 1u) {
-                    const int i = __ffs(fm) - 1;
-                    const float px = __shfl_sync(0xffffffffu, pm.x, i);
-                    const float py = __shfl_sync(0xffffffffu, pm.y, i);
-                    const float pz = __shfl_sync(0xffffffffu, pm.z, i);
-                    const float rho0 = BND ? __shfl_sync(0xffffffffu, rm, i) : 0.f;
-                    const float2 PX = make_float2(px, px), PY = make_float2(py, py), PZ = make_float2(pz, pz);
-                    const float2 RHO = make_float2(rho0, rho0);
-                    const uint32_t t = w0 + (uint32_t)i;
+                return __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
+            };
+            // a neighbour: within the list radius and not at the same place (every consumer of
+            // the lists skips r = 0), so not the member itself
+            auto near = [&](float d2) { return d2 < r2list && d2 > 0.f; };
+            // this lane's pairs. With boundary candidates in the block or without (the usual
+            // case): the weight of a candidate is its mass, or rho0 V for a boundary particle.
+            uint32_t hits = 0;
+            auto walk = [&](auto with_boundary, auto bounded) {
+                constexpr bool BND = decltype(with_boundary)::value;
+                uint32_t p = share;
+                while (p < npairs) {
                     float2 acc = make_float2(0.f, 0.f);
-                    uint32_t mine = 0;  // lane k keeps the mask word of chunk k
-#pragma unroll
-                    for (int pr = 0; pr < kBucketChunks / 2; pr++) {
-                        if (2 * pr < nch) {
-                            float2 dx = __fadd2_rn(PX, NX[pr]), dy = __fadd2_rn(PY, NY[pr]), dz = __fadd2_rn(PZ, NZ[pr]);
-                            if (!SS1) {
-                                const float2 SS = make_float2(ss, ss);
-                                dx = __fmul2_rn(dx, SS);
-                                dy = __fmul2_rn(dy, SS);
-                                dz = __fmul2_rn(dz, SS);
-                            }
-                            float2 dsq = __fmul2_rn(dx, dx);
-                            dsq = __ffma2_rn(dy, dy, dsq);
-                            dsq = __ffma2_rn(dz, dz, dsq);
-                            float2 cc = __ffma2_rn(dsq, NEG1, R2);  // r2 - dsq, rounded once
-                            cc.x = fmaxf(cc.x, 0.f);                // 0 outside h (and for the padding lanes)
-                            cc.y = fmaxf(cc.y, 0.f);
-                            const float2 c3 = __fmul2_rn(__fmul2_rn(cc, cc), cc);
-                            acc = __ffma2_rn(c3, BND ? __ffma2_rn(RHO, CV[pr], CM[pr]) : CM[pr], acc);
-                            // coincident particles stay in the list (every consumer skips r == 0);
-                            // the member itself is cleared below
-                            const uint32_t b0 = __ballot_sync(0xffffffffu, dsq.x < r2list);
-                            const uint32_t b1 = __ballot_sync(0xffffffffu, dsq.y < r2list);
-                            mine = lane == (unsigned)(2 * pr) ? b0 : mine;
-                            mine = lane == (unsigned)(2 * pr + 1) ? b1 : mine;
+                    const uint32_t end = min(npairs, p + 16u * L);
+#pragma unroll 2
+                    for (; p < end; p += L) {
+                        const float4 a = W.pxy[p], b = W.pzw[p];
+                        const float2 d2 = dist2(a, b);
+                        float2 cc = __ffma2_rn(d2, NEG1, R2);  // r2 - d2, rounded once
+                        cc.x = fmaxf(cc.x, 0.f);               // 0 outside h (and for the padding)
+                        cc.y = fmaxf(cc.y, 0.f);
+                        const float2 c3 = __fmul2_rn(__fmul2_rn(cc, cc), cc);
+                        float2 wt = make_float2(b.z, b.w);
+                        if (BND) {
+                            wt.x = wt.x < 0.f ? rho0 * -wt.x : wt.x;
+                            wt.y = wt.y < 0.f ? rho0 * -wt.y : wt.y;
                         }
+                        acc = __ffma2_rn(c3, wt, acc);
+                        // every candidate is stored after the hits so far and stays if it is one
+                        // (no branch; a full row keeps its last byte for this)
+                        row[decltype(bounded)::value ? min(hits, (uint32_t)kDensList) : hits] = (uint8_t)(2u * p);
+                        hits += near(d2.x) ? 1u : 0u;
+                        row[decltype(bounded)::value ? min(hits, (uint32_t)kDensList) : hits] = (uint8_t)(2u * p + 1u);
+                        hits += near(d2.y) ? 1u : 0u;
                     }
-                    const uint32_t es = t + self_base - base;  // the member's own bit, if in this block
-                    if (es < 32u * kBucketChunks && lane == (es >> 5)) mine &= ~(1u << (es & 31u));
-                    if (masked && (int)lane < nch) B.nmask[(size_t)(word0 + lane) * cap + t] = mine;
-                    const float part = warp_sum_f(acc.x + acc.y);
-                    if (lane == (unsigned)i) msum.add(part);
+                    sum.add(acc.x + acc.y);
                 }
             };
-            if (__any_sync(0xffffffffu, bnd))
-                members(std::true_type{});
-            else
-                members(std::false_type{});
-        }
-        if (tl < w1 && pm.w >= 0.f) {
-            B.nbr_cnt[tl] = lst;
-            B.densp[tl] = density_result(P, msum.s, rm);
-        }
-    }
-}
-
-// Index lists from the bucket mask lists: bit e of a member's mask stands for
-// candidate e of its bucket's sequence, whose index is e plus the offset of the
-// sequence range holding e (btab). One thread per in-grid particle; the lanes
-// of a warp emit their n-th entries together and store each group of four as
-// one 16-byte word, so that every group row of the lists is written by one
-// coalesced store. A particle with more
-// than kMaxNbr neighbours keeps its mask list (nbr_cnt = kMaskList | bucket),
-// which the passes decode directly. Particles with more than P.heavy
-// neighbours (their lists flagged kHeavyFlag), with mask lists or left to the
-// cell search are queued in hq for the force and alpha passes.
-__global__ void __launch_bounds__(kThreads) k_expand_lists(const __grid_constant__ DevParams P,
-                                                           const __grid_constant__ DevBuffers B) {
-    const uint32_t t = blockIdx.x * kThreads + threadIdx.x;
-    const uint32_t lst = t < B.cstart[P.G] ? B.nbr_cnt[t] : 0u;
-    const bool mine = (lst & kMaskList) != 0;  // else boundary, index list or cell search already
-    const uint32_t* __restrict__ tab = B.btab + (size_t)(mine ? lst & ~kMaskList : 0u) * kTabStride;
-    const uint32_t nw = mine ? (__ldg(&tab[18]) + 31u) >> 5 : 0u;
-    const size_t cap = (size_t)P.cap;
-    const uint32_t* __restrict__ mw = B.nmask + t;
-    // hits of this particle, then of the warp's busiest lane (the loop bound)
-    uint32_t cnt = 0;
-    for (uint32_t wd = 0; wd < nw; wd++) cnt += __popc(__ldg(mw + (size_t)wd * cap));
-    const bool over = cnt > (uint32_t)kMaxNbr;  // keeps its mask list: nothing to write
-    if (over) cnt = 0;
-    uint32_t rounds = cnt;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) rounds = max(rounds, __shfl_xor_sync(0xffffffffu, rounds, o));
-    uint4* __restrict__ grp = reinterpret_cast<uint4*>(B.nbr) + t;
-    uint32_t q0 = 0, q1 = 0, q2 = 0, q3 = 0;  // the list group being filled
-    // the next mask word and the next range of the table are loaded one ahead, so
-    // that the lockstep rounds wait on neither (only on a run of empty words or ranges)
-    int r = 0;
-    uint32_t end = 0, delta = 0, endn = 0, deltan = 0;
-    if (mine) {
-        end = __ldg(&tab[1]);
-        delta = __ldg(&tab[20]);
-        endn = __ldg(&tab[2]);
-        deltan = __ldg(&tab[21]);
-    }
-    uint32_t wd = 0, m = nw > 0u ? __ldg(mw) : 0u, mn = nw > 1u ? __ldg(mw + cap) : 0u;
-    for (uint32_t n = 0; n < rounds; n++) {
-        if (n < cnt) {
-            while (m == 0u) {
-                m = mn;
-                ++wd;
-                mn = wd + 1u < nw ? __ldg(mw + (size_t)(wd + 1u) * cap) : 0u;
+            if (live) {
+                // four lanes or more a member: at most 64 candidates each, the row holds them all
+                if (L >= 4u) {
+                    if (any_bnd) walk(std::true_type{}, std::false_type{});
+                    else walk(std::false_type{}, std::false_type{});
+                } else {
+                    if (any_bnd) walk(std::true_type{}, std::true_type{});
+                    else walk(std::false_type{}, std::true_type{});
+                }
             }
-            const uint32_t e = (wd << 5) + (uint32_t)(__ffs(m) - 1);
-            m &= m - 1u;
-            while (e >= end) {  // ends at tab[18] = the sequence length > e; reads stay below tab[39]
-                r++;
-                end = endn;
-                delta = deltan;
-                endn = __ldg(&tab[r + 2]);
-                deltan = __ldg(&tab[21 + r]);
+            __syncwarp();
+            // the member's hits before this lane's, and all of them
+            uint32_t before = hits;
+            for (uint32_t o = 1; o < L; o <<= 1) {
+                const uint32_t v = __shfl_up_sync(0xffffffffu, before, o);
+                if (share >= o) before += v;
             }
-            const uint32_t v = e + delta, u = n & 3u;
-            q0 = u == 0u ? v : q0;
-            q1 = u == 1u ? v : q1;
-            q2 = u == 2u ? v : q2;
-            q3 = u == 3u ? v : q3;
-            if (u == 3u || n + 1u == cnt) grp[(size_t)(n >> 2) * cap] = make_uint4(q0, q1, q2, q3);
+            const int last = (int)min(lane - share + L - 1u, 31u);
+            const uint32_t total = __shfl_sync(0xffffffffu, before, last);
+            before -= hits;
+            if (!__any_sync(0xffffffffu, total > (uint32_t)kDensList)) {
+                // join the lanes' rows in the member's first one, then write rows of four
+                uint8_t* const joined = W.list + (lane - share) * kDensRow;
+                if (share != 0u)
+                    for (uint32_t i = 0; i < hits; i++) joined[before + i] = row[i];
+                __syncwarp();
+                if ((count & 3u) == 0u && count + total <= (uint32_t)kMaxNbr) {
+                    uint4* const out = reinterpret_cast<uint4*>(B.nbr) + t;
+                    for (uint32_t k = share; 4u * k < total; k += L) {
+                        const uchar4 e = *reinterpret_cast<const uchar4*>(joined + 4u * k);  // past the end: any bytes
+                        out[((size_t)(count >> 2) + k) * cap] = make_uint4(W.cidx[e.x], W.cidx[e.y], W.cidx[e.z], W.cidx[e.w]);
+                    }
+                } else {
+                    for (uint32_t k = share; k < total; k += L)
+                        if (count + k < (uint32_t)kMaxNbr) B.nbr[nbr_at(cap, t, count + k)] = W.cidx[joined[k]];
+                }
+            } else if (live) {  // too many for the rows: found again, stored one by one
+                uint32_t k = count + before;
+                for (uint32_t p = share; p < npairs; p += L) {
+                    const float2 d2 = dist2(W.pxy[p], W.pzw[p]);
+                    if (near(d2.x)) {
+                        if (k < (uint32_t)kMaxNbr) B.nbr[nbr_at(cap, t, k)] = W.cidx[2u * p];
+                        k++;
+                    }
+                    if (near(d2.y)) {
+                        if (k < (uint32_t)kMaxNbr) B.nbr[nbr_at(cap, t, k)] = W.cidx[2u * p + 1u];
+                        k++;
+                    }
+                }
+            }
+            count += total;
+            __syncwarp();  // before the candidates and rows are rewritten
         }
-    }
-    const bool heavy = (mine && (over || cnt > P.heavy)) || lst == kRescan;
-    if (mine && !over) B.nbr_cnt[t] = heavy ? (cnt | kHeavyFlag) : cnt;
-    const uint32_t hb = __ballot_sync(0xffffffffu, heavy);
-    if (hb) {
-        const unsigned lane = lane_id();
-        uint32_t base = 0;
-        if (lane == 0) base = atomicAdd(B.hq_n, (uint32_t)__popc(hb));
-        base = __shfl_sync(0xffffffffu, base, 0);
-        if (heavy) B.hq[base + __popc(hb & lanemask_lt())] = t;
+        float dens = sum.s - sum.c;  // of this lane and the member's lanes before it
+        for (uint32_t o = 1; o < L; o <<= 1) {
+            const float v = __shfl_up_sync(0xffffffffu, dens, o);
+            if (share >= o) dens += v;
+        }
+        const bool own = live && share == L - 1u;  // holds the whole sum
+        // lists that overflowed: mask lists, or the cell search where the sequence is too long for them
+        const bool over = own && count > (uint32_t)kMaxNbr;
+        const bool masked = T <= 32u * kMaskWords;
+        if (__any_sync(0xffffffffu, over) && masked)
+            overflow_masks<SS1>(P, B, pos4, __reduce_or_sync(0xffffffffu, over ? 1u << src : 0u), pm, w0, bid, T,
+                                W.rows);
+        const bool heavy = own && count > P.heavy;  // P.heavy <= kMaxNbr
+        if (own) {
+            B.nbr_cnt[t] = over ? (masked ? kMaskList | bid : kRescan) : heavy ? count | kHeavyFlag : count;
+            B.densp[t] = density_result(P, dens, rho0);
+        }
+        const uint32_t hb = __ballot_sync(0xffffffffu, heavy);
+        if (hb) {  // queued for the force and alpha passes
+            uint32_t at = 0;
+            if (lane == 0) at = atomicAdd(B.hq_n, (uint32_t)__popc(hb));
+            at = __shfl_sync(0xffffffffu, at, 0);
+            if (heavy) B.hq[at + __popc(hb & lanemask_lt())] = t;
+        }
     }
 }
 
@@ -1633,14 +1672,14 @@ __global__ void __launch_bounds__(kThreads) k_unpack_field(const __grid_constant
 
 inline int blocks_for(int n, int t = kThreads) { return (n + t - 1) / t; }
 
-// Blocks of kThreads that are resident at once on the whole device (for
+// Blocks of `threads` that are resident at once on the whole device (for
 // kernels that loop over a device-side work count).
 template <class K>
-int resident_grid(K kernel) {
+int resident_grid(K kernel, int threads) {
     int dev = 0, sms = 0, per = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, kThreads, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, threads, 0);
     if (sms <= 0) sms = 1;
     if (per <= 0) per = 1;
     return sms * per;
@@ -1714,10 +1753,9 @@ void launch_density_oct(const DevParams& P, const DevBuffers& B, const int* cur,
     const float4* alpha = B.f4[ALPHA][cur[ALPHA]];
     cudaMemsetAsync(B.dctr, 0, sizeof(uint32_t), s);
     if (P.ss == 1.0f)
-        k_density_bucket<true><<<resident_grid(k_density_bucket<true>), kThreads, 0, s>>>(P, B, pos, alpha);
+        k_density_bucket<true><<<resident_grid(k_density_bucket<true>, kDensThreads), kDensThreads, 0, s>>>(P, B, pos, alpha);
     else
-        k_density_bucket<false><<<resident_grid(k_density_bucket<false>), kThreads, 0, s>>>(P, B, pos, alpha);
-    k_expand_lists<<<blocks_for(P.n), kThreads, 0, s>>>(P, B);
+        k_density_bucket<false><<<resident_grid(k_density_bucket<false>, kDensThreads), kDensThreads, 0, s>>>(P, B, pos, alpha);
 }
 
 template <bool F, bool D>
