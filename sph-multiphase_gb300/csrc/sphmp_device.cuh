@@ -250,6 +250,44 @@ __device__ __forceinline__ void warp_for_slot_list(const DevParams& P, const Dev
     });
 }
 
+// The neighbours of particle s shared out over the L lanes of a group (`g` this
+// lane): every L-th group row of its index list, mask word or candidate of the
+// cell search. The caller reduces the lanes' partial sums (group_sum).
+template <int L, class F>
+__device__ __forceinline__ void group_for_slot_list(const DevParams& P, const DevBuffers& B, int s, uint32_t g,
+                                                    float x, float y, float z, F&& f) {
+    if (P.list_mode != 0) {
+        const uint32_t raw = B.nbr_cnt[s];
+        if (raw & kMaskList) {
+            for_mask_words(P, B, s, raw & ~kMaskList, g, (uint32_t)L, f);
+            return;
+        }
+        const uint32_t cnt = raw & ~kHeavyFlag;
+        if (cnt <= (uint32_t)kMaxNbr) {
+            const uint4* __restrict__ grp = reinterpret_cast<const uint4*>(B.nbr) + s;
+            for (uint32_t k = 4u * g; k < cnt; k += 4u * L) {
+                const uint4 q = __ldg(grp + (size_t)(k >> 2) * (size_t)P.cap);
+                f(q.x);
+                if (k + 1u < cnt) f(q.y);
+                if (k + 2u < cnt) f(q.z);
+                if (k + 3u < cnt) f(q.w);
+            }
+            return;
+        }
+    }
+    for_candidate_rows(P, B, B.mgcell[s], x, y, z, [&](uint32_t j0, uint32_t j1) {
+        for (uint32_t j = j0 + g; j < j1; j += L) f(j);
+    });
+}
+
+// The sum of v over the L consecutive lanes of a group (all lanes of the warp call).
+template <int L>
+__device__ __forceinline__ float group_sum(float v) {
+#pragma unroll
+    for (int o = L / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
 // ---------------------------------------------------------------------------
 // Density + EOS (MfComputePressureCUDA)
 // ---------------------------------------------------------------------------
@@ -382,18 +420,20 @@ struct ForceDrift {
         }
     }
 
-    // Sum the lanes' partial sums (warp-cooperative particles); every lane gets the totals.
-    __device__ __forceinline__ void warp_reduce() {
+    // Sum the partial sums of the L lanes that share a particle (32: warp-cooperative
+    // particles); every lane gets the totals.
+    template <int L>
+    __device__ __forceinline__ void reduce() {
         if (FORCE) {
-            fx = warp_sum_f(fx);
-            fy = warp_sum_f(fy);
-            fz = warp_sum_f(fz);
+            fx = group_sum<L>(fx);
+            fy = group_sum<L>(fy);
+            fz = group_sum<L>(fz);
         }
         if (DRIFT) {
 #pragma unroll
             for (int k = 0; k < NP; k++) {
-                dv[k].x = warp_sum_f(dv[k].x); dv[k].y = warp_sum_f(dv[k].y); dv[k].z = warp_sum_f(dv[k].z);
-                ag[k].x = warp_sum_f(ag[k].x); ag[k].y = warp_sum_f(ag[k].y); ag[k].z = warp_sum_f(ag[k].z);
+                dv[k].x = group_sum<L>(dv[k].x); dv[k].y = group_sum<L>(dv[k].y); dv[k].z = group_sum<L>(dv[k].z);
+                ag[k].x = group_sum<L>(ag[k].x); ag[k].y = group_sum<L>(ag[k].y); ag[k].z = group_sum<L>(ag[k].z);
             }
         }
     }
@@ -604,17 +644,18 @@ struct AlphaChange {
         }
     }
 
-    // Sum the lanes' compensated partial sums (warp-cooperative particles).
-    __device__ __forceinline__ void warp_reduce() {
+    // Sum the compensated partial sums of the L lanes that share a particle.
+    template <int L>
+    __device__ __forceinline__ void reduce() {
 #pragma unroll
         for (int k = 0; k < NP; k++) {
-            acc[k].s = warp_sum_f(acc[k].s - acc[k].c);
+            acc[k].s = group_sum<L>(acc[k].s - acc[k].c);
             acc[k].c = 0.f;
         }
-        sdot = warp_sum_f(sdot);
-        sdx = warp_sum_f(sdx);
-        sdy = warp_sum_f(sdy);
-        sdz = warp_sum_f(sdz);
+        sdot = group_sum<L>(sdot);
+        sdx = group_sum<L>(sdx);
+        sdy = group_sum<L>(sdy);
+        sdz = group_sum<L>(sdz);
     }
 
     // dalpha * dt clamped at -0.99, added to the start-of-step fraction.

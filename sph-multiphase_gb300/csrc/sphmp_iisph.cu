@@ -323,13 +323,6 @@ __device__ __forceinline__ void ii_walk(const DevParams& P, const DevBuffers& B,
     }
 }
 
-template <int L>
-__device__ __forceinline__ float group_sum(float v) {
-#pragma unroll
-    for (int o = L / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-
 // ComputeDii, first half (:673-760): the advection acceleration (the boundary's
 // artificial viscosity within 2h plus gravity; the fluid terms are commented
 // out in the reference) and veleval = vel + a dt.

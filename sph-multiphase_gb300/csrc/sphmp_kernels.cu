@@ -985,17 +985,17 @@ __device__ __forceinline__ void force_drift_warp(const DevParams& P, const DevBu
         const float4 aj = DRIFT ? __ldg(&alpha4[j]) : make_float4(0.f, 0.f, 0.f, 0.f);
         acc.pair(P, pj, dpj, vj, aj);
     });
-    acc.warp_reduce();
+    acc.template reduce<32>();
     if (lane_id() == 0)
         acc.finish(P, B, s, DRIFT ? aprev4[s] : make_float4(0.f, 0.f, 0.f, 0.f),
                    FORCE && DRIFT ? vev4[s] : make_float4(0.f, 0.f, 0.f, 0.f));
 }
 
-// Force + drift, one thread per particle; every warp first takes heavy
+// Force + drift, L lanes per particle (walk_lanes); every warp first takes heavy
 // particles from the queue (whole warp per particle) while any are left. With
 // both, it also writes every in-grid particle's neighbour record for the fused
 // alpha pass.
-template <bool FORCE, bool DRIFT, int NP>
+template <bool FORCE, bool DRIFT, int NP, int L>
 __global__ void __launch_bounds__(kThreads, 4) k_force_drift(const __grid_constant__ DevParams P,
                                                              const __grid_constant__ DevBuffers B,
                                                              const float4* __restrict__ pos4,
@@ -1009,20 +1009,41 @@ __global__ void __launch_bounds__(kThreads, 4) k_force_drift(const __grid_consta
         for (uint32_t h = next_item(&B.hctr[0], nh, lane); h < nh; h = next_item(&B.hctr[0], nh, lane))
             force_drift_warp<FORCE, DRIFT, NP>(P, B, pos4, vel4, alpha4, aprev4, vev4, (int)B.hq[h]);
     }
-    const int s = blockIdx.x * kThreads + threadIdx.x;
-    if (s >= active_n(B) || B.mgcell[s] == kUndef) return;
-    const float4 pi = pos4[s];
-    if (pi.w < 0.f) {
+    const int s = (int)((blockIdx.x * (unsigned)kThreads + threadIdx.x) / L);
+    const unsigned g = threadIdx.x % L;
+    const bool in = s < active_n(B) && B.mgcell[s] != kUndef;
+    if (L == 1 && !in) return;
+    const float4 pi = in ? pos4[s] : make_float4(0.f, 0.f, 0.f, -1.f);
+    if (in && g == 0 && pi.w < 0.f) {
         if (FORCE) B.accel4[s] = make_float4(0.f, 0.f, 0.f, 0.f);
         if (FORCE && DRIFT) {
             const float a0[3] = {0.f, 0.f, 0.f};
             const float u0[9] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
             write_nrec(B, s, pi, -1.f, make_float4(0.f, 0.f, 0.f, 0.f), a0, u0);
         }
+    }
+    const bool walk = !(pi.w < 0.f) && !is_heavy(P, B.nbr_cnt[s]);  // heavy: taken from the queue
+    if (L == 1) {
+        if (walk) force_drift_one<FORCE, DRIFT, NP>(P, B, pos4, vel4, alpha4, aprev4, vev4, s, pi);
         return;
     }
-    if (is_heavy(P, B.nbr_cnt[s])) return;  // taken from the queue
-    force_drift_one<FORCE, DRIFT, NP>(P, B, pos4, vel4, alpha4, aprev4, vev4, s, pi);
+    if (!__any_sync(0xffffffffu, walk)) return;
+    ForceDrift<FORCE, DRIFT, NP> acc;
+    const int si = walk ? s : 0;
+    acc.init(P, pi, vel4[si], B.densp[si], alpha4[si]);
+    if (walk)
+        group_for_slot_list<L>(P, B, s, g, pi.x, pi.y, pi.z, [&](uint32_t j) {
+            const float4 pj = __ldg(&pos4[j]);
+            const float2 dpj = __ldg(&B.densp[j]);
+            const float4 vj = FORCE ? __ldg(&vel4[j]) : make_float4(0.f, 0.f, 0.f, 0.f);
+            const float4 aj = DRIFT ? __ldg(&alpha4[j]) : make_float4(0.f, 0.f, 0.f, 0.f);
+            acc.pair(P, pj, dpj, vj, aj);
+        });
+    __syncwarp();
+    acc.template reduce<L>();
+    if (walk && g == 0)
+        acc.finish(P, B, s, DRIFT ? aprev4[s] : make_float4(0.f, 0.f, 0.f, 0.f),
+                   FORCE && DRIFT ? vev4[s] : make_float4(0.f, 0.f, 0.f, 0.f));
 }
 
 // Force + drift of a corrected large step: the same pass, also filling the
@@ -1251,24 +1272,28 @@ __global__ void __launch_bounds__(kThreads) k_advance(const __grid_constant__ De
     aprev4[s] = ap;
 }
 
-// Alpha change of in-grid particle s with its neighbours' data from the
-// neighbour records the force + drift pass of this step wrote (five 16-byte
+// The pair of a particle and its neighbour j in the alpha change, j's data from
+// the neighbour record the force + drift pass of this step wrote (five 16-byte
 // loads per neighbour instead of seven separate gathers).
+template <int NP>
+__device__ __forceinline__ void nrec_pair(const DevParams& P, const DevBuffers& B, uint32_t j, AlphaChange<NP>& acc) {
+    float4 q[5];
+    read_nrec<NP>(B, j, q);
+    const float4 r0 = q[0], r1 = q[1], r2 = q[2], r3 = q[3], r4 = q[4];
+    float4 uj[NP];
+    uj[0] = make_float4(r2.z, r2.w, r3.x, 0.f);
+    if (NP > 1) uj[NP > 1 ? 1 : 0] = make_float4(r3.y, r3.z, r3.w, 0.f);
+    if (NP > 2) uj[NP > 2 ? 2 : 0] = make_float4(r4.x, r4.y, r4.z, 0.f);
+    acc.pair(P, r0, r0.w, make_float4(r1.x, r1.y, r1.z, 0.f), make_float4(r1.w, r2.x, r2.y, 0.f), uj);
+}
+
+// Alpha change of in-grid particle s, by one thread.
 template <int NP>
 __device__ __forceinline__ void alpha_change_nrec(const DevParams& P, const DevBuffers& B, int s, const float4 pi,
                                                   const float4 vei, const float4 ai, float (&out)[3]) {
     AlphaChange<NP> acc;
     acc.init(pi, vei, ai, B.drift4 + s, (size_t)P.cap);
-    for_slot_list(P, B, s, pi.x, pi.y, pi.z, [&](uint32_t j) {
-        float4 q[5];
-        read_nrec<NP>(B, j, q);
-        const float4 r0 = q[0], r1 = q[1], r2 = q[2], r3 = q[3], r4 = q[4];
-        float4 uj[NP];
-        uj[0] = make_float4(r2.z, r2.w, r3.x, 0.f);
-        if (NP > 1) uj[NP > 1 ? 1 : 0] = make_float4(r3.y, r3.z, r3.w, 0.f);
-        if (NP > 2) uj[NP > 2 ? 2 : 0] = make_float4(r4.x, r4.y, r4.z, 0.f);
-        acc.pair(P, r0, r0.w, make_float4(r1.x, r1.y, r1.z, 0.f), make_float4(r1.w, r2.x, r2.y, 0.f), uj);
-    });
+    for_slot_list(P, B, s, pi.x, pi.y, pi.z, [&](uint32_t j) { nrec_pair<NP>(P, B, j, acc); });
     acc.result(P, out);
 }
 
@@ -1280,17 +1305,8 @@ __device__ __forceinline__ void alpha_change_nrec_warp(const DevParams& P, const
     const float4 pi = S.in[POS][s], vei = S.in[VEV][s], ai = S.in[ALPHA][s];
     AlphaChange<NP> acc;
     acc.init(pi, vei, ai, B.drift4 + s, (size_t)P.cap);
-    warp_for_slot_list(P, B, s, pi.x, pi.y, pi.z, [&](uint32_t j) {
-        float4 q[5];
-        read_nrec<NP>(B, j, q);
-        const float4 r0 = q[0], r1 = q[1], r2 = q[2], r3 = q[3], r4 = q[4];
-        float4 uj[NP];
-        uj[0] = make_float4(r2.z, r2.w, r3.x, 0.f);
-        if (NP > 1) uj[NP > 1 ? 1 : 0] = make_float4(r3.y, r3.z, r3.w, 0.f);
-        if (NP > 2) uj[NP > 2 ? 2 : 0] = make_float4(r4.x, r4.y, r4.z, 0.f);
-        acc.pair(P, r0, r0.w, make_float4(r1.x, r1.y, r1.z, 0.f), make_float4(r1.w, r2.x, r2.y, 0.f), uj);
-    });
-    acc.warp_reduce();
+    warp_for_slot_list(P, B, s, pi.x, pi.y, pi.z, [&](uint32_t j) { nrec_pair<NP>(P, B, j, acc); });
+    acc.template reduce<32>();
     acc.result(P, out);
 }
 
@@ -1316,7 +1332,7 @@ __device__ __forceinline__ void pass_c_finish(const DevParams& P, const DevBuffe
 // cur buffers, writes every float4 field of every particle into the other
 // buffer. Every warp first takes heavy particles from the queue (whole warp per
 // alpha sum, lane 0 finishes the particle) while any are left.
-template <int NP, bool MP>
+template <int NP, bool MP, int L>
 __global__ void __launch_bounds__(kThreads, 4) k_pass_c(const __grid_constant__ DevParams P,
                                                         const __grid_constant__ DevBuffers B,
                                                         const __grid_constant__ F4Set S) {
@@ -1330,16 +1346,30 @@ __global__ void __launch_bounds__(kThreads, 4) k_pass_c(const __grid_constant__ 
             if (lane == 0) pass_c_finish<NP, MP>(P, B, S, sh, false, S.in[POS][sh], S.in[VEV][sh], S.in[ALPHA][sh], a);
         }
     }
-    const int s = blockIdx.x * kThreads + threadIdx.x;
-    if (s >= active_n(B)) return;
-    const float4 p = S.in[POS][s], ve = S.in[VEV][s], al = S.in[ALPHA][s];
-    const bool undef = B.mgcell[s] == kUndef;
+    const int s = (int)((blockIdx.x * (unsigned)kThreads + threadIdx.x) / L);
+    const unsigned g = threadIdx.x % L;
+    const bool in = s < active_n(B);
+    if (L == 1 && !in) return;
+    const int si = in ? s : 0;
+    const float4 p = S.in[POS][si], ve = S.in[VEV][si], al = S.in[ALPHA][si];
+    const bool undef = B.mgcell[si] == kUndef;
     // the alpha sum is needed for in-grid fluid particles (pass_c_slot)
-    const bool walk = MP && !undef && !(p.w < 0.f);
-    if (walk && is_heavy(P, B.nbr_cnt[s])) return;  // taken from the queue
+    const bool sum = MP && in && !undef && !(p.w < 0.f);
+    const bool heavy = sum && is_heavy(P, B.nbr_cnt[si]);  // taken from the queue
+    const bool walk = sum && !heavy;
     float anew[3] = {al.x, al.y, al.z};
-    if (walk) alpha_change_nrec<NP>(P, B, s, p, ve, al, anew);
-    pass_c_finish<NP, MP>(P, B, S, s, undef, p, ve, al, anew);
+    if (L == 1) {
+        if (heavy) return;
+        if (walk) alpha_change_nrec<NP>(P, B, s, p, ve, al, anew);
+    } else if (__any_sync(0xffffffffu, walk)) {
+        AlphaChange<NP> acc;
+        acc.init(p, ve, al, B.drift4 + si, (size_t)P.cap);
+        if (walk) group_for_slot_list<L>(P, B, s, g, p.x, p.y, p.z, [&](uint32_t j) { nrec_pair<NP>(P, B, j, acc); });
+        __syncwarp();
+        acc.template reduce<L>();
+        if (walk) acc.result(P, anew);
+    }
+    if (L == 1 || (in && g == 0 && !heavy)) pass_c_finish<NP, MP>(P, B, S, s, undef, p, ve, al, anew);
 }
 
 // ---------------------------------------------------------------------------
@@ -1672,6 +1702,9 @@ __global__ void __launch_bounds__(kThreads) k_unpack_field(const __grid_constant
 
 inline int blocks_for(int n, int t = kThreads) { return (n + t - 1) / t; }
 
+// Blocks of kThreads for `lanes` threads per particle.
+inline int walk_blocks(int n, int lanes) { return (int)(((long long)n * lanes + kThreads - 1) / kThreads); }
+
 // Blocks of `threads` that are resident at once on the whole device (for
 // kernels that loop over a device-side work count).
 template <class K>
@@ -1758,24 +1791,42 @@ void launch_density_oct(const DevParams& P, const DevBuffers& B, const int* cur,
         k_density_bucket<false><<<resident_grid(k_density_bucket<false>, kDensThreads), kDensThreads, 0, s>>>(P, B, pos, alpha);
 }
 
-template <bool F, bool D>
-static void fd_dispatch(const DevParams& P, const DevBuffers& B, const int* cur, cudaStream_t s) {
-    cudaMemsetAsync(&B.hctr[0], 0, sizeof(uint32_t), s);  // the heavy-particle queue's work counter
+// Lanes that share a particle in the list walks of the force and alpha passes. One
+// thread a particle walks its neighbours as a chain of dependent gathers, which
+// only many warps hide: a chip of 152 SMs holds 155,648 threads of these kernels
+// (four blocks of 256 an SM). With fewer particles more lanes each are faster
+// until they fill it; with more, the lanes' shuffles and repeated loads of the
+// particle's own data only cost. Force + drift and alpha passes together, us, at
+// one, two, four and eight lanes: 51, 33, 25, 21 at 22 K slots; 54, 38, 30, 38 at
+// 49 K; 60, 57, 59, 69 at 106 K; 127, 107, 123, 165 at 244 K; 199, 186, 222, 299
+// at 421 K; 322, 338, 420, 585 at 778 K; 518, 580, 720, 1012 at 1.3 M.
+static int walk_lanes(int n) {
+    constexpr int kResident = 152 * 4 * kThreads;
+    return n <= kResident / 6 ? 8 : n <= kResident / 2 ? 4 : n <= 3 * kResident ? 2 : 1;
+}
+
+template <bool F, bool D, int NP>
+static void fd_lanes(const DevParams& P, const DevBuffers& B, const int* cur, cudaStream_t s) {
     const float4* pos = B.f4[POS][cur[POS]];
     const float4* vel = B.f4[VEL][cur[VEL]];
     const float4* al = B.f4[ALPHA][cur[ALPHA]];
     const float4* ap = B.f4[APREV][cur[APREV]];
     const float4* ve = B.f4[VEV][cur[VEV]];
-    const int g = blocks_for(P.n);
-    if (!D) {
-        k_force_drift<F, false, 0><<<g, kThreads, 0, s>>>(P, B, pos, vel, al, ap, ve);
-        return;
+    switch (walk_lanes(P.n)) {
+        case 8: k_force_drift<F, D, NP, 8><<<walk_blocks(P.n, 8), kThreads, 0, s>>>(P, B, pos, vel, al, ap, ve); break;
+        case 4: k_force_drift<F, D, NP, 4><<<walk_blocks(P.n, 4), kThreads, 0, s>>>(P, B, pos, vel, al, ap, ve); break;
+        case 2: k_force_drift<F, D, NP, 2><<<walk_blocks(P.n, 2), kThreads, 0, s>>>(P, B, pos, vel, al, ap, ve); break;
+        default: k_force_drift<F, D, NP, 1><<<walk_blocks(P.n, 1), kThreads, 0, s>>>(P, B, pos, vel, al, ap, ve); break;
     }
-    switch (P.nphase) {
-        case 1: k_force_drift<F, true, 1><<<g, kThreads, 0, s>>>(P, B, pos, vel, al, ap, ve); break;
-        case 2: k_force_drift<F, true, 2><<<g, kThreads, 0, s>>>(P, B, pos, vel, al, ap, ve); break;
-        default: k_force_drift<F, true, 3><<<g, kThreads, 0, s>>>(P, B, pos, vel, al, ap, ve); break;
-    }
+}
+
+template <bool F, bool D>
+static void fd_dispatch(const DevParams& P, const DevBuffers& B, const int* cur, cudaStream_t s) {
+    cudaMemsetAsync(&B.hctr[0], 0, sizeof(uint32_t), s);  // the heavy-particle queue's work counter
+    if (!D) fd_lanes<F, false, 0>(P, B, cur, s);
+    else if (P.nphase == 1) fd_lanes<F, true, 1>(P, B, cur, s);
+    else if (P.nphase == 2) fd_lanes<F, true, 2>(P, B, cur, s);
+    else fd_lanes<F, true, 3>(P, B, cur, s);
 }
 
 void launch_force_drift(const DevParams& P, const DevBuffers& B, const int* cur, bool force, bool drift,
@@ -1861,20 +1912,24 @@ void launch_advance(const DevParams& P, const DevBuffers& B, const int* cur, cud
                                                     B.f4[VEV][cur[VEV]], B.f4[APREV][cur[APREV]]);
 }
 
+template <int NP>
+static void pass_c_lanes(const DevParams& P, const DevBuffers& B, const F4Set& S, cudaStream_t s) {
+    switch (walk_lanes(P.n)) {
+        case 8: k_pass_c<NP, true, 8><<<walk_blocks(P.n, 8), kThreads, 0, s>>>(P, B, S); break;
+        case 4: k_pass_c<NP, true, 4><<<walk_blocks(P.n, 4), kThreads, 0, s>>>(P, B, S); break;
+        case 2: k_pass_c<NP, true, 2><<<walk_blocks(P.n, 2), kThreads, 0, s>>>(P, B, S); break;
+        default: k_pass_c<NP, true, 1><<<walk_blocks(P.n, 1), kThreads, 0, s>>>(P, B, S); break;
+    }
+}
+
 void launch_pass_c(const DevParams& P, const DevBuffers& B, const int* cur, cudaStream_t s) {
     if (P.n <= 0) return;
     const F4Set S = make_set(B, cur, true);
-    const int g = blocks_for(P.n);
     cudaMemsetAsync(&B.hctr[1], 0, sizeof(uint32_t), s);  // the heavy-particle queue's work counter
-    if (!P.multiphase) {
-        k_pass_c<1, false><<<g, kThreads, 0, s>>>(P, B, S);
-        return;
-    }
-    switch (P.nphase) {
-        case 1: k_pass_c<1, true><<<g, kThreads, 0, s>>>(P, B, S); break;
-        case 2: k_pass_c<2, true><<<g, kThreads, 0, s>>>(P, B, S); break;
-        default: k_pass_c<3, true><<<g, kThreads, 0, s>>>(P, B, S); break;
-    }
+    if (!P.multiphase) k_pass_c<1, false, 1><<<blocks_for(P.n), kThreads, 0, s>>>(P, B, S);
+    else if (P.nphase == 1) pass_c_lanes<1>(P, B, S, s);
+    else if (P.nphase == 2) pass_c_lanes<2>(P, B, S, s);
+    else pass_c_lanes<3>(P, B, S, s);
 }
 
 void launch_conservation(const DevParams& P, const DevBuffers& B, const int* cur, cudaStream_t s) {
