@@ -36,6 +36,8 @@ struct sphmp_ctx {
     bool oct_valid = false;       // the internal order is octant-grouped for the current cell list
     bool pos_sorted = false;      // positions unchanged since the cell list was built from them
     int hash_n = -1;              // particle count the cell keys were computed for (-1: none)
+    bool listed = false;          // GetGridList has run since the last hash
+    bool counts_clear = true;     // the hash's counts (B.ccount ...) are zero: a step's sort leaves them so
     int list_mode = 0;            // kind of list the last density pass wrote (DevParams::list_mode)
     int device = 0;
     cudaStream_t own_stream = nullptr;
@@ -229,9 +231,9 @@ void free_buffers(sphmp_ctx* c) {
     for (int f = 0; f < kNumFloat4Fields; f++)
         for (int b = 0; b < 2; b++) cudaFree(B.f4[f][b]);
     void* ptrs[] = {B.densp, B.accel4, B.drift4, B.velxcor, B.pmod, B.mgcell, B.midsort, B.mgndx, B.mgridoff, B.mgridcnt,
-                    B.key, B.octk, B.arank, B.sidx, B.ccount, B.cstart, B.cend, B.corder, B.bsum, B.uchunk, B.big, B.color, B.bornid,
-                    B.mass_raw, B.err, B.red, B.vtmp, B.nbr, B.nbr_cnt, B.nmask, B.btab, B.dctr, B.wq, B.wq_n, B.hq, B.hq_n, B.hctr, B.iis_dii, B.iis_dijpj, B.iis_aii, B.iis_rho_adv, B.iis_pl, B.iis_dsum, B.iis_pm, B.iis_ctl, B.iis_list, B.nrec, B.opos, B.oidx, B.osrc, B.oct_start,
-                    B.act, B.act_n, B.nact, B.frame, c->stage};
+                    B.key, B.octk, B.arank, B.sidx, B.ccount, B.cstart, B.cend, B.corder, B.uchunk, B.big, B.ctl, B.color, B.bornid,
+                    B.mass_raw, B.err, B.red, B.vtmp, B.nbr, B.nbr_cnt, B.nmask, B.btab, B.wq, B.hq, B.iis_dii, B.iis_dijpj, B.iis_aii, B.iis_rho_adv, B.iis_pl, B.iis_dsum, B.iis_pm, B.iis_ctl, B.iis_list, B.nrec, B.opos, B.oidx, B.osrc, B.oct_start,
+                    B.act, B.nact, B.frame, c->stage};
     for (void* q : ptrs) cudaFree(q);
     memset(&c->B, 0, sizeof(c->B));
     c->stage = nullptr;
@@ -262,12 +264,15 @@ sphmp_status alloc_buffers(sphmp_ctx* c) {
     CK(dalloc(&B.octk, N));
     CK(dalloc(&B.arank, N));
     CK(dalloc(&B.sidx, N));
-    CK(dalloc(&B.ccount, G + 1));
+    const size_t nb = G / kScanPer + 2, nu = N / ((size_t)kHashBlock * kHashBlock) + 2;
+    const size_t nc = (G + 4) / 4 * 4;  // the sums behind the counts start on 16 bytes
+    B.count_bytes = sizeof(uint32_t) * (nc + nb + nu);
+    CK(dalloc(&B.ccount, nc + nb + nu));
+    B.bsum = B.ccount + nc;
+    B.usum = B.bsum + nb;
     CK(dalloc(&B.cstart, G + 2));
     CK(dalloc(&B.cend, G));
     CK(dalloc(&B.corder, G));
-    const size_t per = (size_t)kScanBlock * kScanItems;
-    CK(dalloc(&B.bsum, (G + per - 1) / per + 1));
     CK(dalloc(&B.uchunk, N / kHashBlock + 2));
     CK(dalloc(&B.big, N / (kWarpSortMax + 1) + 2));
     CK(dalloc(&B.color, N));
@@ -280,14 +285,16 @@ sphmp_status alloc_buffers(sphmp_ctx* c) {
     CK(dalloc(&B.nbr_cnt, N));
     CK(dalloc(&B.nmask, (size_t)kMaskWords * N));
     CK(dalloc(&B.btab, 8 * G * kTabStride));
-    CK(dalloc(&B.dctr, 1));
     CK(dalloc(&B.wq, N / kBucketWindowMin + 16));
-    CK(dalloc(&B.wq_n, 1));
-    CK(cudaMemset(B.wq_n, 0, sizeof(uint32_t)));
     CK(dalloc(&B.hq, N));
-    CK(dalloc(&B.hq_n, 1));
-    CK(dalloc(&B.hctr, 2));
-    CK(cudaMemset(B.hq_n, 0, sizeof(uint32_t)));
+    CK(dalloc(&B.ctl, kCtlWords));
+    CK(cudaMemset(B.ctl, 0, sizeof(uint32_t) * kCtlWords));
+    B.act_n = B.ctl;
+    B.wq_n = B.ctl + 1;
+    B.hq_n = B.ctl + 2;
+    B.dctr = B.ctl + 3;
+    B.big_n = B.ctl + 4;
+    B.hctr = B.ctl + 5;
     CK(dalloc(&B.iis_dii, N));
     CK(dalloc(&B.iis_dijpj, N));
     CK(dalloc(&B.iis_aii, N));
@@ -306,8 +313,6 @@ sphmp_status alloc_buffers(sphmp_ctx* c) {
     CK(dalloc(&B.osrc, N));
     CK(dalloc(&B.oct_start, 8 * G));
     CK(dalloc(&B.act, G));
-    CK(dalloc(&B.act_n, 1));
-    CK(cudaMemset(B.act_n, 0, sizeof(uint32_t)));
     CK(dalloc(&B.nact, 1));
     CK(dalloc(&B.frame, 1));
     CK(cudaMemset(B.nact, 0, sizeof(int32_t)));
@@ -332,6 +337,7 @@ sphmp_status alloc_buffers(sphmp_ctx* c) {
     CK(cudaMemset(B.mgridoff, 0, sizeof(int32_t) * G));
     CK(cudaMemset(B.mgridcnt, 0, sizeof(int32_t) * G));
     CK(cudaMemset(B.cstart, 0, sizeof(uint32_t) * (G + 2)));
+    CK(cudaMemset(B.ccount, 0, B.count_bytes));
     CK(cudaMemset(B.err, 0, sizeof(uint32_t)));
     CK(cudaMemset(B.color, 0, sizeof(float4) * N));
     CK(cudaMemset(B.bornid, 0, sizeof(int32_t) * N));
@@ -394,18 +400,18 @@ inline void swap_all(sphmp_ctx* c) {
 
 // Density pass: the bucket kernel when the internal order of this sort is
 // octant-grouped, otherwise the cell-search kernel; both write neighbour lists.
-void run_density(sphmp_ctx* c, cudaStream_t s) {
+void run_density(sphmp_ctx* c, bool fresh, cudaStream_t s) {
     const DevParams P = dev_params(c);
-    if (c->oct_valid) launch_density_oct(P, c->B, c->cur, s);
+    if (c->oct_valid) launch_density_oct(P, c->B, c->cur, fresh, s);
     else launch_density(P, c->B, c->cur, s);
     c->list_mode = 1;
     c->nbr_valid = true;
     c->ii_valid = false;  // one list storage
 }
 
-void run_force_drift(sphmp_ctx* c, bool force, bool drift, cudaStream_t s) {
+void run_force_drift(sphmp_ctx* c, bool force, bool drift, bool fresh, cudaStream_t s) {
     const DevParams P = dev_params(c);
-    launch_force_drift(P, c->B, c->cur, force, drift, s);
+    launch_force_drift(P, c->B, c->cur, force, drift, fresh, s);
 }
 
 // Optional event marks between the stages of a step (for sphmp_step_profile).
@@ -455,15 +461,17 @@ sphmp_status enqueue_step(sphmp_ctx* c, int schedule, StageTimer* T = nullptr, c
             c->n_stale = true;
             mark("emit");
         }
+        if (!c->counts_clear) launch_clear_counts(c->B, s);
         launch_hash(P, c->B, c->cur, s);
         mark("hash");
         c->hash_n = c->emit_on ? -1 : c->n;  // with an emitter the count is only known on the device
-        launch_cell_starts(P, c->B, s);
+        launch_cell_starts(P, c->B, true, true, s);
         mark("cell_starts");
         launch_cell_order(P, c->B, c->cur, s);
         mark("cell_order");
-        launch_rearrange(P, c->B, c->cur, false, s);
+        launch_rearrange(P, c->B, c->cur, false, true, s);
         mark("rearrange");
+        c->counts_clear = c->listed = true;
         swap_all(c);
         c->alpha_advanced = false;
         c->grid_valid = true;
@@ -471,7 +479,7 @@ sphmp_status enqueue_step(sphmp_ctx* c, int schedule, StageTimer* T = nullptr, c
         c->oct_built = false;
         c->nbr_valid = c->ii_valid = false;
         c->pos_sorted = true;
-        run_density(c, s);
+        run_density(c, true, s);
         mark("density");
     }
     const DevParams PL = dev_params(c);  // neighbour passes read the list
@@ -483,7 +491,7 @@ sphmp_status enqueue_step(sphmp_ctx* c, int schedule, StageTimer* T = nullptr, c
             launch_force_drift_features(PL, c->B, c->cur, c->lfeat, c->lids, vs, L->dt, s);
             mark("force_drift_features");
         } else {
-            run_force_drift(c, true, PL.multiphase != 0, s);
+            run_force_drift(c, true, PL.multiphase != 0, !reuse, s);
             mark("force_drift");
         }
         if (PL.st_on) {
@@ -504,7 +512,7 @@ sphmp_status enqueue_step(sphmp_ctx* c, int schedule, StageTimer* T = nullptr, c
         c->pos_sorted = false;
     } else {
         if (PL.multiphase) {
-            run_force_drift(c, false, true, s);
+            run_force_drift(c, false, true, !reuse, s);
             mark("drift");
             launch_alpha_advance(PL, c->B, c->cur, s);
             mark("alpha_advance");
@@ -517,7 +525,7 @@ sphmp_status enqueue_step(sphmp_ctx* c, int schedule, StageTimer* T = nullptr, c
             launch_force_projectu(PL, c->B, c->cur, c->cur[ALPHA] ^ 1, s);
             mark("force_projectu");
         } else {
-            run_force_drift(c, true, false, s);
+            run_force_drift(c, true, false, !reuse, s);
             mark("force");
         }
         if (PL.st_on) {
@@ -942,7 +950,9 @@ sphmp_status sphmp_upload_field(sphmp_ctx* c, int32_t field, const void* host, i
             DevParams P = dev_params(c);
             const int saved = P.n;
             P.n = 0;  // scan only: no scatter / cell sort
-            launch_grid_list(P, c->B, c->cur, c->stream);
+            c->counts_clear = false;
+            launch_hash(P, c->B, c->cur, c->stream);  // nothing to hash: clears the control words
+            launch_cell_starts(P, c->B, false, false, c->stream);
             P.n = saved;
             // cstart[G+1] must still be n
             const uint32_t nn = (uint32_t)c->n;
@@ -964,9 +974,12 @@ sphmp_status sphmp_upload_field(sphmp_ctx* c, int32_t field, const void* host, i
 sphmp_status sphmp_get_particle_index(sphmp_ctx* c) {
     if (sphmp_status st = need_ctx(c)) return st;
     if (sphmp_status st = refresh_n(c)) return st;
+    if (!c->counts_clear) launch_clear_counts(c->B, c->stream);
+    c->counts_clear = false;
     launch_hash(dev_params(c), c->B, c->cur, c->stream);
     CHECK_LAUNCH("GetParticleIndex");
     c->hash_n = c->n;
+    c->listed = false;
     c->grid_valid = false;
     c->nbr_valid = c->ii_valid = false;
     c->oct_valid = false;
@@ -980,7 +993,13 @@ sphmp_status sphmp_get_grid_list(sphmp_ctx* c) {
     // the scatter places every slot by its cell key and rank: both must exist for the current count
     if (c->hash_n != c->n)
         return fail(SPHMP_ERR_STATE, "no cell keys for the current %d particles (run GetParticleIndex first)", c->n);
-    launch_grid_list(dev_params(c), c->B, c->cur, c->stream);
+    // called again without a new hash, the words that the first call counted with are cleared here
+    if (c->listed) CK(cudaMemsetAsync(c->B.ctl, 0, sizeof(uint32_t) * kCtlWords, c->stream));
+    c->listed = true;
+    if (c->counts_clear) launch_recount(dev_params(c), c->B, c->stream);  // a step's sort has cleared them
+    c->counts_clear = false;
+    launch_cell_starts(dev_params(c), c->B, true, false, c->stream);
+    launch_cell_order(dev_params(c), c->B, c->cur, c->stream);
     CHECK_LAUNCH("GetGridList");
     c->oct_built = true;
     return SPHMP_OK;
@@ -990,7 +1009,7 @@ sphmp_status sphmp_rearrange_data(sphmp_ctx* c) {
     if (sphmp_status st = need_ctx(c)) return st;
     // without this library's grid list (sort arrays uploaded by the caller) the
     // new internal order is the plain sorted slot order
-    launch_rearrange(dev_params(c), c->B, c->cur, !c->oct_built, c->stream);
+    launch_rearrange(dev_params(c), c->B, c->cur, !c->oct_built, false, c->stream);
     CHECK_LAUNCH("RearrageData");
     swap_all(c);
     c->alpha_advanced = false;
@@ -1014,7 +1033,7 @@ sphmp_status sphmp_compute_boundary_density(sphmp_ctx* c) {
 sphmp_status sphmp_compute_pressure(sphmp_ctx* c) {
     if (sphmp_status st = need_ctx(c)) return st;
     if (sphmp_status st = need_grid(c)) return st;
-    run_density(c, c->stream);
+    run_density(c, false, c->stream);
     CHECK_LAUNCH("MfComputePressure");
     return SPHMP_OK;
 }
@@ -1022,7 +1041,7 @@ sphmp_status sphmp_compute_pressure(sphmp_ctx* c) {
 sphmp_status sphmp_compute_drift_vel(sphmp_ctx* c) {
     if (sphmp_status st = need_ctx(c)) return st;
     if (sphmp_status st = need_grid(c)) return st;
-    run_force_drift(c, false, true, c->stream);
+    run_force_drift(c, false, true, false, c->stream);
     CHECK_LAUNCH("MfComputeDriftVel");
     return SPHMP_OK;
 }
@@ -1051,7 +1070,7 @@ sphmp_status sphmp_compute_force(sphmp_ctx* c) {
     if (sphmp_status st = need_ctx(c)) return st;
     if (sphmp_status st = need_grid(c)) return st;
     const DevParams P = dev_params(c);
-    run_force_drift(c, true, false, c->stream);
+    run_force_drift(c, true, false, false, c->stream);
     if (P.st_on) launch_surface_tension(P, c->B, c->cur, c->stream);
     CHECK_LAUNCH("MfComputeForce");
     return SPHMP_OK;
@@ -1343,6 +1362,8 @@ sphmp_status sphmp_step(sphmp_ctx* c, int32_t nsteps, int32_t schedule, int32_t 
         if (!c->graph || c->graph_n != key || c->graph_schedule != schedule ||
             memcmp(c->graph_cur, c->cur, sizeof(c->graph_cur)) != 0) {
             drop_graph(c);
+            if (!c->counts_clear) launch_clear_counts(c->B, c->stream);  // before the capture: a captured step leaves them clear
+            c->counts_clear = true;
             cudaStream_t cap = c->stream;
             CK(cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal));
             int saved[kNumFloat4Fields];
@@ -1370,6 +1391,8 @@ sphmp_status sphmp_step(sphmp_ctx* c, int32_t nsteps, int32_t schedule, int32_t 
             c->graph_schedule = schedule;
             memcpy(c->graph_cur, c->cur, sizeof(c->graph_cur));
         }
+        if (!c->counts_clear) launch_clear_counts(c->B, c->stream);
+        c->counts_clear = c->listed = true;
         for (int t = 0; t + per <= nsteps; t += per) CK(cudaGraphLaunch(c->graph, c->stream));
         if (c->emit_on) c->n_stale = true;
         // the state a step leaves behind (as enqueue_step sets it)
@@ -1549,7 +1572,9 @@ static sphmp_status clone_state(sphmp_ctx* dst, sphmp_ctx* src) {
     CK(cp(b.mgridcnt, a.mgridcnt, sizeof(int32_t) * G));
     CK(cp(b.key, a.key, sizeof(uint32_t) * N));
     CK(cp(b.octk, a.octk, sizeof(uint8_t) * N));
-    CK(cp(b.ccount, a.ccount, sizeof(uint32_t) * (G + 1)));
+    CK(cp(b.ccount, a.ccount, a.count_bytes));
+    CK(cp(b.uchunk, a.uchunk, sizeof(uint32_t) * (N / kHashBlock + 2)));
+    CK(cp(b.arank, a.arank, sizeof(uint32_t) * N));
     CK(cp(b.cstart, a.cstart, sizeof(uint32_t) * (G + 2)));
     CK(cp(b.cend, a.cend, sizeof(uint32_t) * G));
     CK(cp(b.opos, a.opos, sizeof(uint32_t) * N));
@@ -1557,7 +1582,8 @@ static sphmp_status clone_state(sphmp_ctx* dst, sphmp_ctx* src) {
     CK(cp(b.osrc, a.osrc, sizeof(uint32_t) * N));
     CK(cp(b.oct_start, a.oct_start, sizeof(uint32_t) * 8 * G));
     CK(cp(b.act, a.act, sizeof(uint32_t) * G));
-    CK(cp(b.act_n, a.act_n, sizeof(uint32_t)));
+    CK(cp(b.ctl, a.ctl, sizeof(uint32_t) * kCtlWords));
+    CK(cp(b.wq, a.wq, sizeof(uint2) * (N / kBucketWindowMin + 16)));
     CK(cp(b.nact, a.nact, sizeof(int32_t)));
     CK(cp(b.frame, a.frame, sizeof(int32_t)));
     CK(cp(b.color, a.color, sizeof(float4) * N));
@@ -1574,6 +1600,8 @@ static sphmp_status clone_state(sphmp_ctx* dst, sphmp_ctx* src) {
     dst->oct_built = src->oct_built;
     dst->pos_sorted = src->pos_sorted;
     dst->hash_n = src->hash_n;
+    dst->listed = src->listed;
+    dst->counts_clear = src->counts_clear;
     dst->list_mode = src->list_mode;
     dst->nbr_valid = dst->ii_valid = false;
     dst->n_stale = false;

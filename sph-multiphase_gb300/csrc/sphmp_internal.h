@@ -37,6 +37,8 @@ constexpr uint32_t kUndef = 0xFFFFFFFFu;
 constexpr int kHashBlock = 256;       // threads per hash block (= one chunk for out-of-grid ranks)
 constexpr int kScanBlock = 1024;      // threads per scan block
 constexpr int kScanItems = 4;         // items per thread in the scan
+constexpr uint32_t kScanPer = kScanBlock * kScanItems;  // cells per scan block
+constexpr int kCtlWords = 16;         // control words of the sort and the passes (DevBuffers::ctl)
 constexpr int kWarpSortMax = 256;     // cells up to this size are sorted by one warp
 constexpr int kCtaSortMax = 8192;     // larger cells up to this size are sorted by one CTA
 constexpr int kNumFloat4Fields = 5;   // pos4, vel4, vev4, alpha4, aprev4
@@ -120,14 +122,22 @@ struct DevBuffers {
     uint8_t* octk;      // [cap] octant (h-subcell inside the cell) per slot, in-grid slots only
     uint32_t* arank;    // [cap] rank inside the bin (atomic order; exact for out-of-grid)
     uint32_t* sidx;     // [cap] scatter target (pre-sort slots grouped by cell)
-    uint32_t* ccount;   // [G + 1] histogram, bin G = out-of-grid
+    // One allocation of count_bytes, all zero between a step's sort and the next hash (the
+    // steps' sorts clear what they have read; other calls leave it to a memset before the next hash):
+    uint32_t* ccount;   // [G + 4] particles per cell
+    uint32_t* bsum;     // [G / kScanPer + 2] particles per kScanPer cells (linear order)
+    uint32_t* usum;     // [cap / kHashBlock^2 + 2] out-of-grid slots per kHashBlock hash chunks
+    size_t count_bytes;
     uint32_t* cstart;   // [G + 2] exclusive scan of ccount in the cell order; cstart[G] = in-grid count,
                         // cstart[G+1] = n
     uint32_t* cend;     // [G] end of each cell's range (cstart[c + 1] in the linear order only)
     uint32_t* corder;   // [G] cells in Z-order (the scan order of the Morton mode)
-    uint32_t* bsum;     // [nblocks] scan block sums
-    uint32_t* uchunk;   // [cap / kHashBlock + 1] out-of-grid count per hash chunk, scanned in place
-    uint32_t* big;      // [cap / (kWarpSortMax+1) + 2]: big[0] = count, then big cell ids
+    uint32_t* uchunk;   // [cap / kHashBlock + 2] out-of-grid count per hash chunk
+    uint32_t* big;      // [cap / (kWarpSortMax+1) + 2] cells above the warp sort's size
+    // Control words, one allocation of kCtlWords cleared by the hash: the pointers to
+    // single words below (act_n, wq_n, hq_n, dctr, hctr, big_n) point into it
+    uint32_t* ctl;
+    uint32_t* big_n;    // [1] entries in big
     float4* color;      // [cap] per origin
     int32_t* bornid;    // [cap] per origin
     float* mass_raw;    // [cap] per origin
@@ -141,10 +151,10 @@ struct DevBuffers {
     uint32_t* dctr;     // [1] work counter of the bucket density kernel
     uint2* wq;          // [cap / kBucketWindowMin + 16] member windows after the first of large buckets:
                         // x = bucket (cell * 8 + octant), y = first member (internal index)
-    uint32_t* wq_n;     // [1] entries in wq (cleared by the scan, filled by the cell sort)
-    uint32_t* hq;       // [cap] heavy particles (internal index), filled by the list expansion
-    uint32_t* hq_n;     // [1] entries in hq (cleared by the scan)
-    uint32_t* hctr;     // [2] work counters over hq of the force and the alpha pass
+    uint32_t* wq_n;     // [1] entries in wq (filled by the cell sort)
+    uint32_t* hq;       // [cap] heavy particles (internal index), filled by the density pass
+    uint32_t* hq_n;     // [1] entries in hq
+    uint32_t* hctr;     // [3] work counters over hq of the drift (or force + drift), force and alpha passes
     // IISPH step (sphmp_iisph.cu): d_ii, sum_j d_ij p_j, d_ii p_l + sum_j d_ij p_j (float4,
     // w unused), a_ii, the predicted density, the pressure iterate p_l, p_l m / rho^2
     float4* iis_dii;
@@ -203,22 +213,31 @@ sphmp_status record_error(sphmp_status st, const char* msg);
 
 // ---- launchers (sphmp_kernels.cu) ----
 // All take the current double-buffer selectors in `cur` (one per Field4).
+// zero the counts the hash adds to (DevBuffers::ccount)
+void launch_clear_counts(const DevBuffers& B, cudaStream_t s);
+// cell keys, ranks and counts (the counts zero before), control words cleared
 void launch_hash(const DevParams& P, const DevBuffers& B, const int* cur, cudaStream_t s);
-// (reads the pre-sort positions pos4[cur[POS]] to build the next internal order)
-void launch_grid_list(const DevParams& P, const DevBuffers& B, const int* cur, cudaStream_t s);
-// the two halves of launch_grid_list: cell starts (histogram scan), then the
-// scatter, the per-cell stable ordering and the per-cell octant order
-void launch_cell_starts(const DevParams& P, const DevBuffers& B, cudaStream_t s);
+// the counts again from the last hash's keys, after they were cleared
+void launch_recount(const DevParams& P, const DevBuffers& B, cudaStream_t s);
+// GetGridList in two halves: cell starts (a scan of the counts, which the hash
+// left with `hashed`; with `clear` the counts are zeroed), then the scatter, the
+// per-cell stable ordering and the per-cell octant order (which reads the
+// pre-sort positions pos4[cur[POS]] to build the next internal order)
+void launch_cell_starts(const DevParams& P, const DevBuffers& B, bool hashed, bool clear, cudaStream_t s);
 void launch_cell_order(const DevParams& P, const DevBuffers& B, const int* cur, cudaStream_t s);
 // move every particle to its new internal index (osrc) and update opos; with
 // `slot_order`, the new internal order is the reference's sorted slot order
-// (for a rearrange that did not follow this library's grid list)
-void launch_rearrange(const DevParams& P, const DevBuffers& B, const int* cur, bool slot_order, cudaStream_t s);
+// (for a rearrange that did not follow this library's grid list); with `clear`
+// the rest of the counts is zeroed
+void launch_rearrange(const DevParams& P, const DevBuffers& B, const int* cur, bool slot_order, bool clear,
+                      cudaStream_t s);
 void launch_boundary_volume(const DevParams& P, const DevBuffers& B, const int* cur, cudaStream_t s);
 void launch_density(const DevParams& P, const DevBuffers& B, const int* cur, cudaStream_t s);
-// octant-order density (needs the octant order of this sort); writes slot lists
-void launch_density_oct(const DevParams& P, const DevBuffers& B, const int* cur, cudaStream_t s);
-void launch_force_drift(const DevParams& P, const DevBuffers& B, const int* cur, bool force, bool drift,
+// octant-order density (needs the octant order of this sort); writes slot lists.
+// `fresh` here and below: the control words the pass counts with are still as the
+// hash of this step cleared them (otherwise they are cleared first)
+void launch_density_oct(const DevParams& P, const DevBuffers& B, const int* cur, bool fresh, cudaStream_t s);
+void launch_force_drift(const DevParams& P, const DevBuffers& B, const int* cur, bool force, bool drift, bool fresh,
                         cudaStream_t s);
 void launch_surface_tension(const DevParams& P, const DevBuffers& B, const int* cur, cudaStream_t s);
 // project-U force: start-of-step fractions in alpha4[pre], rest densities in alpha4[cur[ALPHA]]
@@ -229,7 +248,7 @@ void launch_alpha_advance(const DevParams& P, const DevBuffers& B, const int* cu
 void launch_correction(const DevParams& P, const DevBuffers& B, const int* cur, int pre, cudaStream_t s);
 // advance in place on the cur buffers
 void launch_advance(const DevParams& P, const DevBuffers& B, const int* cur, cudaStream_t s);
-// fused alpha + correction + advance: reads cur, writes cur^1 for all five float4 fields
+// fused alpha + correction + advance of a step: reads cur, writes cur^1 for all five float4 fields
 void launch_pass_c(const DevParams& P, const DevBuffers& B, const int* cur, cudaStream_t s);
 void launch_conservation(const DevParams& P, const DevBuffers& B, const int* cur, cudaStream_t s);
 // IISPH step (sphmp_iisph.cu): density (densp.x = rho, and the index lists in nbr /

@@ -36,13 +36,17 @@ using namespace dev;
 
 // One block = one chunk of kHashBlock slots. In-grid slots take a rank inside
 // their cell from a warp-aggregated atomic (the order is fixed later by the
-// cell sort); out-of-grid slots get their exact rank inside the chunk, and the
-// chunk totals are scanned later, which places them in slot order.
+// cell sort) and are counted per kScanPer cells as well, so that the scan of the
+// cell counts needs no pass of its own for its blocks' sums; out-of-grid slots
+// get their exact rank inside the chunk, and the chunk totals, also summed per
+// kHashBlock chunks, place them in slot order. The first block clears the
+// control words of the sort and the passes after it.
 __global__ void __launch_bounds__(kHashBlock) k_hash(const __grid_constant__ DevParams P,
                                                      const __grid_constant__ DevBuffers B,
                                                      const float4* __restrict__ pos4) {
     __shared__ uint32_t wcount[kHashBlock / 32];
     const int i = blockIdx.x * kHashBlock + threadIdx.x;
+    if (i < kCtlWords) B.ctl[i] = 0u;
     const bool valid = i < active_n(B);
     uint32_t key = kUndef;
     if (valid) {
@@ -53,8 +57,33 @@ __global__ void __launch_bounds__(kHashBlock) k_hash(const __grid_constant__ Dev
         if (key != kUndef) B.octk[i] = (uint8_t)octant_of(P, p);  // for the per-cell octant order
     }
     const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
+    const bool in = valid && key != kUndef;
+    const unsigned im = __ballot_sync(0xffffffffu, in);
+    if (in) {
+        const unsigned peers = __match_any_sync(im, key);
+        const int leader = __ffs(peers) - 1;
+        uint32_t base = 0;
+        if ((int)lane == leader) base = atomicAdd(&B.ccount[key], (uint32_t)__popc(peers));
+        base = __shfl_sync(peers, base, leader);
+        B.arank[i] = base + __popc(peers & lanemask_lt());
+    }
+    // The Morton order scans the cells in another sequence (k_scan_reduce). Slots are
+    // nearly in cell order, so a block mostly counts into one sum, with one atomic
+    // (one per warp took 20 us at 1.3 M slots: they all go to the same few words).
+    if (!P.morton) {
+        __shared__ uint32_t first;
+        if (threadIdx.x == 0) first = in ? key / kScanPer : 0u;
+        __syncthreads();
+        const int same = __syncthreads_count((int)(in && key / kScanPer == first));
+        if (threadIdx.x == 0 && same) atomicAdd(&B.bsum[first], (uint32_t)same);
+        if (in && key / kScanPer != first) atomicAdd(&B.bsum[key / kScanPer], 1u);
+    }
     const bool und = valid && key == kUndef;
     const unsigned ub = __ballot_sync(0xffffffffu, und);
+    if (!__syncthreads_or((int)und)) {  // the usual case
+        if (threadIdx.x == 0) B.uchunk[blockIdx.x] = 0u;
+        return;
+    }
     if (lane == 0) wcount[warp] = __popc(ub);
     __syncthreads();
     if (warp == 0) {
@@ -67,20 +96,24 @@ __global__ void __launch_bounds__(kHashBlock) k_hash(const __grid_constant__ Dev
             if ((int)lane >= o) x += y;
         }
         if ((int)lane < nw) wcount[lane] = x - v;
-        if ((int)lane == nw - 1) B.uchunk[blockIdx.x] = x;
+        if ((int)lane == nw - 1) {
+            B.uchunk[blockIdx.x] = x;
+            atomicAdd(&B.usum[blockIdx.x / kHashBlock], x);
+        }
     }
     __syncthreads();
     if (und) B.arank[i] = wcount[warp] + __popc(ub & lanemask_lt());
-    const bool in = valid && key != kUndef;
-    const unsigned im = __ballot_sync(0xffffffffu, in);
-    if (in) {
-        const unsigned peers = __match_any_sync(im, key);
-        const int leader = __ffs(peers) - 1;
-        uint32_t base = 0;
-        if ((int)lane == leader) base = atomicAdd(&B.ccount[key], (uint32_t)__popc(peers));
-        base = __shfl_sync(peers, base, leader);
-        B.arank[i] = base + __popc(peers & lanemask_lt());
-    }
+}
+
+// The counts again from the keys of the last hash, for a GetGridList after a step's
+// sort has cleared them.
+__global__ void __launch_bounds__(kHashBlock) k_recount(const __grid_constant__ DevParams P,
+                                                        const __grid_constant__ DevBuffers B) {
+    const int i = blockIdx.x * kHashBlock + threadIdx.x;
+    if (threadIdx.x == 0 && B.uchunk[blockIdx.x]) atomicAdd(&B.usum[blockIdx.x / kHashBlock], B.uchunk[blockIdx.x]);
+    if (i >= active_n(B) || B.key[i] == kUndef) return;
+    atomicAdd(&B.ccount[B.key[i]], 1u);
+    if (!P.morton) atomicAdd(&B.bsum[B.key[i] / kScanPer], 1u);
 }
 
 // ---------------------------------------------------------------------------
@@ -88,28 +121,29 @@ __global__ void __launch_bounds__(kHashBlock) k_hash(const __grid_constant__ Dev
 // ---------------------------------------------------------------------------
 
 // Exclusive scan of one value per thread across a 1024-thread block.
-__device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t* total) {
-    __shared__ uint32_t ws[32];
+template <class T>
+__device__ __forceinline__ T block_excl_scan(T v, T* total) {
+    __shared__ T ws[32];
     const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
-    uint32_t x = v;
+    T x = v;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+        T y = __shfl_up_sync(0xffffffffu, x, o);
         if ((int)lane >= o) x += y;
     }
     if (lane == 31) ws[warp] = x;
     __syncthreads();
     if (warp == 0) {
-        uint32_t w = ws[lane];
+        T w = ws[lane];
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-            uint32_t y = __shfl_up_sync(0xffffffffu, w, o);
+            T y = __shfl_up_sync(0xffffffffu, w, o);
             if ((int)lane >= o) w += y;
         }
         ws[lane] = w;
     }
     __syncthreads();
-    const uint32_t off = warp ? ws[warp - 1] : 0u;
+    const T off = warp ? ws[warp - 1] : T(0);
     *total = ws[31];
     __syncthreads();
     return off + x - v;
@@ -136,7 +170,8 @@ __device__ __forceinline__ void load4_cells(const DevParams& P, const DevBuffers
     for (int k = 0; k < 4; k++) v[k] = idx + k < P.G ? B.ccount[B.corder[idx + k]] : 0u;
 }
 
-// Phase A: block sums of the cell histogram.
+// Block sums of the cell counts in scan order, where the hash has not left them
+// (the Morton order; counts uploaded by the caller).
 __global__ void __launch_bounds__(kScanBlock) k_scan_reduce(const __grid_constant__ DevParams P,
                                                             const __grid_constant__ DevBuffers B) {
     const int idx = (blockIdx.x * kScanBlock + threadIdx.x) * kScanItems;
@@ -147,48 +182,36 @@ __global__ void __launch_bounds__(kScanBlock) k_scan_reduce(const __grid_constan
     if (threadIdx.x == 0) B.bsum[blockIdx.x] = total;
 }
 
-// Phase B: one block scans the block sums and the out-of-grid chunk counts.
-__global__ void __launch_bounds__(kScanBlock) k_scan_top(const __grid_constant__ DevParams P,
-                                                         const __grid_constant__ DevBuffers B, int nblocks,
-                                                         int nchunks) {
-    uint32_t carry = 0;
-    for (int base = 0; base < nblocks; base += kScanBlock) {
-        const int k = base + threadIdx.x;
-        const uint32_t v = k < nblocks ? B.bsum[k] : 0u;
-        uint32_t total;
-        const uint32_t e = block_excl_scan(v, &total);
-        if (k < nblocks) B.bsum[k] = carry + e;
-        carry += total;
-    }
-    const uint32_t nin = carry;
-    carry = 0;
-    for (int base = 0; base < nchunks; base += kScanBlock) {
-        const int k = base + threadIdx.x;
-        const uint32_t v = k < nchunks ? B.uchunk[k] : 0u;
-        uint32_t total;
-        const uint32_t e = block_excl_scan(v, &total);
-        if (k < nchunks) B.uchunk[k] = carry + e;
-        carry += total;
-    }
-    if (threadIdx.x == 0) {
-        B.cstart[P.G] = nin;
-        B.cstart[P.G + 1] = (uint32_t)active_n(B);
-        B.big[0] = 0u;
-        *B.act_n = 0u;
-        *B.wq_n = 0u;
-        *B.hq_n = 0u;
-    }
-}
-
-// Phase C: cell starts, the reference's mgridoff / mgridcnt, and the list of
-// cells too large for the warp sort.
-__global__ void __launch_bounds__(kScanBlock) k_scan_apply(const __grid_constant__ DevParams P,
-                                                           const __grid_constant__ DevBuffers B) {
+// Cell starts, the reference's mgridoff / mgridcnt, the list of occupied cells and
+// the list of cells too large for the warp sort, in one pass: every block adds up
+// the sums of the blocks before it (a few dozen words) and scans its kScanPer
+// counts together with their occupied flags (counts in the low 40 bits, flags
+// above). `clear`: the counts are zeroed for the next hash. (Three kernels, one
+// of them a single block over the block sums and the chunks' out-of-grid counts,
+// took 13 us at 11 K particles and 21 us at 1.3 M.)
+__global__ void __launch_bounds__(kScanBlock) k_scan(const __grid_constant__ DevParams P,
+                                                     const __grid_constant__ DevBuffers B, int clear) {
+    __shared__ uint32_t act_base;
+    uint32_t before = 0;
+    for (unsigned k = threadIdx.x; k < blockIdx.x; k += kScanBlock) before += B.bsum[k];
+    uint32_t run;
+    block_excl_scan(before, &run);
     const int idx = (blockIdx.x * kScanBlock + threadIdx.x) * kScanItems;
     uint32_t v[4];
     load4_cells(P, B, idx, v);
-    uint32_t total;
-    uint32_t run = B.bsum[blockIdx.x] + block_excl_scan(v[0] + v[1] + v[2] + v[3], &total);
+    uint64_t sum = 0;
+#pragma unroll
+    for (int k = 0; k < 4; k++) sum += (uint64_t)v[k] + (v[k] ? 1ull << 40 : 0ull);
+    uint64_t total;
+    const uint64_t excl = block_excl_scan(sum, &total);
+    if (threadIdx.x == 0) act_base = total >> 40 ? atomicAdd(B.act_n, (uint32_t)(total >> 40)) : 0u;
+    __syncthreads();
+    uint32_t at = act_base + (uint32_t)(excl >> 40);
+    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) {
+        B.cstart[P.G] = run + (uint32_t)total;
+        B.cstart[P.G + 1] = (uint32_t)active_n(B);
+    }
+    run += (uint32_t)excl;
 #pragma unroll
     for (int k = 0; k < 4; k++) {
         if (idx + k < P.G) {
@@ -197,14 +220,14 @@ __global__ void __launch_bounds__(kScanBlock) k_scan_apply(const __grid_constant
             B.cend[c] = run + v[k];
             B.mgridoff[c] = v[k] ? (int32_t)run : 0;
             B.mgridcnt[c] = (int32_t)v[k];
-            if (v[k]) B.act[atomicAdd(B.act_n, 1u)] = (uint32_t)c;
+            if (clear) B.ccount[c] = 0u;
+            if (v[k]) B.act[at++] = (uint32_t)c;
             if (v[k] > (uint32_t)kWarpSortMax) {
                 if (v[k] > (uint32_t)kCtaSortMax) {
                     set_err(B, kErrCellOverflow);  // left unsorted; keep its octant ranges in bounds
                     for (int b = 0; b < 8; b++) B.oct_start[(size_t)c * 8 + b] = run;
                 } else {
-                    const uint32_t slot = atomicAdd(&B.big[0], 1u);
-                    B.big[1 + slot] = (uint32_t)c;
+                    B.big[atomicAdd(B.big_n, 1u)] = (uint32_t)c;
                 }
             }
         }
@@ -216,22 +239,34 @@ __global__ void __launch_bounds__(kScanBlock) k_scan_apply(const __grid_constant
 // Scatter + per-cell stable order (GetGridListCUDA, part 2)
 // ---------------------------------------------------------------------------
 
+static_assert(kThreads == kHashBlock, "a scatter block holds one chunk of the hash");
+
 __global__ void __launch_bounds__(kThreads) k_scatter(const __grid_constant__ DevParams P,
                                                       const __grid_constant__ DevBuffers B) {
+    __shared__ uint32_t part[kThreads / 32];
     const int i = blockIdx.x * kThreads + threadIdx.x;
-    if (i >= active_n(B)) return;
-    const uint32_t key = B.key[i];
-    const uint32_t r = B.arank[i];
-    if (key != kUndef) {
-        B.sidx[B.cstart[key] + r] = (uint32_t)i;
-    } else {
-        const uint32_t d = B.cstart[P.G] + B.uchunk[i / kHashBlock] + r;
-        B.midsort[d] = (uint32_t)i;
-        B.mgcell[d] = kUndef;
-        B.mgndx[d] = kUndef;
-        B.osrc[d] = B.opos[i];  // out-of-grid particles keep slot order at the end
-        B.oidx[d] = d;
-    }
+    const bool valid = i < active_n(B);
+    const uint32_t key = valid ? B.key[i] : 0u;
+    if (valid && key != kUndef) B.sidx[B.cstart[key] + B.arank[i]] = (uint32_t)i;
+    const bool und = valid && key == kUndef;
+    if (!__syncthreads_or((int)und)) return;
+    // out-of-grid slots in the chunks before this one: whole groups of chunks, then this group's
+    uint32_t v = 0;
+    const unsigned grp = blockIdx.x / kHashBlock;
+    for (unsigned k = threadIdx.x; k < grp; k += kThreads) v += B.usum[k];
+    if (grp * kHashBlock + threadIdx.x < blockIdx.x) v += B.uchunk[grp * kHashBlock + threadIdx.x];
+    v = __reduce_add_sync(0xffffffffu, v);
+    if (lane_id() == 0) part[threadIdx.x >> 5] = v;
+    __syncthreads();
+    if (!und) return;
+    uint32_t d = B.cstart[P.G] + B.arank[i];
+#pragma unroll
+    for (int w = 0; w < kThreads / 32; w++) d += part[w];
+    B.midsort[d] = (uint32_t)i;
+    B.mgcell[d] = kUndef;
+    B.mgndx[d] = kUndef;
+    B.osrc[d] = B.opos[i];  // out-of-grid particles keep slot order at the end
+    B.oidx[d] = d;
 }
 
 // Bitonic sort of 32*E keys held E per lane (element index = lane*E + r),
@@ -404,9 +439,9 @@ __global__ void __launch_bounds__(1024) k_big_cell_sort(const __grid_constant__ 
                                                         const __grid_constant__ DevBuffers B,
                                                         const float4* __restrict__ pos_in) {
     __shared__ uint32_t sm[kCtaSortMax];
-    const uint32_t nbig = B.big[0];
+    const uint32_t nbig = *B.big_n;
     for (uint32_t b = blockIdx.x; b < nbig; b += gridDim.x) {
-        const uint32_t c = B.big[1 + b];
+        const uint32_t c = B.big[b];
         const uint32_t start = B.cstart[c];
         const uint32_t cnt = B.cend[c] - start;
         uint32_t M = 1;
@@ -454,9 +489,13 @@ __global__ void __launch_bounds__(1024) k_big_cell_sort(const __grid_constant__ 
 // cell order, which reads the old map, and this one).
 __global__ void __launch_bounds__(kThreads) k_rearrange(const __grid_constant__ DevParams P,
                                                         const __grid_constant__ DevBuffers B,
-                                                        const __grid_constant__ F4Set S) {
+                                                        const __grid_constant__ F4Set S, int clear) {
     const int o = blockIdx.x * kThreads + threadIdx.x;
     const int n = active_n(B);
+    if (clear) {  // the sums the hash adds to, for the next one
+        for (int k = o; k <= P.G / (int)kScanPer; k += (int)gridDim.x * kThreads) B.bsum[k] = 0u;
+        for (int k = o; k <= (int)gridDim.x / kHashBlock; k += (int)gridDim.x * kThreads) B.usum[k] = 0u;
+    }
     if (o >= n) return;
     uint32_t src = B.osrc[o];
     if (src >= (uint32_t)n) src = o;  // only after a cell-overflow error (flagged by the scan)
@@ -554,7 +593,8 @@ __global__ void __launch_bounds__(kThreads) k_boundary_volume_store(const __grid
 // candidate sequence. A warp takes one window of up to P.bwin (<= 32) members of a
 // bucket and stages the bucket's candidates in shared memory, 256 at a time. The
 // window's n fluid members share the lanes out: 32 / n lanes a member, each
-// testing every 32 / n-th pair of candidates in packed FP32 arithmetic, adding its density terms and appending the hits to a
+// testing its share of the sequence two candidates at a time in packed FP32
+// arithmetic, adding its density terms and appending the hits to a
 // list of its own in shared memory. The lanes' lists of a member are then joined
 // and written as rows of four indices. Bound by shared-memory accesses (78 % of
 // the L1 data pipe) and the issue slots (64 %): about 14 instructions a candidate
@@ -562,7 +602,9 @@ __global__ void __launch_bounds__(kThreads) k_boundary_volume_store(const __grid
 // hold the candidates and walked the members, with ballots and selects per 32
 // candidates and a shuffle reduction per member, and left mask words that a
 // second kernel expanded: 174 M warp instructions at 442 K fluid particles
-// against 117 M here; 404 against 338 us at 1.05 M, 33 against 16 us at 4 K.) A lane adds at most 16
+// against 117 M here; 404 against 350 us at 1.05 M, 33 against 16 us at 4 K. Shares
+// that interleave measured 338 us, but put the lists out of sequence order, which
+// cost the force and alpha passes 27 us of cache misses.) A lane adds at most 16
 // pairs of terms before they go to its Kahan-compensated sum, and the lanes of a
 // member are added pairwise (a scan). Warps take work items from a shared counter (their
 // costs differ by orders of magnitude): the first window of every bucket, then
@@ -781,7 +823,10 @@ __global__ void __launch_bounds__(kDensThreads, 7) k_density_bucket(const __grid
             }
             const bool any_bnd = __any_sync(0xffffffffu, wmin < 0.f);
             __syncwarp();
+            // this lane's pairs, an odd number (lanes in step then read different banks)
             const uint32_t npairs = (n + 1u) >> 1;
+            const uint32_t each = (uint32_t)__fdividef((float)(npairs + L) - 0.5f, (float)L) | 1u;
+            const uint32_t p0 = min(npairs, share * each), p1 = min(npairs, p0 + each);
             auto dist2 = [&](const float4 a, const float4 b) {
                 float2 dx = __ffma2_rn(make_float2(a.x, a.y), NEG1, PX), dy = __ffma2_rn(make_float2(a.z, a.w), NEG1, PY),
                        dz = __ffma2_rn(make_float2(b.x, b.y), NEG1, PZ);
@@ -795,17 +840,17 @@ __global__ void __launch_bounds__(kDensThreads, 7) k_density_bucket(const __grid
             // a neighbour: within the list radius and not at the same place (every consumer of
             // the lists skips r = 0), so not the member itself
             auto near = [&](float d2) { return d2 < r2list && d2 > 0.f; };
-            // this lane's pairs. With boundary candidates in the block or without (the usual
+            // the walk over them. With boundary candidates in the block or without (the usual
             // case): the weight of a candidate is its mass, or rho0 V for a boundary particle.
             uint32_t hits = 0;
             auto walk = [&](auto with_boundary, auto bounded) {
                 constexpr bool BND = decltype(with_boundary)::value;
-                uint32_t p = share;
-                while (p < npairs) {
+                uint32_t p = p0;
+                while (p < p1) {
                     float2 acc = make_float2(0.f, 0.f);
-                    const uint32_t end = min(npairs, p + 16u * L);
+                    const uint32_t end = min(p1, p + 16u);
 #pragma unroll 2
-                    for (; p < end; p += L) {
+                    for (; p < end; p++) {
                         const float4 a = W.pxy[p], b = W.pzw[p];
                         const float2 d2 = dist2(a, b);
                         float2 cc = __ffma2_rn(d2, NEG1, R2);  // r2 - d2, rounded once
@@ -829,7 +874,7 @@ __global__ void __launch_bounds__(kDensThreads, 7) k_density_bucket(const __grid
                 }
             };
             if (live) {
-                // four lanes or more a member: at most 64 candidates each, the row holds them all
+                // four lanes or more a member: at most 33 pairs each, the row holds them all
                 if (L >= 4u) {
                     if (any_bnd) walk(std::true_type{}, std::false_type{});
                     else walk(std::false_type{}, std::false_type{});
@@ -866,7 +911,7 @@ __global__ void __launch_bounds__(kDensThreads, 7) k_density_bucket(const __grid
                 }
             } else if (live) {  // too many for the rows: found again, stored one by one
                 uint32_t k = count + before;
-                for (uint32_t p = share; p < npairs; p += L) {
+                for (uint32_t p = p0; p < p1; p++) {
                     const float2 d2 = dist2(W.pxy[p], W.pzw[p]);
                     if (near(d2.x)) {
                         if (k < (uint32_t)kMaxNbr) B.nbr[nbr_at(cap, t, k)] = W.cidx[2u * p];
@@ -995,6 +1040,11 @@ __device__ __forceinline__ void force_drift_warp(const DevParams& P, const DevBu
 // particles from the queue (whole warp per particle) while any are left. With
 // both, it also writes every in-grid particle's neighbour record for the fused
 // alpha pass.
+// The work counter (hctr) of each pass over the queue of heavy particles.
+template <bool FORCE, bool DRIFT>
+constexpr int kHeavyCounter = FORCE && !DRIFT ? 1 : 0;
+constexpr int kHeavyCounterAlpha = 2;
+
 template <bool FORCE, bool DRIFT, int NP, int L>
 __global__ void __launch_bounds__(kThreads, 4) k_force_drift(const __grid_constant__ DevParams P,
                                                              const __grid_constant__ DevBuffers B,
@@ -1006,7 +1056,8 @@ __global__ void __launch_bounds__(kThreads, 4) k_force_drift(const __grid_consta
     if (P.list_mode != 0) {
         const unsigned lane = lane_id();
         const uint32_t nh = *B.hq_n;
-        for (uint32_t h = next_item(&B.hctr[0], nh, lane); h < nh; h = next_item(&B.hctr[0], nh, lane))
+        uint32_t* ctr = &B.hctr[kHeavyCounter<FORCE, DRIFT>];
+        for (uint32_t h = next_item(ctr, nh, lane); h < nh; h = next_item(ctr, nh, lane))
             force_drift_warp<FORCE, DRIFT, NP>(P, B, pos4, vel4, alpha4, aprev4, vev4, (int)B.hq[h]);
     }
     const int s = (int)((blockIdx.x * (unsigned)kThreads + threadIdx.x) / L);
@@ -1339,7 +1390,8 @@ __global__ void __launch_bounds__(kThreads, 4) k_pass_c(const __grid_constant__ 
     if (MP && P.list_mode != 0) {
         const unsigned lane = lane_id();
         const uint32_t nh = *B.hq_n;
-        for (uint32_t h = next_item(&B.hctr[1], nh, lane); h < nh; h = next_item(&B.hctr[1], nh, lane)) {
+        uint32_t* ctr = &B.hctr[kHeavyCounterAlpha];
+        for (uint32_t h = next_item(ctr, nh, lane); h < nh; h = next_item(ctr, nh, lane)) {
             const int sh = (int)B.hq[h];
             float a[3];
             alpha_change_nrec_warp<NP>(P, B, S, sh, a);
@@ -1733,39 +1785,41 @@ F4Set make_set(const DevBuffers& B, const int* cur, bool to_alt) {
 // Launchers
 // ---------------------------------------------------------------------------
 
+void launch_clear_counts(const DevBuffers& B, cudaStream_t s) { cudaMemsetAsync(B.ccount, 0, B.count_bytes, s); }
+
 void launch_hash(const DevParams& P, const DevBuffers& B, const int* cur, cudaStream_t s) {
-    cudaMemsetAsync(B.ccount, 0, sizeof(uint32_t) * (size_t)(P.G + 1), s);
-    if (P.n <= 0) return;
+    if (P.n <= 0) {
+        cudaMemsetAsync(B.ctl, 0, sizeof(uint32_t) * kCtlWords, s);
+        return;
+    }
     k_hash<<<blocks_for(P.n, kHashBlock), kHashBlock, 0, s>>>(P, B, B.f4[POS][cur[POS]]);
 }
 
-void launch_cell_starts(const DevParams& P, const DevBuffers& B, cudaStream_t s) {
-    const int per = kScanBlock * kScanItems;
-    const int nb = (P.G + per - 1) / per;
-    const int nchunks = blocks_for(P.n, kHashBlock);
-    k_scan_reduce<<<nb, kScanBlock, 0, s>>>(P, B);
-    k_scan_top<<<1, kScanBlock, 0, s>>>(P, B, nb, nchunks);
-    k_scan_apply<<<nb, kScanBlock, 0, s>>>(P, B);
+void launch_recount(const DevParams& P, const DevBuffers& B, cudaStream_t s) {
+    if (P.n > 0) k_recount<<<blocks_for(P.n, kHashBlock), kHashBlock, 0, s>>>(P, B);
+}
+
+void launch_cell_starts(const DevParams& P, const DevBuffers& B, bool hashed, bool clear, cudaStream_t s) {
+    const int nb = (P.G + (int)kScanPer - 1) / (int)kScanPer;
+    if (P.morton || !hashed) k_scan_reduce<<<nb, kScanBlock, 0, s>>>(P, B);
+    k_scan<<<nb, kScanBlock, 0, s>>>(P, B, clear ? 1 : 0);
 }
 
 void launch_cell_order(const DevParams& P, const DevBuffers& B, const int* cur, cudaStream_t s) {
     if (P.n <= 0) return;
     const float4* pos_in = B.f4[POS][cur[POS]];
     k_scatter<<<blocks_for(P.n), kThreads, 0, s>>>(P, B);
-    const int grid = min(blocks_for(P.G * 32), 152 * 16);
+    // one warp a cell, at most one cell a particle
+    const int grid = min(blocks_for(min(P.G, P.n), kThreads / 32), 152 * 16);
     k_cell_sort<<<grid, kThreads, 0, s>>>(P, B, pos_in);
     k_big_cell_sort<<<64, 1024, 0, s>>>(P, B, pos_in);
 }
 
-void launch_grid_list(const DevParams& P, const DevBuffers& B, const int* cur, cudaStream_t s) {
-    launch_cell_starts(P, B, s);
-    launch_cell_order(P, B, cur, s);
-}
-
-void launch_rearrange(const DevParams& P, const DevBuffers& B, const int* cur, bool slot_order, cudaStream_t s) {
+void launch_rearrange(const DevParams& P, const DevBuffers& B, const int* cur, bool slot_order, bool clear,
+                      cudaStream_t s) {
     if (P.n <= 0) return;
     if (slot_order) k_slot_order<<<blocks_for(P.n), kThreads, 0, s>>>(P, B);
-    k_rearrange<<<blocks_for(P.n), kThreads, 0, s>>>(P, B, make_set(B, cur, true));
+    k_rearrange<<<blocks_for(P.n), kThreads, 0, s>>>(P, B, make_set(B, cur, true), clear ? 1 : 0);
 }
 
 void launch_boundary_volume(const DevParams& P, const DevBuffers& B, const int* cur, cudaStream_t s) {
@@ -1780,11 +1834,15 @@ void launch_density(const DevParams& P, const DevBuffers& B, const int* cur, cud
     k_density<<<blocks_for(P.n), kThreads, 0, s>>>(P, B, B.f4[POS][cur[POS]], B.f4[ALPHA][cur[ALPHA]]);
 }
 
-void launch_density_oct(const DevParams& P, const DevBuffers& B, const int* cur, cudaStream_t s) {
+// `fresh`: the hash of this step has cleared the control words and no pass has used them since.
+void launch_density_oct(const DevParams& P, const DevBuffers& B, const int* cur, bool fresh, cudaStream_t s) {
     if (P.n <= 0) return;
     const float4* pos = B.f4[POS][cur[POS]];
     const float4* alpha = B.f4[ALPHA][cur[ALPHA]];
-    cudaMemsetAsync(B.dctr, 0, sizeof(uint32_t), s);
+    if (!fresh) {
+        cudaMemsetAsync(B.dctr, 0, sizeof(uint32_t), s);
+        cudaMemsetAsync(B.hq_n, 0, sizeof(uint32_t), s);
+    }
     if (P.ss == 1.0f)
         k_density_bucket<true><<<resident_grid(k_density_bucket<true>, kDensThreads), kDensThreads, 0, s>>>(P, B, pos, alpha);
     else
@@ -1821,20 +1879,21 @@ static void fd_lanes(const DevParams& P, const DevBuffers& B, const int* cur, cu
 }
 
 template <bool F, bool D>
-static void fd_dispatch(const DevParams& P, const DevBuffers& B, const int* cur, cudaStream_t s) {
-    cudaMemsetAsync(&B.hctr[0], 0, sizeof(uint32_t), s);  // the heavy-particle queue's work counter
+static void fd_dispatch(const DevParams& P, const DevBuffers& B, const int* cur, bool fresh, cudaStream_t s) {
+    // the heavy-particle queue's work counter
+    if (!fresh) cudaMemsetAsync(&B.hctr[kHeavyCounter<F, D>], 0, sizeof(uint32_t), s);
     if (!D) fd_lanes<F, false, 0>(P, B, cur, s);
     else if (P.nphase == 1) fd_lanes<F, true, 1>(P, B, cur, s);
     else if (P.nphase == 2) fd_lanes<F, true, 2>(P, B, cur, s);
     else fd_lanes<F, true, 3>(P, B, cur, s);
 }
 
-void launch_force_drift(const DevParams& P, const DevBuffers& B, const int* cur, bool force, bool drift,
+void launch_force_drift(const DevParams& P, const DevBuffers& B, const int* cur, bool force, bool drift, bool fresh,
                         cudaStream_t s) {
     if (P.n <= 0 || (!force && !drift)) return;
-    if (force && drift) fd_dispatch<true, true>(P, B, cur, s);
-    else if (force) fd_dispatch<true, false>(P, B, cur, s);
-    else fd_dispatch<false, true>(P, B, cur, s);
+    if (force && drift) fd_dispatch<true, true>(P, B, cur, fresh, s);
+    else if (force) fd_dispatch<true, false>(P, B, cur, fresh, s);
+    else fd_dispatch<false, true>(P, B, cur, fresh, s);
 }
 
 void launch_force_drift_features(const DevParams& P, const DevBuffers& B, const int* cur, float* feat, int32_t* ids,
@@ -1925,7 +1984,6 @@ static void pass_c_lanes(const DevParams& P, const DevBuffers& B, const F4Set& S
 void launch_pass_c(const DevParams& P, const DevBuffers& B, const int* cur, cudaStream_t s) {
     if (P.n <= 0) return;
     const F4Set S = make_set(B, cur, true);
-    cudaMemsetAsync(&B.hctr[1], 0, sizeof(uint32_t), s);  // the heavy-particle queue's work counter
     if (!P.multiphase) k_pass_c<1, false, 1><<<blocks_for(P.n), kThreads, 0, s>>>(P, B, S);
     else if (P.nphase == 1) pass_c_lanes<1>(P, B, S, s);
     else if (P.nphase == 2) pass_c_lanes<2>(P, B, S, s);
