@@ -180,17 +180,12 @@ struct sphmp_corrector {
     float* grads = nullptr;
     float* adam_m = nullptr;
     float* adam_v = nullptr;
-    bf16 *w1 = nullptr, *w2 = nullptr, *w3 = nullptr, *w4 = nullptr, *w2t = nullptr, *w3t = nullptr, *w4t = nullptr;
+    bf16 *w1 = nullptr, *w2 = nullptr, *w3 = nullptr, *w4 = nullptr;
     float* bias = nullptr;      // [3 * 128 + 16]
     float* norm = nullptr;      // fshift [48], fscale [48], out_scale [4]
     uint32_t* err = nullptr;
-    // training buffers (max_batch rows): the hidden layers' z (FP16), outputs,
-    // the layer inputs transposed, the output gradient
-    __half *z1 = nullptr, *z2 = nullptr, *z3 = nullptr;
-    float* y = nullptr;
-    bf16 *h0t = nullptr, *h1t = nullptr, *h2t = nullptr, *h3t = nullptr;
-    bf16* dy = nullptr;
-    float* bpart = nullptr;     // the fused backward's per-CTA gradient partials [num_sms][kParams]
+    // training scratch
+    float* bpart = nullptr;     // per-CTA gradient partials [num_sms][kParams]
     float* loss_part = nullptr;
     float* loss = nullptr;
     std::vector<void*> allocs;
@@ -229,7 +224,7 @@ mlp::Packed packed(const sphmp_corrector* c) {
 }
 
 mlp::PackedMut packed_mut(const sphmp_corrector* c) {
-    return mlp::PackedMut{c->w1, c->w2, c->w3, c->w4, c->w2t, c->w3t, c->w4t, c->bias};
+    return mlp::PackedMut{c->w1, c->w2, c->w3, c->w4, c->bias};
 }
 
 sphmp_status take_errors(sphmp_corrector* c) {
@@ -246,11 +241,8 @@ sphmp_status enqueue_backward(sphmp_corrector* c, const float* x, const float* t
                               const mlp::AdamStep& adam, bool want_loss) {
     using namespace mlp;
     const cudaStream_t s = c->stream;
-    const int ld = c->max_batch;
-    const Saves S{c->z1, c->z2, c->z3, c->h0t, c->h1t, c->h2t, c->h3t, ld};
-    LCK(launch_forward(x, batch, packed(c), S, c->y, c->err, c->num_sms, s));
-    LCK(launch_out_grad(c->y, t, batch, ld, c->dy, nullptr, c->loss_part, want_loss ? c->loss : nullptr, s));
-    LCK(launch_backward(c->dy, S, packed_mut(c), batch, c->bpart, c->grads, adam, c->err, c->num_sms, s));
+    LCK(launch_train(x, t, batch, packed(c), c->bpart, c->loss_part, c->grads, adam, want_loss ? c->loss : nullptr,
+                     c->err, c->num_sms, s));
     return SPHMP_OK;
 }
 
@@ -267,7 +259,7 @@ sphmp_status check_batch(const sphmp_corrector* c, const float* x, const float* 
 namespace sphmp {
 cudaError_t corrector_forward_on(sphmp_corrector* c, const float* x, int n, float* y, uint32_t* err,
                                  cudaStream_t s) {
-    return mlp::launch_forward(x, n, packed(c), mlp::Saves{}, y, err, c->num_sms, s);
+    return mlp::launch_forward(x, n, packed(c), y, err, c->num_sms, s);
 }
 const float* corrector_out_scale(const sphmp_corrector* c) { return c->norm + 2 * mlp::kFeatures; }
 int corrector_device(const sphmp_corrector* c) { return c->device; }
@@ -297,17 +289,12 @@ sphmp_status sphmp_corrector_create(int32_t max_batch, void* stream, sphmp_corre
     };
     A(&c->params, kParams); A(&c->grads, kParams); A(&c->adam_m, kParams); A(&c->adam_v, kParams);
     A(&c->w1, kHidden * kInPad); A(&c->w2, kHidden * kHidden); A(&c->w3, kHidden * kHidden);
-    A(&c->w4, kOutPad * kHidden); A(&c->w2t, kHidden * kHidden); A(&c->w3t, kHidden * kHidden);
-    A(&c->w4t, kHidden * kOutPad); A(&c->bias, 3 * kHidden + kOutPad); A(&c->norm, 2 * kFeatures + kOutputs);
+    A(&c->w4, kOutPad * kHidden); A(&c->bias, 3 * kHidden + kOutPad); A(&c->norm, 2 * kFeatures + kOutputs);
     A(&c->err, 1);
     const size_t B = (size_t)max_batch;
     if (B > 0) {
-        A(&c->z1, kHidden * B); A(&c->z2, kHidden * B); A(&c->z3, kHidden * B);  // [128][max_batch]
-        A(&c->y, B * 4);
-        A(&c->h0t, (size_t)kInPad * B); A(&c->h1t, kHidden * B); A(&c->h2t, kHidden * B); A(&c->h3t, kHidden * B);
-        A(&c->dy, B * kOutPad);
         A(&c->bpart, (size_t)c->num_sms * kParams);
-        A(&c->loss_part, B / 256 + 1);
+        A(&c->loss_part, B / 32);
         A(&c->loss, 1);
     }
     if (st == SPHMP_OK && cudaDeviceSynchronize() != cudaSuccess)  // the zero fills (legacy default stream)
@@ -373,7 +360,7 @@ sphmp_status sphmp_corrector_set_normalisation(sphmp_corrector* c, const float* 
 
 sphmp_status sphmp_corrector_forward(sphmp_corrector* c, const float* x, int32_t n, float* y) {
     if (!c || !x || !y || n < 0) return lfail(SPHMP_ERR_INVALID_ARG, "bad arguments");
-    LCK(mlp::launch_forward(x, n, packed(c), mlp::Saves{}, y, c->err, c->num_sms, c->stream));
+    LCK(mlp::launch_forward(x, n, packed(c), y, c->err, c->num_sms, c->stream));
     return SPHMP_OK;
 }
 

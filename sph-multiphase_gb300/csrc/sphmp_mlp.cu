@@ -7,19 +7,19 @@
 //   kernel, four tiles in flight per CTA. The weights stay in shared memory;
 //   each layer is one chain of MMAs
 //   into TMEM, and its epilogue (bias, SiLU, bf16) writes the next layer's
-//   operand tile back into shared memory. With the training saves it also
-//   stores z of each hidden layer (FP16) and the bf16 layer inputs transposed
-//   (feature-major), the operands of the backward pass.
-// * k_mlp_backward: the whole backward pass in one persistent kernel, one CTA
-//   per SM over 128-row tiles: dH GEMMs, the SiLU backward in their epilogues,
-//   and the weight and bias gradients accumulated in TMEM over the CTA's tiles;
+//   operand tile back into shared memory.
+// * k_mlp_train: forward and backward pass of a batch in one persistent kernel, one
+//   CTA per SM over 128-row tiles: the layer inputs stay in shared memory and the
+//   pre-activations in registers from the forward half of a tile to its backward
+//   half, the transposes are taken by the operand descriptors (MN-major), and the
+//   weight and bias gradients accumulate in TMEM over the CTA's tiles;
 //   k_sum_partials adds the CTAs' partial gradients in a fixed order.
 // * k_gemm_tn: D = A B^T for K-major bf16 A [M][K] and B [N][K] (N <= 128),
 //   M in tiles of 128, K split over gridDim.y into FP32 partials (the library's
 //   GEMM entry point).
-// * elementwise kernels: the output gradient, the sum of the partial gradients
-//   with the Adam step, and the packing of the FP32 master parameters into the
-//   padded bf16 operand layouts.
+// * elementwise kernels: the loss, the sum of the partial gradients with the Adam
+//   step, and the packing of the FP32 master parameters into the padded bf16
+//   operand layouts.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -36,19 +36,10 @@ using bf16 = __nv_bfloat16;
 
 namespace {
 
-// SiLU of the forward pass as z/2 (1 + tanh(z/2)) with the hardware tanh
-// (tanh.approx.f32, relative error about 2^-11, below the bf16 rounding of the
-// result): one special-function operation per element instead of two (exp and
-// reciprocal), which bound the forward kernel's epilogues.
 __device__ __forceinline__ float tanh_approx(float x) {
     float y;
     asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
-}
-
-__device__ __forceinline__ float silu(float z) {
-    const float hz = 0.5f * z;
-    return fmaf(hz, tanh_approx(hz), hz);
 }
 
 __device__ __forceinline__ float silu_grad(float z) {
@@ -65,13 +56,12 @@ __device__ __forceinline__ uint32_t pack2(float a, float b) {
 // Fused forward
 // ---------------------------------------------------------------------------
 
-constexpr int kGroups = 4;                     // tiles in flight per CTA
-constexpr int kGroupThreads = 128;             // 4 warps: one TMEM lane quadrant each
-constexpr int kFwdThreads = kGroups * kGroupThreads;
+constexpr int kGroups = 4;                     // tiles in flight per CTA, at most
+constexpr int kFwdThreads = 1024;              // 32 warps, shared equally by the groups
 constexpr int kTile = 128;
 // dynamic shared memory of the forward kernel
-constexpr int kOffW1 = 0;                                  // [128 rows][64] kc 64
-constexpr int kOffW2 = kOffW1 + kHidden * kInPad * 2;      // [128][128]
+constexpr int kOffW1 = 0;                                  // [128 rows][48] kc 48
+constexpr int kOffW2 = kOffW1 + kHidden * kFeatures * 2;   // [128][128]
 constexpr int kOffW3 = kOffW2 + kHidden * kHidden * 2;     // [128][128]
 constexpr int kOffW4 = kOffW3 + kHidden * kHidden * 2;     // [16][128]
 constexpr int kOffAct = kOffW4 + kOutPad * kHidden * 2;    // kGroups x [128][128] operand tiles
@@ -80,19 +70,38 @@ constexpr int kOffBias = kOffAct + kGroups * kActBytes;    // 3 * 128 + 16 float
 constexpr int kOffNorm = kOffBias + (3 * kHidden + kOutPad) * 4;  // shift[48], scale[48]
 constexpr int kFwdSmem = kOffNorm + 2 * kFeatures * 4;
 // TMEM: group g uses columns [128 g, 128 g + 128) for layers 1-3 and the first
-// 16 of them again for layer 4 (after layer 3's epilogue has read them)
+// 16 of them again for layer 4 (after layer 3's epilogue has read them). With one
+// CTA per SM the allocation always takes every column.
 constexpr uint32_t kGroupTmemCols = 128;
 constexpr uint32_t kFwdTmemCols = kGroups * kGroupTmemCols;
 static_assert(kFwdTmemCols <= 512, "TMEM holds 512 columns");
 static_assert(kFwdSmem > 116 * 1024, "one CTA per SM: the TMEM allocation takes every column");
 static_assert(kFwdSmem <= 227 * 1024, "shared memory of one CTA");
 
-__device__ __forceinline__ void stage_weights(uint8_t* dst, const bf16* src, int rows, int kc, int tid,
+__device__ __forceinline__ void cp_async16(uint8_t* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(tc::smem_addr(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+// A read-only 16-byte load that stays where it is written (an ordinary one sinks down
+// to its use, past the waits that it should overlap).
+__device__ __forceinline__ float4 load_early(const float4* p) {
+    float4 v;
+    asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
+}
+
+// The first kc columns of weights [rows][stride] as a K-major tile (16-byte copies in
+// flight together; the caller commits and waits).
+__device__ __forceinline__ void stage_weights(uint8_t* dst, const bf16* src, int rows, int kc, int stride, int tid,
                                               int nthreads) {
     for (int q = tid; q < rows * (kc / 8); q += nthreads) {
         const int r = q / (kc / 8), k = (q % (kc / 8)) * 8;
-        *reinterpret_cast<uint4*>(dst + tc::kmajor_offset(r, k, kc)) =
-            *reinterpret_cast<const uint4*>(src + (size_t)r * kc + k);
+        cp_async16(dst + tc::kmajor_offset(r, k, kc), src + (size_t)r * stride + k);
     }
 }
 
@@ -120,10 +129,12 @@ __device__ __forceinline__ void handoff_to_mma() {
     __syncthreads();
 }
 
-// The same for the 128 threads of one tile group (named barrier 1 + g).
+// The same for the T threads of one tile group (named barrier 1 + g).
+template <int T>
 __device__ __forceinline__ void group_sync(int g) {
-    asm volatile("bar.sync %0, %1;" ::"r"(1 + g), "r"(kGroupThreads) : "memory");
+    asm volatile("bar.sync %0, %1;" ::"r"(1 + g), "n"(T) : "memory");
 }
+template <int T>
 __device__ __forceinline__ bool group_all(int g, bool v) {
     uint32_t r;
     asm volatile(
@@ -132,99 +143,160 @@ __device__ __forceinline__ bool group_all(int g, bool v) {
         "bar.red.and.pred q, %2, %3, p;\n\t"
         "selp.u32 %0, 1, 0, q;\n\t}"
         : "=r"(r)
-        : "r"((uint32_t)v), "r"(1 + g), "r"(kGroupThreads)
+        : "r"((uint32_t)v), "r"(1 + g), "n"(T)
         : "memory");
     return r != 0;
 }
+template <int T>
 __device__ __forceinline__ bool group_wait(uint64_t* bar, uint32_t& parity, int g) {
     const bool ok = tc::mbar_wait(bar, parity, tc::kWaitLimitNs);
     parity ^= 1u;
-    const bool all = group_all(g, ok);
+    const bool all = group_all<T>(g, ok);
     tc::fence_after_sync();
     return all;
 }
+template <int T>
 __device__ __forceinline__ void group_handoff(int g) {
     tc::fence_async_smem();
     tc::fence_before_sync();
-    group_sync(g);
+    group_sync<T>(g);
 }
 
-// Epilogue of a hidden layer for this thread's row (all 128 columns): bias +
-// SiLU, the bf16 activations into the operand tile (K = 128), the training saves.
-__device__ __forceinline__ void hidden_epilogue(uint32_t tmem, int warp, int lane, const float* bias, uint8_t* act,
-                                                int row0, int n, __half* z_save, bf16* ht_save, int ldh) {
-    const int r = (warp & 3) * 32 + lane;
-    const int grow = row0 + r;
-    const bool live = grow < n;
-#pragma unroll 1
-    for (int c0 = 0; c0 < kHidden; c0 += 16) {
-        float v[16];
-        tc::tmem_ld16(tc::tmem_lane_addr(tmem, warp, c0), v);
-        float h[16];
+// SiLU of 16 columns (c0 on) of a hidden layer's accumulator row, the bf16
+// activations into the operand tile (row r, K = 128); z (FP16) into zs if wanted.
+// SiLU is z/2 (1 + tanh(z/2)) with the hardware tanh (tanh.approx.f32, relative
+// error about 2^-11, below the bf16 rounding of the result): one special-function
+// operation per element instead of two (exp and reciprocal). hb = bias / 2: z/2 is
+// then one multiply-add (exactly half of the rounded z).
+template <bool SAVE>
+__device__ __forceinline__ void silu16(const uint32_t (&v)[16], int c0, const float* hb, uint8_t* act, int r,
+                                       uint32_t* zs) {
+    const float2 half = make_float2(0.5f, 0.5f);
 #pragma unroll
-        for (int i = 0; i < 16; i++) {
-            const float z = v[i] + bias[c0 + i];
-            v[i] = z;
-            h[i] = silu(z);
+    for (int q = 0; q < 2; q++) {
+        const int c = c0 + 8 * q;
+        const float4 b[2] = {*reinterpret_cast<const float4*>(hb + c), *reinterpret_cast<const float4*>(hb + c + 4)};
+        uint32_t hw[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const float2 bb = i & 1 ? make_float2(b[i >> 1].z, b[i >> 1].w) : make_float2(b[i >> 1].x, b[i >> 1].y);
+            const float2 a = make_float2(__uint_as_float(v[8 * q + 2 * i]), __uint_as_float(v[8 * q + 2 * i + 1]));
+            const float2 hz = __ffma2_rn(a, half, bb);
+            const float2 h = __ffma2_rn(hz, make_float2(tanh_approx(hz.x), tanh_approx(hz.y)), hz);
+            hw[i] = pack2(h.x, h.y);
+            if (SAVE) {
+                const float2 z = __fadd2_rn(hz, hz);
+                const __half2 zz = __floats2half2_rn(z.x, z.y);
+                zs[4 * q + i] = *reinterpret_cast<const uint32_t*>(&zz);
+            }
         }
-        uint4 lo, hi;
-        lo.x = pack2(h[0], h[1]); lo.y = pack2(h[2], h[3]); lo.z = pack2(h[4], h[5]); lo.w = pack2(h[6], h[7]);
-        hi.x = pack2(h[8], h[9]); hi.y = pack2(h[10], h[11]); hi.z = pack2(h[12], h[13]); hi.w = pack2(h[14], h[15]);
-        *reinterpret_cast<uint4*>(act + tc::kmajor_offset(r, c0, kHidden)) = lo;
-        *reinterpret_cast<uint4*>(act + tc::kmajor_offset(r, c0 + 8, kHidden)) = hi;
-        // the training saves, transposed ([feature][row]): rows 2k and 2k + 1 are adjacent,
-        // so the even lane stores both with one 32-bit store (a warp writes 64 contiguous
-        // bytes per feature): z in FP16 (relative error 2^-11) and the bf16 activations
-        if (ht_save) {
+        *reinterpret_cast<uint4*>(act + tc::kmajor_offset(r, c, kHidden)) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
+    }
+}
+
+// NC columns from c0 on, the accumulator's next 16 loading while the last 16 are
+// processed.
+template <int NC>
+__device__ __forceinline__ void hidden_epilogue(uint32_t tmem, int warp, int c0, const float* hb, uint8_t* act, int r) {
+    uint32_t va[16], vb[16];
+    tc::tmem_issue16(tc::tmem_lane_addr(tmem, warp, c0), va);
 #pragma unroll
-            for (int i = 0; i < 16; i++) {
-                const float oh = __shfl_down_sync(0xffffffffu, h[i], 1);
-                const float oz = __shfl_down_sync(0xffffffffu, v[i], 1);
-                const size_t at = (size_t)(c0 + i) * ldh + grow;
-                if ((lane & 1) == 0 && grow + 1 < n) {
-                    *reinterpret_cast<uint32_t*>(ht_save + at) = pack2(h[i], oh);
-                    const __half2 zz = __floats2half2_rn(v[i], oz);
-                    *reinterpret_cast<__half2*>(z_save + at) = zz;
-                } else if ((lane & 1) == 0 && live) {
-                    ht_save[at] = __float2bfloat16_rn(h[i]);
-                    z_save[at] = __float2half_rn(v[i]);
-                }
+    for (int c = 0; c < NC; c += 32) {
+        tc::tmem_wait16(va);
+        if (c + 16 < NC) tc::tmem_issue16(tc::tmem_lane_addr(tmem, warp, c0 + c + 16), vb);
+        silu16<false>(va, c0 + c, hb, act, r, nullptr);
+        if (c + 16 < NC) {
+            tc::tmem_wait16(vb);
+            if (c + 32 < NC) tc::tmem_issue16(tc::tmem_lane_addr(tmem, warp, c0 + c + 32), va);
+            silu16<false>(vb, c0 + c + 16, hb, act, r, nullptr);
+        }
+    }
+}
+
+// The input tile of rows [row0, row0 + 128) by T threads: normalised features,
+// bf16 (K = 48). Four lanes a row, so that a warp's load touches eight contiguous
+// pieces of 64 bytes.
+template <int T>
+struct InputTile {
+    static constexpr int kRows = T / 4, kPasses = kTile / kRows;
+    static_assert(kRows * kPasses == kTile, "whole passes");
+    float4 f[kPasses][3];
+    __device__ __forceinline__ void load(const float* __restrict__ x, int row0, int n, int gt) {
+#pragma unroll
+        for (int p = 0; p < kPasses; p++) {
+            const int grow = row0 + (gt >> 2) + p * kRows;
+            const float4* src = reinterpret_cast<const float4*>(x + (size_t)(grow < n ? grow : 0) * kFeatures) + (gt & 3);
+#pragma unroll
+            for (int m = 0; m < 3; m++) f[p][m] = load_early(src + 4 * m);
+        }
+    }
+    __device__ __forceinline__ void store(int row0, int n, const float* fshift, const float* fscale, uint8_t* act,
+                                          int gt) const {
+#pragma unroll
+        for (int m = 0; m < 3; m++) {
+            const int c = 4 * ((gt & 3) + 4 * m);
+            const float4 sh = *reinterpret_cast<const float4*>(fshift + c);
+            const float4 sc = *reinterpret_cast<const float4*>(fscale + c);
+#pragma unroll
+            for (int p = 0; p < kPasses; p++) {
+                const int r = (gt >> 2) + p * kRows;
+                const float4 a = f[p][m];
+                uint2 q;
+                q.x = pack2((a.x - sh.x) * sc.x, (a.y - sh.y) * sc.y);
+                q.y = pack2((a.z - sh.z) * sc.z, (a.w - sh.w) * sc.w);
+                if (row0 + r >= n) q = make_uint2(0u, 0u);
+                *reinterpret_cast<uint2*>(act + tc::kmajor_offset(r, c, kFeatures)) = q;
             }
         }
     }
+};
+
+// Biases (halved for the hidden layers) and normalisation into shared memory.
+__device__ __forceinline__ void stage_constants(const Packed& W, float* bias, float* norm, int tid, int nthreads) {
+    for (int i = tid; i < 3 * kHidden + kOutPad; i += nthreads) bias[i] = (i < 3 * kHidden ? 0.5f : 1.f) * W.bias[i];
+    for (int i = tid; i < kFeatures; i += nthreads) {
+        norm[i] = W.fshift[i];
+        norm[kFeatures + i] = W.fscale[i];
+    }
 }
 
-// kGroups independent tile pipelines per CTA (4 warps each), so that one
-// group's epilogue runs while the others' MMAs and loads are in flight; the
-// weights in shared memory are shared.
+// kGroups independent tile pipelines per CTA (8 warps each), so that one group's
+// epilogue runs while the others' MMAs and loads are in flight; the weights in
+// shared memory are shared. The warps of a group split each epilogue by lane
+// quadrant and by columns. Few tiles are spread over the CTAs first.
+// Bound: one tanh per hidden activation, 16 a clock and SM (76 us per million rows,
+// 55 % of the time), beside the chain of a tile (its load, four MMAs and three
+// epilogues). A million rows: 139 us; 204 us with 4 warps a group, a thread reading
+// whole rows of features and no load of the accumulators beside the arithmetic.
+// Up to 128 rows: 11 us and 14 us (32 or 16 warps a tile instead of 8 change nothing).
 __global__ void __launch_bounds__(kFwdThreads, 1) k_mlp_forward(const float* __restrict__ x, int n,
-                                                                 const Packed W, const Saves S,
-                                                                 float* __restrict__ y, uint32_t* err) {
-    extern __shared__ __align__(1024) uint8_t smem[];
+                                                                 const Packed W, float* __restrict__ y,
+                                                                 uint32_t* err) {
+    constexpr int T = kFwdThreads / kGroups;  // threads of a group
+    constexpr int NC = kHidden / (T / 128);   // epilogue columns of a warp
+    extern __shared__ __align__(128) uint8_t smem[];
     __shared__ uint64_t bars[kGroups];
     __shared__ uint32_t tmem_base;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int g = tid / kGroupThreads, gt = tid % kGroupThreads;
+    const int tid = threadIdx.x, warp = tid >> 5;
+    const int g = tid / T, gt = tid % T;
+    const int r = gt & 127, c0 = (gt >> 7) * NC;  // this thread's row and first column
     uint8_t* act = smem + kOffAct + g * kActBytes;
     float* bias = reinterpret_cast<float*>(smem + kOffBias);
-    float* fshift = reinterpret_cast<float*>(smem + kOffNorm);
-    float* fscale = fshift + kFeatures;
+    float* norm = reinterpret_cast<float*>(smem + kOffNorm);
 
-    stage_weights(smem + kOffW1, W.w1, kHidden, kInPad, tid, kFwdThreads);
-    stage_weights(smem + kOffW2, W.w2, kHidden, kHidden, tid, kFwdThreads);
-    stage_weights(smem + kOffW3, W.w3, kHidden, kHidden, tid, kFwdThreads);
-    stage_weights(smem + kOffW4, W.w4, kOutPad, kHidden, tid, kFwdThreads);
-    for (int i = tid; i < 3 * kHidden + kOutPad; i += kFwdThreads) bias[i] = W.bias[i];
-    for (int i = tid; i < kFeatures; i += kFwdThreads) {
-        fshift[i] = W.fshift[i];
-        fscale[i] = W.fscale[i];
-    }
+    stage_weights(smem + kOffW1, W.w1, kHidden, kFeatures, kInPad, tid, kFwdThreads);
+    stage_weights(smem + kOffW2, W.w2, kHidden, kHidden, kHidden, tid, kFwdThreads);
+    stage_weights(smem + kOffW3, W.w3, kHidden, kHidden, kHidden, tid, kFwdThreads);
+    stage_weights(smem + kOffW4, W.w4, kOutPad, kHidden, kHidden, tid, kFwdThreads);
+    cp_async_commit();
+    stage_constants(W, bias, norm, tid, kFwdThreads);
     if (warp == 0) {
         tc::tmem_alloc(&tmem_base, kFwdTmemCols);
         tc::tmem_relinquish();
     }
     if (tid == 0)
         for (int k = 0; k < kGroups; k++) tc::mbar_init(&bars[k], 1);
+    cp_async_wait<0>();
     tc::fence_async_smem();
     tc::fence_before_sync();
     __syncthreads();
@@ -235,82 +307,52 @@ __global__ void __launch_bounds__(kFwdThreads, 1) k_mlp_forward(const float* __r
     uint32_t parity = 0;
     bool ok = true;
     const int ntiles = (n + kTile - 1) / kTile;
-    for (int t = kGroups * blockIdx.x + g; t < ntiles && ok; t += kGroups * gridDim.x) {
+    for (int t = g * gridDim.x + blockIdx.x; t < ntiles && ok; t += kGroups * gridDim.x) {
         const int row0 = t * kTile;
-        // input tile: normalised features, bf16, K padded to 64 with zeros
         {
-            const int r = gt;
-            const int grow = row0 + r;
-            const bool live = grow < n;
-            const float4* src = reinterpret_cast<const float4*>(x + (size_t)(live ? grow : 0) * kFeatures);
-#pragma unroll 2
-            for (int c = 0; c < kFeatures / 8; c++) {  // 8 features at a time
-                float f[8];
-                const float4 a = live ? src[2 * c] : make_float4(0.f, 0.f, 0.f, 0.f);
-                const float4 b = live ? src[2 * c + 1] : make_float4(0.f, 0.f, 0.f, 0.f);
-                f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
-#pragma unroll
-                for (int i = 0; i < 8; i++) f[i] = live ? (f[i] - fshift[8 * c + i]) * fscale[8 * c + i] : 0.f;
-                uint4 q;
-                q.x = pack2(f[0], f[1]); q.y = pack2(f[2], f[3]); q.z = pack2(f[4], f[5]); q.w = pack2(f[6], f[7]);
-                *reinterpret_cast<uint4*>(act + tc::kmajor_offset(r, 8 * c, kInPad)) = q;
-                if (S.h0t) {  // transposed, a 32-bit store per row pair (as in the hidden layers)
-#pragma unroll
-                    for (int i = 0; i < 8; i++) {
-                        const float o = __shfl_down_sync(0xffffffffu, f[i], 1);
-                        bf16* dst = S.h0t + (size_t)(8 * c + i) * S.ldh + grow;
-                        if ((gt & 1) == 0 && grow + 1 < n) *reinterpret_cast<uint32_t*>(dst) = pack2(f[i], o);
-                        else if ((gt & 1) == 0 && live) *dst = __float2bfloat16_rn(f[i]);
-                    }
-                }
-            }
-            const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
-            *reinterpret_cast<uint4*>(act + tc::kmajor_offset(r, 48, kInPad)) = zero;
-            *reinterpret_cast<uint4*>(act + tc::kmajor_offset(r, 56, kInPad)) = zero;
+            InputTile<T> in;
+            in.load(x, row0, n, gt);
+            in.store(row0, n, norm, norm + kFeatures, act, gt);
         }
-        group_handoff(g);
+        group_handoff<T>(g);
         // layer 1
         if (gt == 0) {
             tc::fence_after_sync();
-            issue_layer(tmem, a_act, tc::smem_addr(smem + kOffW1), kInPad, kHidden, bar);
+            issue_layer(tmem, a_act, tc::smem_addr(smem + kOffW1), kFeatures, kHidden, bar);
         }
-        if (!(ok = group_wait(bar, parity, g))) break;
-        hidden_epilogue(tmem, warp, lane, bias, act, row0, n, S.z1, S.h1t, S.ldh);
-        group_handoff(g);
+        if (!(ok = group_wait<T>(bar, parity, g))) break;
+        hidden_epilogue<NC>(tmem, warp, c0, bias, act, r);
+        group_handoff<T>(g);
         // layer 2
         if (gt == 0) {
             tc::fence_after_sync();
             issue_layer(tmem, a_act, tc::smem_addr(smem + kOffW2), kHidden, kHidden, bar);
         }
-        if (!(ok = group_wait(bar, parity, g))) break;
-        hidden_epilogue(tmem, warp, lane, bias + kHidden, act, row0, n, S.z2, S.h2t, S.ldh);
-        group_handoff(g);
+        if (!(ok = group_wait<T>(bar, parity, g))) break;
+        hidden_epilogue<NC>(tmem, warp, c0, bias + kHidden, act, r);
+        group_handoff<T>(g);
         // layer 3
         if (gt == 0) {
             tc::fence_after_sync();
             issue_layer(tmem, a_act, tc::smem_addr(smem + kOffW3), kHidden, kHidden, bar);
         }
-        if (!(ok = group_wait(bar, parity, g))) break;
-        hidden_epilogue(tmem, warp, lane, bias + 2 * kHidden, act, row0, n, S.z3, S.h3t, S.ldh);
-        group_handoff(g);
+        if (!(ok = group_wait<T>(bar, parity, g))) break;
+        hidden_epilogue<NC>(tmem, warp, c0, bias + 2 * kHidden, act, r);
+        group_handoff<T>(g);
         // layer 4 (N = 16: outputs 0..3 and zero padding)
         if (gt == 0) {
             tc::fence_after_sync();
             issue_layer(tmem, a_act, tc::smem_addr(smem + kOffW4), kHidden, kOutPad, bar);
         }
-        if (!(ok = group_wait(bar, parity, g))) break;
-        {
+        if (!(ok = group_wait<T>(bar, parity, g))) break;
+        if (gt < kTile) {
             float v[16];
             tc::tmem_ld16(tc::tmem_lane_addr(tmem, warp, 0), v);
-            const int grow = row0 + gt;
             const float* b4 = bias + 3 * kHidden;
-            if (grow < n)
-                reinterpret_cast<float4*>(y)[grow] = make_float4(v[0] + b4[0], v[1] + b4[1], v[2] + b4[2], v[3] + b4[3]);
+            if (row0 + gt < n)
+                reinterpret_cast<float4*>(y)[row0 + gt] = make_float4(v[0] + b4[0], v[1] + b4[1], v[2] + b4[2], v[3] + b4[3]);
         }
-        // the accumulator reads above come before the next tile's first MMA
-        tc::fence_before_sync();
-        group_sync(g);
-        tc::fence_after_sync();
+        // the accumulator reads above come before the next tile's first MMA (its handoff)
     }
     if (!ok) {
         if (gt == 0) atomicOr(err, kErrMmaTimeout);
@@ -336,7 +378,7 @@ constexpr int kGemmSmem = 2 * kStageBytes;
 __global__ void __launch_bounds__(kGemmThreads) k_gemm_tn(const bf16* __restrict__ A, int lda,
                                                           const bf16* __restrict__ B, int ldb, float* __restrict__ D,
                                                           int M, int N, int K, int kper, uint32_t* err) {
-    extern __shared__ __align__(1024) uint8_t smem[];
+    extern __shared__ __align__(128) uint8_t smem[];
     __shared__ uint64_t bar;
     __shared__ uint32_t tmem_base;
     // two stages of (A tile, B tile): chunk c + 1 loads while chunk c's MMAs run
@@ -416,126 +458,76 @@ __global__ void __launch_bounds__(kGemmThreads) k_gemm_tn(const bf16* __restrict
 }
 
 // ---------------------------------------------------------------------------
-// Fused backward: one persistent CTA per SM, 128-row tiles in turn
+// Fused training pass: one persistent CTA per SM, 128-row tiles in turn
 // ---------------------------------------------------------------------------
 //
-// For each tile (rows r of the batch), with dY = the output gradient:
+// For each tile (rows r of the batch), the forward pass
+//   Z1 = H0 W1^T + b1,  H1 = SiLU(Z1),  Z2, H2, Z3, H3 likewise,  Y = H3 W4^T + b4
+// and with dY = 2 (Y - T) / batch, the gradient of the mean squared output error,
 //   dW4^T += H3^T dY          dH3 = dY W4
-//   dZ3 = dH3 * SiLU'(Z3)     dW3 += dZ3^T H2   db3 += sum_r dZ3   dH2 = dZ3 W3   (Z saved in FP16)
+//   dZ3 = dH3 * SiLU'(Z3)     dW3 += dZ3^T H2   db3 += sum_r dZ3   dH2 = dZ3 W3   (Z kept in FP16)
 //   dZ2 = dH2 * SiLU'(Z2)     dW2 += dZ2^T H1   db2 += sum_r dZ2   dH1 = dZ2 W2
 //   dZ1 = dH1 * SiLU'(Z1)     dW1 += dZ1^T H0   db1 += sum_r dZ1
-// The weight and bias gradients accumulate in TMEM over all tiles of the CTA
-// (the bias sums as MMAs against a tile of ones), so nothing but the CTA's
-// final partial sums goes to memory; dH of the current layer lives in the
-// first 128 columns. Operands in shared memory, K-major without swizzling:
-// the weights W4^T, W3^T, W2^T (resident), dY [rows][16] and dY^T [16][rows],
-// dZ [rows][128] and dZ^T [128][rows] (written by the epilogues), and the saved
-// layer inputs H^T [width][rows], double-buffered and copied with cp.async one
-// step ahead of their MMA. The batch is a multiple of 128 rows (no tails). Warp
-// w handles rows 32 (w % 4) .. + 31 (its TMEM lane quadrant) and columns
-// 64 (w / 4) .. + 63 of every epilogue.
-constexpr int kBwdThreads = 256;  // 8 warps: two per TMEM lane quadrant, one per column half
-constexpr int kBOffW4t = 0;                                   // [128][16]   kc 16
-constexpr int kBOffW3t = kBOffW4t + kHidden * kOutPad * 2;    // [128][128]  kc 128
-constexpr int kBOffW2t = kBOffW3t + kHidden * kHidden * 2;    // [128][128]
-constexpr int kBOffOnes = kBOffW2t + kHidden * kHidden * 2;   // [16][128]   kc 128, all 1
-constexpr int kBOffDy = kBOffOnes + kOutPad * kTile * 2;      // [128][16]   kc 16
-constexpr int kBOffDyt = kBOffDy + kTile * kOutPad * 2;       // [16][128]   kc 128
-constexpr int kBOffDz = kBOffDyt + kOutPad * kTile * 2;       // [128][128]  kc 128
-constexpr int kBOffDzt = kBOffDz + kTile * kHidden * 2;       // [128][128]  kc 128
-constexpr int kBOffH = kBOffDzt + kHidden * kTile * 2;        // 2 x [128][128] kc 128
-constexpr int kBwdSmem = kBOffH + 2 * kHidden * kTile * 2;
-static_assert(kBwdSmem <= 227 * 1024, "shared memory of one CTA");
-static_assert(kBwdSmem > 116 * 1024, "one CTA per SM: the TMEM allocation takes every column");
-static_assert(kBwdSmem - kBOffDz >= kHidden * (kHidden + 4) * 4, "the partials' staging tile fits the operand buffers");
+// Nothing of a tile but its rows of x and T comes from memory and nothing goes
+// there: the layer inputs H stay in shared memory, Z in registers (each thread's
+// row and 32 columns of three layers: 48 registers), and the weight and bias
+// gradients accumulate in TMEM over all tiles of the CTA (the bias sums as MMAs
+// against a tile of ones); Z or dH of the current layer lives in the first 128
+// columns. Every operand is in shared memory once, without swizzling, and its
+// transpose is the same tile read MN-major. The batch is a multiple of 128 rows
+// (no tails). Warp w handles rows 32 (w % 4) .. + 31 (its TMEM lane quadrant) and
+// columns 32 (w / 4) .. + 31 of every epilogue.
+// Bound: the chain of a tile, seven GEMMs each with an epilogue after it (one special-
+// function operation an element forward, two backward, 16 a clock and SM). In the
+// backward half dH is issued and committed first and the weight gradients' MMAs
+// run beside the epilogue, which writes dZ elsewhere than they read: dZ3 into a tile of
+// its own, dZ2 over H3, dZ1 over dZ3 (MMAs complete in order, so the commit that an
+// epilogue waits for covers everything before it).
+// 65,536 rows (a step with the sum of the partials and Adam): 60 us; as two
+// kernels that passed Z and H through memory 80 us, with transposed copies of
+// H and dZ as well 145 us. 8,192 rows: 26, 37 and 87 us.
+constexpr int kTrnThreads = 512;  // 16 warps: four per TMEM lane quadrant, one per column quarter
+constexpr int kTHid = kTile * kHidden * 2;                    // bytes of a [128][128] tile
+constexpr int kTOffW1 = 0;                                    // [128][48]   kc 48
+constexpr int kTOffW2 = kTOffW1 + kHidden * kFeatures * 2;    // [128][128]  kc 128
+constexpr int kTOffW3 = kTOffW2 + kHidden * kHidden * 2;      // [128][128]
+constexpr int kTOffW4 = kTOffW3 + kHidden * kHidden * 2;      // [16][128]
+constexpr int kTOffOnes = kTOffW4 + kOutPad * kHidden * 2;    // [16][16]    kc 16, all 1 (for every step of K)
+constexpr int kTOffDy = kTOffOnes + kOutPad * 16 * 2;         // [128][16]   kc 16
+constexpr int kTOffBias = kTOffDy + kTile * kOutPad * 2;
+constexpr int kTOffNorm = kTOffBias + (3 * kHidden + kOutPad) * 4;
+constexpr int kTOffH0 = kTOffNorm + 2 * kFeatures * 4;        // [128][48]   kc 48
+constexpr int kTOffH1 = kTOffH0 + kTile * kFeatures * 2;      // [128][128]  kc 128
+constexpr int kTOffH2 = kTOffH1 + kTHid;
+constexpr int kTOffH3 = kTOffH2 + kTHid;                      // later dZ2
+constexpr int kTOffDz = kTOffH3 + kTHid;                      // dZ3, later dZ1
+constexpr int kTrnSmem = kTOffDz + kTHid;
+static_assert(kTrnSmem + 256 <= 227 * 1024, "shared memory of one CTA (with the static part)");
+static_assert(kTrnSmem > 116 * 1024, "one CTA per SM: the TMEM allocation takes every column");
+static_assert(kTrnSmem - kTOffH1 >= kHidden * (kHidden + 4) * 4, "the partials' staging tile fits the operand tiles");
+static_assert(kTOffBias % 16 == 0 && kTOffNorm % 16 == 0 && kTOffH0 % 16 == 0, "16-byte tiles");
 // TMEM columns
-constexpr uint32_t kTcDh = 0, kTcW3 = 128, kTcW2 = 256, kTcW1 = 384, kTcW4 = 448, kTcB3 = 464, kTcB2 = 480,
-                   kTcB1 = 496, kBwdTmemCols = 512;
+constexpr uint32_t kTcD = 0, kTcW3 = 128, kTcW2 = 256, kTcW1 = 384, kTcW4 = 448, kTcB3 = 464, kTcB2 = 480,
+                   kTcB1 = 496, kTrnTmemCols = 512;
 
-__device__ __forceinline__ void cp_async16(uint8_t* dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(tc::smem_addr(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
-
-// Copy the tile's columns [row0, row0 + 128) of ht [width][ld] into buf as a
-// K-major operand (width rows, K = 128), 16 bytes per cp.async; one group.
-__device__ __forceinline__ void issue_h_tile(uint8_t* buf, const bf16* ht, int width, int ld, int row0, int tid) {
-    for (int q = tid; q < width * (kTile / 8); q += kBwdThreads) {
-        const int f = q >> 4, j = q & 15;
-        cp_async16(buf + tc::kmajor_offset(f, 8 * j, kTile), ht + (size_t)f * ld + row0 + 8 * j);
-    }
-    cp_async_commit();
-}
-
-// MMA chain D (+)= A B^T, K = 16 * ksteps, A and B K-major with K extent kc
-__device__ __forceinline__ void mma_chain(uint32_t d, uint32_t a, uint32_t b, int kc, int ksteps, int n,
-                                          bool accumulate) {
-    const uint32_t idesc = tc::idesc_bf16_f32(kTile, n);
-    for (int ks = 0; ks < ksteps; ks++)
-        tc::mma_bf16(d, tc::kmajor_desc(a, kc, ks), tc::kmajor_desc(b, kc, ks), idesc,
-                     (accumulate || ks > 0) ? 1u : 0u);
-}
-
-// This thread's row of z (FP16, saved transposed [feature][ldh]) for the 64
-// features of its column half: one 2-byte load per feature, a warp reading 64
-// contiguous bytes per feature.
-__device__ __forceinline__ void load_z_half(const __half* __restrict__ zt, int ldh, int row0, int r, int half,
-                                            __half (&zb)[64]) {
-    const __half* src = zt + (size_t)(half * 64) * ldh + row0 + r;
-#pragma unroll
-    for (int f = 0; f < 64; f++) zb[f] = src[(size_t)f * ldh];
-}
-
-// Epilogue of a hidden layer: dZ = dH * SiLU'(Z) for this thread's row and column
-// half, into the dZ operand (unless null) and the dZ^T operand. zb holds that
-// half of the row of z (FP16, loaded by the caller before the MMAs it waited
-// for). In dZ^T two lanes (rows 2k, 2k + 1) write one 32-bit word per feature.
-__device__ __forceinline__ void bwd_epilogue(uint32_t tmem_dh, int warp, int lane, uint8_t* dz, uint8_t* dzt,
-                                             const __half (&zb)[64]) {
-    const int r = (warp & 3) * 32 + lane;
-    const int half = warp >> 2;
-#pragma unroll
-    for (int ch = 0; ch < 4; ch++) {
-        const int c0 = half * 64 + ch * 16;
-        float v[16];
-        tc::tmem_ld16(tc::tmem_lane_addr(tmem_dh, warp, c0), v);
-        float h[16];
-#pragma unroll
-        for (int i = 0; i < 16; i++) h[i] = v[i] * silu_grad(__half2float(zb[ch * 16 + i]));
-        if (dz) {
-            uint4 lo, hi;
-            lo.x = pack2(h[0], h[1]); lo.y = pack2(h[2], h[3]); lo.z = pack2(h[4], h[5]); lo.w = pack2(h[6], h[7]);
-            hi.x = pack2(h[8], h[9]); hi.y = pack2(h[10], h[11]); hi.z = pack2(h[12], h[13]); hi.w = pack2(h[14], h[15]);
-            *reinterpret_cast<uint4*>(dz + tc::kmajor_offset(r, c0, kHidden)) = lo;
-            *reinterpret_cast<uint4*>(dz + tc::kmajor_offset(r, c0 + 8, kHidden)) = hi;
-        }
-        // dZ^T: element (feature, row) at kmajor_offset(feature, row): rows 2k and 2k + 1 are
-        // adjacent bf16, so the even lane stores both (its odd neighbour's value by shuffle)
-#pragma unroll
-        for (int i = 0; i < 16; i++) {
-            const float other = __shfl_down_sync(0xffffffffu, h[i], 1);
-            if ((lane & 1) == 0)
-                *reinterpret_cast<uint32_t*>(dzt + tc::kmajor_offset(c0 + i, r, kTile)) = pack2(h[i], other);
-        }
-    }
+// MMA chain D (+)= A B^T over K = 16 * ksteps; a and b give the descriptors of step ks.
+template <class A, class B>
+__device__ __forceinline__ void mma_chain(uint32_t d, A&& a, B&& b, int ksteps, uint32_t idesc, bool accumulate) {
+    for (int ks = 0; ks < ksteps; ks++) tc::mma_bf16(d, a(ks), b(ks), idesc, (accumulate || ks > 0) ? 1u : 0u);
 }
 
 // This CTA's partial gradients, in the flat parameter layout: row r of the
-// accumulators is TMEM lane r; the two warps of a lane quadrant share the
+// accumulators is TMEM lane r; the four warps of a lane quadrant share the
 // columns. The weight blocks go through a shared-memory tile (rows padded by 4
 // floats) so that the global stores are contiguous; called by every thread
 // once the operand buffers are free (tile: at least 128 x 132 floats).
-__device__ __forceinline__ void bwd_store_partials(uint32_t tmem, int warp, int lane, int tid, bool have,
+__device__ __forceinline__ void store_partials(uint32_t tmem, int warp, int lane, int tid, bool have,
                                                    const float* db4, float* tile, float* __restrict__ out) {
     const int r = (warp & 3) * 32 + lane;
-    const int half = warp >> 2;
+    const int quarter = warp >> 2;
     auto block = [&](uint32_t col, int ncols, float* dst) {  // dst [128][ncols] = D[.][col .. col + ncols)
         const int ts = ncols + 4;
-        for (int c0 = 16 * half; c0 < ncols; c0 += 32) {
+        for (int c0 = 16 * quarter; c0 < ncols; c0 += 64) {
             float v[16];
             if (have) tc::tmem_ld16(tc::tmem_lane_addr(tmem + col, warp, c0), v);
 #pragma unroll
@@ -546,7 +538,7 @@ __device__ __forceinline__ void bwd_store_partials(uint32_t tmem, int warp, int 
         }
         __syncthreads();
         const int q4 = ncols / 4;
-        for (int q = tid; q < kHidden * q4; q += kBwdThreads) {
+        for (int q = tid; q < kHidden * q4; q += kTrnThreads) {
             const int rr = q / q4, cc = (q % q4) * 4;
             *reinterpret_cast<float4*>(dst + (size_t)rr * ncols + cc) = *reinterpret_cast<const float4*>(tile + rr * ts + cc);
         }
@@ -556,168 +548,218 @@ __device__ __forceinline__ void bwd_store_partials(uint32_t tmem, int warp, int 
     block(kTcW2, kHidden, out + kOffParamW2);
     block(kTcW1, kFeatures, out + kOffParamW1);
     // W4 (D[h][o] = dW4[o][h]) and the biases: one value per row and column, contiguous across lanes
+    const uint32_t col = quarter == 0 ? kTcW4 : quarter == 1 ? kTcB3 : quarter == 2 ? kTcB2 : kTcB1;
     float v[16];
-    if (half == 0) {
-        if (have) tc::tmem_ld16(tc::tmem_lane_addr(tmem + kTcW4, warp, 0), v);
+    if (have) tc::tmem_ld16(tc::tmem_lane_addr(tmem + col, warp, 0), v);
+    if (quarter == 0) {
 #pragma unroll
         for (int o = 0; o < kOutputs; o++) out[kOffParamW4 + o * kHidden + r] = have ? v[o] : 0.f;
-        if (have) tc::tmem_ld16(tc::tmem_lane_addr(tmem + kTcB3, warp, 0), v);
-        out[kOffParamB3 + r] = have ? v[0] : 0.f;
         if (r < kOutputs) out[kOffParamB4 + r] = db4[r];
     } else {
-        if (have) tc::tmem_ld16(tc::tmem_lane_addr(tmem + kTcB2, warp, 0), v);
-        out[kOffParamB2 + r] = have ? v[0] : 0.f;
-        if (have) tc::tmem_ld16(tc::tmem_lane_addr(tmem + kTcB1, warp, 0), v);
-        out[kOffParamB1 + r] = have ? v[0] : 0.f;
+        out[(quarter == 1 ? kOffParamB3 : quarter == 2 ? kOffParamB2 : kOffParamB1) + r] = have ? v[0] : 0.f;
     }
 }
 
-__global__ void __launch_bounds__(kBwdThreads, 1) k_mlp_backward(const bf16* __restrict__ dy, const Saves S,
-                                                                 const bf16* __restrict__ w2t,
-                                                                 const bf16* __restrict__ w3t,
-                                                                 const bf16* __restrict__ w4t, int batch,
-                                                                 float* __restrict__ part, uint32_t* err) {
-    extern __shared__ __align__(1024) uint8_t smem[];
+__global__ void __launch_bounds__(kTrnThreads, 1) k_mlp_train(const float* __restrict__ x, const float* __restrict__ t,
+                                                              int batch, const Packed W, float* __restrict__ part,
+                                                              float* __restrict__ loss_part, uint32_t* err) {
+    extern __shared__ __align__(128) uint8_t smem[];
     __shared__ uint64_t bar;
     __shared__ uint32_t tmem_base;
     __shared__ float db4s[4][kOutputs];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    uint8_t* hb[2] = {smem + kBOffH, smem + kBOffH + kHidden * kTile * 2};
+    const int r = tid & 127, quarter = warp >> 2, c0 = 32 * quarter;
     const int ntiles = batch / kTile;
-    int t = blockIdx.x;
-    if (t < ntiles) {  // the first tile's H3^T and H2^T, in flight while the weights are staged
-        issue_h_tile(hb[0], S.h3t, kHidden, S.ldh, t * kTile, tid);
-        issue_h_tile(hb[1], S.h2t, kHidden, S.ldh, t * kTile, tid);
-    }
-    stage_weights(smem + kBOffW4t, w4t, kHidden, kOutPad, tid, kBwdThreads);
-    stage_weights(smem + kBOffW3t, w3t, kHidden, kHidden, tid, kBwdThreads);
-    stage_weights(smem + kBOffW2t, w2t, kHidden, kHidden, tid, kBwdThreads);
-    {
-        const bf16 one = __float2bfloat16_rn(1.f);
-        for (int q = tid; q < kOutPad * kTile; q += kBwdThreads)
-            *reinterpret_cast<bf16*>(smem + kBOffOnes + tc::kmajor_offset(q / kTile, q % kTile, kTile)) = one;
-    }
+    float* bias = reinterpret_cast<float*>(smem + kTOffBias);
+    float* norm = reinterpret_cast<float*>(smem + kTOffNorm);
+
+    stage_weights(smem + kTOffW1, W.w1, kHidden, kFeatures, kInPad, tid, kTrnThreads);
+    cp_async_commit();
+    stage_weights(smem + kTOffW2, W.w2, kHidden, kHidden, kHidden, tid, kTrnThreads);
+    stage_weights(smem + kTOffW3, W.w3, kHidden, kHidden, kHidden, tid, kTrnThreads);
+    stage_weights(smem + kTOffW4, W.w4, kOutPad, kHidden, kHidden, tid, kTrnThreads);
+    cp_async_commit();
+    InputTile<kTrnThreads> in;
+    in.load(x, blockIdx.x * kTile, batch, tid);
+    stage_constants(W, bias, norm, tid, kTrnThreads);
+    if (tid < 32)  // bf16 ones
+        *reinterpret_cast<uint4*>(smem + kTOffOnes + 16 * tid) = make_uint4(0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u);
     if (warp == 0) {
-        tc::tmem_alloc(&tmem_base, kBwdTmemCols);
+        tc::tmem_alloc(&tmem_base, kTrnTmemCols);
         tc::tmem_relinquish();
     }
     if (tid == 0) tc::mbar_init(&bar, 1);
-    tc::fence_async_smem();
-    tc::fence_before_sync();
-    __syncthreads();
+    cp_async_wait<1>();  // W1; the others before layer 2
+    handoff_to_mma();
     tc::fence_after_sync();
     const uint32_t tmem = tmem_base;
-    const uint32_t a_w4t = tc::smem_addr(smem + kBOffW4t), a_w3t = tc::smem_addr(smem + kBOffW3t);
-    const uint32_t a_w2t = tc::smem_addr(smem + kBOffW2t), a_ones = tc::smem_addr(smem + kBOffOnes);
-    const uint32_t a_dy = tc::smem_addr(smem + kBOffDy), a_dyt = tc::smem_addr(smem + kBOffDyt);
-    const uint32_t a_dz = tc::smem_addr(smem + kBOffDz), a_dzt = tc::smem_addr(smem + kBOffDzt);
-    const uint32_t a_h[2] = {tc::smem_addr(hb[0]), tc::smem_addr(hb[1])};
-    const int r = (warp & 3) * 32 + lane;
+    auto at = [&](int off) { return tc::smem_addr(smem + off); };
+    constexpr int kSteps = kTile / 16;
+    // operands: a tile of kc columns by rows, transposed, and the ones
+    auto rows = [](uint32_t a, int kc) { return [a, kc](int ks) { return tc::kmajor_desc(a, kc, ks); }; };
+    auto cols = [](uint32_t a, int kc) { return [a, kc](int ks) { return tc::mnmajor_desc(a, kc, ks); }; };
+    auto ones = [&](int) { return tc::kmajor_desc(at(kTOffOnes), 16, 0); };
     float db4[kOutputs] = {0.f, 0.f, 0.f, 0.f};
     uint32_t parity = 0;
-    bool ok = true;
-    int done = 0;  // tiles of this CTA finished (the accumulators hold data once it is > 0)
-    for (; t < ntiles && ok; t += gridDim.x) {
-        const int row0 = t * kTile;
-        const int tn = t + gridDim.x;  // the next tile of this CTA
-        const bool acc = done > 0;
-        // dY [rows][16] and dY^T [16][rows] from the output gradient (bf16 [batch][16], zero padded)
-        if (warp < 4) {
-            const uint4* src = reinterpret_cast<const uint4*>(dy + (size_t)(row0 + r) * kOutPad);
-            const uint4 lo = src[0], hi = src[1];
-            *reinterpret_cast<uint4*>(smem + kBOffDy + tc::kmajor_offset(r, 0, kOutPad)) = lo;
-            *reinterpret_cast<uint4*>(smem + kBOffDy + tc::kmajor_offset(r, 8, kOutPad)) = hi;
-            const bf16* e = reinterpret_cast<const bf16*>(&lo);
-            const bf16* e2 = reinterpret_cast<const bf16*>(&hi);
+    bool ok = true, any = false;
+    uint32_t z1[16], z2[16], z3[16];  // this thread's row and columns, FP16 pairs
+    uint32_t v[2][16];
+    auto load_d = [&]() {
+        tc::tmem_issue16(tc::tmem_lane_addr(tmem + kTcD, warp, c0), v[0]);
+        tc::tmem_issue16(tc::tmem_lane_addr(tmem + kTcD, warp, c0 + 16), v[1]);
+        tc::tmem_wait16(v[0]);
+        tc::tmem_wait16(v[1]);
+    };
+    // H = SiLU(Z) into the tile at off
+    auto forward_epilogue = [&](const float* hb, int off, uint32_t(&z)[16]) {
+        load_d();
+        silu16<true>(v[0], c0, hb, smem + off, r, z);
+        silu16<true>(v[1], c0 + 16, hb, smem + off, r, z + 8);
+    };
+    // dZ = dH * SiLU'(Z) into the tile at off
+    auto backward_epilogue = [&](const uint32_t(&z)[16], int off) {
+        load_d();
 #pragma unroll
-            for (int o = 0; o < 8; o++) {
-                *reinterpret_cast<bf16*>(smem + kBOffDyt + tc::kmajor_offset(o, r, kTile)) = e[o];
-                *reinterpret_cast<bf16*>(smem + kBOffDyt + tc::kmajor_offset(o + 8, r, kTile)) = e2[o];
+        for (int c = 0; c < 4; c++) {
+            uint32_t w[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const float2 zz = __half22float2(*reinterpret_cast<const __half2*>(&z[4 * c + k]));
+                w[k] = pack2(__uint_as_float(v[c >> 1][8 * (c & 1) + 2 * k]) * silu_grad(zz.x),
+                             __uint_as_float(v[c >> 1][8 * (c & 1) + 2 * k + 1]) * silu_grad(zz.y));
+            }
+            *reinterpret_cast<uint4*>(smem + off + tc::kmajor_offset(r, c0 + 8 * c, kHidden)) =
+                make_uint4(w[0], w[1], w[2], w[3]);
+        }
+    };
+    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+        const int row0 = tile * kTile;
+        float4 target = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (quarter == 0) target = load_early(reinterpret_cast<const float4*>(t) + row0 + r);
+        in.store(row0, batch, norm, norm + kFeatures, smem + kTOffH0, tid);
+        handoff_to_mma();
+        if (tid == 0) {
+            tc::fence_after_sync();
+            issue_layer(tmem + kTcD, at(kTOffH0), at(kTOffW1), kFeatures, kHidden, &bar);
+        }
+        if (!(ok = wait_all(&bar, parity))) break;
+        forward_epilogue(bias, kTOffH1, z1);
+        cp_async_wait<0>();
+        handoff_to_mma();
+        if (tid == 0) {
+            tc::fence_after_sync();
+            issue_layer(tmem + kTcD, at(kTOffH1), at(kTOffW2), kHidden, kHidden, &bar);
+        }
+        if (!(ok = wait_all(&bar, parity))) break;
+        forward_epilogue(bias + kHidden, kTOffH2, z2);
+        handoff_to_mma();
+        if (tid == 0) {
+            tc::fence_after_sync();
+            issue_layer(tmem + kTcD, at(kTOffH2), at(kTOffW3), kHidden, kHidden, &bar);
+        }
+        if (!(ok = wait_all(&bar, parity))) break;
+        forward_epilogue(bias + 2 * kHidden, kTOffH3, z3);
+        handoff_to_mma();
+        if (tid == 0) {  // N = 16: outputs 0..3 and zero padding
+            tc::fence_after_sync();
+            issue_layer(tmem + kTcD, at(kTOffH3), at(kTOffW4), kHidden, kOutPad, &bar);
+        }
+        if (!(ok = wait_all(&bar, parity))) break;
+        if (quarter == 0) {  // dY [rows][16] (bf16, zero padded), the warp's sum of squared errors
+            float o[16];
+            tc::tmem_ld16(tc::tmem_lane_addr(tmem + kTcD, warp, 0), o);
+            const float* b4 = bias + 3 * kHidden;
+            const float d[4] = {(o[0] + b4[0]) - target.x, (o[1] + b4[1]) - target.y, (o[2] + b4[2]) - target.z,
+                                (o[3] + b4[3]) - target.w};
+            const float s = 2.f / (float)batch;
+            const uint32_t q[2] = {pack2(s * d[0], s * d[1]), pack2(s * d[2], s * d[3])};
+            *reinterpret_cast<uint4*>(smem + kTOffDy + tc::kmajor_offset(r, 0, kOutPad)) = make_uint4(q[0], q[1], 0u, 0u);
+            *reinterpret_cast<uint4*>(smem + kTOffDy + tc::kmajor_offset(r, 8, kOutPad)) = make_uint4(0u, 0u, 0u, 0u);
+            float se = 0.f;
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                se += d[k] * d[k];
+                db4[k] += __bfloat162float(reinterpret_cast<const bf16*>(q)[k]);
             }
 #pragma unroll
-            for (int o = 0; o < kOutputs; o++) db4[o] += __bfloat162float(e[o]);
+            for (int k = 16; k > 0; k >>= 1) se += __shfl_xor_sync(0xffffffffu, se, k);
+            if (lane == 0) loss_part[(row0 + r) >> 5] = se;
         }
-        __half zb[64];
-        load_z_half(S.z3, S.ldh, row0, r, warp >> 2, zb);  // in flight while the MMAs run
-        cp_async_wait<1>();  // H3^T
         handoff_to_mma();
         if (tid == 0) {
             tc::fence_after_sync();
-            mma_chain(tmem + kTcW4, a_h[0], a_dyt, kTile, kTile / 16, kOutPad, acc);  // dW4^T += H3^T dY
-            mma_chain(tmem + kTcDh, a_dy, a_w4t, kOutPad, 1, kHidden, false);          // dH3 = dY W4
+            mma_chain(tmem + kTcD, rows(at(kTOffDy), kOutPad), cols(at(kTOffW4), kHidden), 1,
+                      tc::idesc_bf16_f32(kTile, kHidden, false, true), false);  // dH3 = dY W4
             tc::mma_commit(&bar);
+            mma_chain(tmem + kTcW4, cols(at(kTOffH3), kHidden), cols(at(kTOffDy), kOutPad), kSteps,
+                      tc::idesc_bf16_f32(kTile, kOutPad, true, true), any);  // dW4^T += H3^T dY
         }
         if (!(ok = wait_all(&bar, parity))) break;
-        issue_h_tile(hb[0], S.h1t, kHidden, S.ldh, row0, tid);
-        bwd_epilogue(tmem + kTcDh, warp, lane, smem + kBOffDz, smem + kBOffDzt, zb);
-        load_z_half(S.z2, S.ldh, row0, r, warp >> 2, zb);
-        cp_async_wait<1>();  // H2^T
+        backward_epilogue(z3, kTOffDz);
         handoff_to_mma();
         if (tid == 0) {
             tc::fence_after_sync();
-            mma_chain(tmem + kTcW3, a_dzt, a_h[1], kTile, kTile / 16, kHidden, acc);  // dW3 += dZ3^T H2
-            mma_chain(tmem + kTcB3, a_dzt, a_ones, kTile, kTile / 16, kOutPad, acc);  // db3 (every column)
-            mma_chain(tmem + kTcDh, a_dz, a_w3t, kHidden, kHidden / 16, kHidden, false);  // dH2 = dZ3 W3
+            mma_chain(tmem + kTcD, rows(at(kTOffDz), kHidden), cols(at(kTOffW3), kHidden), kSteps,
+                      tc::idesc_bf16_f32(kTile, kHidden, false, true), false);  // dH2 = dZ3 W3
             tc::mma_commit(&bar);
+            mma_chain(tmem + kTcW3, cols(at(kTOffDz), kHidden), cols(at(kTOffH2), kHidden), kSteps,
+                      tc::idesc_bf16_f32(kTile, kHidden, true, true), any);  // dW3 += dZ3^T H2
+            mma_chain(tmem + kTcB3, cols(at(kTOffDz), kHidden), ones, kSteps,
+                      tc::idesc_bf16_f32(kTile, kOutPad, true, false), any);  // db3 (every column)
         }
         if (!(ok = wait_all(&bar, parity))) break;
-        issue_h_tile(hb[1], S.h0t, kInPad, S.ldh, row0, tid);
-        bwd_epilogue(tmem + kTcDh, warp, lane, smem + kBOffDz, smem + kBOffDzt, zb);
-        load_z_half(S.z1, S.ldh, row0, r, warp >> 2, zb);
-        cp_async_wait<1>();  // H1^T
+        backward_epilogue(z2, kTOffH3);
+        if (tile + (int)gridDim.x < ntiles) in.load(x, row0 + (int)gridDim.x * kTile, batch, tid);
         handoff_to_mma();
         if (tid == 0) {
             tc::fence_after_sync();
-            mma_chain(tmem + kTcW2, a_dzt, a_h[0], kTile, kTile / 16, kHidden, acc);  // dW2 += dZ2^T H1
-            mma_chain(tmem + kTcB2, a_dzt, a_ones, kTile, kTile / 16, kOutPad, acc);
-            mma_chain(tmem + kTcDh, a_dz, a_w2t, kHidden, kHidden / 16, kHidden, false);  // dH1 = dZ2 W2
+            mma_chain(tmem + kTcD, rows(at(kTOffH3), kHidden), cols(at(kTOffW2), kHidden), kSteps,
+                      tc::idesc_bf16_f32(kTile, kHidden, false, true), false);  // dH1 = dZ2 W2
             tc::mma_commit(&bar);
+            mma_chain(tmem + kTcW2, cols(at(kTOffH3), kHidden), cols(at(kTOffH1), kHidden), kSteps,
+                      tc::idesc_bf16_f32(kTile, kHidden, true, true), any);  // dW2 += dZ2^T H1
+            mma_chain(tmem + kTcB2, cols(at(kTOffH3), kHidden), ones, kSteps,
+                      tc::idesc_bf16_f32(kTile, kOutPad, true, false), any);  // db2
         }
         if (!(ok = wait_all(&bar, parity))) break;
-        if (tn < ntiles) issue_h_tile(hb[0], S.h3t, kHidden, S.ldh, tn * kTile, tid);
-        bwd_epilogue(tmem + kTcDh, warp, lane, nullptr, smem + kBOffDzt, zb);
-        if (tn < ntiles) cp_async_wait<1>();  // H0^T (the next tile's H3^T may still be in flight)
-        else cp_async_wait<0>();
+        backward_epilogue(z1, kTOffDz);
         handoff_to_mma();
         if (tid == 0) {
             tc::fence_after_sync();
-            mma_chain(tmem + kTcW1, a_dzt, a_h[1], kTile, kTile / 16, kInPad, acc);  // dW1 += dZ1^T H0
-            mma_chain(tmem + kTcB1, a_dzt, a_ones, kTile, kTile / 16, kOutPad, acc);
+            mma_chain(tmem + kTcW1, cols(at(kTOffDz), kHidden), cols(at(kTOffH0), kFeatures), kSteps,
+                      tc::idesc_bf16_f32(kTile, kFeatures, true, true), any);  // dW1 += dZ1^T H0
+            mma_chain(tmem + kTcB1, cols(at(kTOffDz), kHidden), ones, kSteps,
+                      tc::idesc_bf16_f32(kTile, kOutPad, true, false), any);  // db1
             tc::mma_commit(&bar);
         }
-        if (!(ok = wait_all(&bar, parity))) break;
-        if (tn < ntiles) issue_h_tile(hb[1], S.h2t, kHidden, S.ldh, tn * kTile, tid);
-        done++;
+        if (!(ok = wait_all(&bar, parity))) break;  // the tile's operands are free
+        any = true;
     }
     cp_async_wait<0>();
     if (!ok) {
         if (tid == 0) atomicOr(err, kErrMmaTimeout);
         tc::mbar_wait(&bar, parity ^ 1u, tc::kWaitLimitNs);  // the chain still in flight, bounded
     }
-    // db4: the sum over this CTA's rows (warps 0-3), in a fixed order
+    // db4: the sum over this CTA's rows (held by warps 0-3), in a fixed order
 #pragma unroll
     for (int o = 0; o < kOutputs; o++) {
-        float v = db4[o];
+        float s = db4[o];
 #pragma unroll
-        for (int d = 16; d > 0; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
-        if (lane == 0 && warp < 4) db4s[warp][o] = v;
+        for (int d = 16; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
+        if (lane == 0 && quarter == 0) db4s[warp][o] = s;
     }
     __syncthreads();
     float db4t[kOutputs];
 #pragma unroll
-    for (int o = 0; o < kOutputs; o++) db4t[o] = db4s[0][o] + db4s[1][o] + db4s[2][o] + db4s[3][o];
-    bwd_store_partials(tmem, warp, lane, tid, ok && done > 0, db4t, reinterpret_cast<float*>(smem + kBOffDz),
-                       part + (size_t)blockIdx.x * kParams);
+    for (int o = 0; o < kOutputs; o++) db4t[o] = (db4s[0][o] + db4s[1][o]) + (db4s[2][o] + db4s[3][o]);
+    store_partials(tmem, warp, lane, tid, ok && any, db4t, reinterpret_cast<float*>(smem + kTOffH1),
+                   part + (size_t)blockIdx.x * kParams);
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
-    if (warp == 0) tc::tmem_dealloc(tmem_base, kBwdTmemCols);
+    if (warp == 0) tc::tmem_dealloc(tmem_base, kTrnTmemCols);
 }
 
-// grads[p] = the sum over the CTAs' partials: 64 parameters per block, four
-// threads per parameter summing every fourth CTA's partial (a warp reads 32
-// consecutive parameters of one partial), the four sums added in a fixed order;
-// with an Adam step (adam.lr > 0) the parameter is updated in the same pass.
 // Parameter p (flat layout) into its bf16 operand positions, as k_pack writes them.
 __device__ __forceinline__ void pack_param(const PackedMut& W, int p, float val) {
     const bf16 b = __float2bfloat16_rn(val);
@@ -725,40 +767,52 @@ __device__ __forceinline__ void pack_param(const PackedMut& W, int p, float val)
         W.w1[(p / kFeatures) * kInPad + p % kFeatures] = b;
     } else if (p < kOffParamW2) {
         W.bias[p - kOffParamB1] = val;
-    } else if (p < kOffParamB2) {  // W2 [128][128], and transposed
-        const int i = p - kOffParamW2;
-        W.w2[i] = b;
-        W.w2t[(i % kHidden) * kHidden + i / kHidden] = b;
+    } else if (p < kOffParamB2) {
+        W.w2[p - kOffParamW2] = b;
     } else if (p < kOffParamW3) {
         W.bias[kHidden + p - kOffParamB2] = val;
     } else if (p < kOffParamB3) {
-        const int i = p - kOffParamW3;
-        W.w3[i] = b;
-        W.w3t[(i % kHidden) * kHidden + i / kHidden] = b;
+        W.w3[p - kOffParamW3] = b;
     } else if (p < kOffParamW4) {
         W.bias[2 * kHidden + p - kOffParamB3] = val;
-    } else if (p < kOffParamB4) {  // W4 [4][128] -> w4 [16][128], w4t [128][16]
-        const int i = p - kOffParamW4;
-        W.w4[i] = b;
-        W.w4t[(i % kHidden) * kOutPad + i / kHidden] = b;
+    } else if (p < kOffParamB4) {  // W4 [4][128] -> w4 [16][128]
+        W.w4[p - kOffParamW4] = b;
     } else {
         W.bias[3 * kHidden + p - kOffParamB4] = val;
     }
 }
 
-constexpr int kSumParams = 64;
-__global__ void __launch_bounds__(4 * kSumParams) k_sum_partials(const float* __restrict__ part, int nparts,
-                                                                 float* __restrict__ grads, const AdamStep adam) {
-    __shared__ float sh[4][kSumParams];
-    const int j = threadIdx.x / kSumParams, q = threadIdx.x % kSumParams;
-    const int p = blockIdx.x * kSumParams + q;
-    float s = 0.f;
-    if (p < kParams)
-        for (int k = j; k < nparts; k += 4) s += part[(size_t)k * kParams + p];
+// grads[p] = the sum over the CTAs' partials: 128 parameters per block, eight
+// threads per four parameters summing every eighth CTA's partial (a warp reads 512
+// contiguous bytes of one partial), the eight sums added in a fixed order; with an
+// Adam step (adam.lr > 0) the parameter is updated in the same pass. Bound by the
+// latency of reading the partials from L2 (152 of 159 KB: 24 MB), so every
+// thread keeps eight 16-byte loads in flight. (With 4-byte loads, four threads per
+// parameter: 10.8 us instead of 7.1.)
+constexpr int kSumParams = 128, kSumSlices = 8;
+static_assert(kParams % 4 == 0, "16-byte loads of the partials");
+__global__ void __launch_bounds__(kSumSlices* kSumParams / 4) k_sum_partials(const float* __restrict__ part, int nparts,
+                                                                             float* __restrict__ grads,
+                                                                             const AdamStep adam) {
+    __shared__ float4 sh[kSumSlices][kSumParams / 4];
+    const int j = threadIdx.x / (kSumParams / 4), q = threadIdx.x % (kSumParams / 4);
+    const int p4 = blockIdx.x * (kSumParams / 4) + q;
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (p4 < kParams / 4) {
+        const float4* src = reinterpret_cast<const float4*>(part) + p4;
+#pragma unroll 8
+        for (int k = j; k < nparts; k += kSumSlices) {
+            const float4 v = __ldg(src + (size_t)k * (kParams / 4));
+            s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+        }
+    }
     sh[j][q] = s;
     __syncthreads();
-    if (j != 0 || p >= kParams) return;
-    const float g = (sh[0][q] + sh[1][q]) + (sh[2][q] + sh[3][q]);
+    const int p = blockIdx.x * kSumParams + threadIdx.x;
+    if (threadIdx.x >= kSumParams || p >= kParams) return;
+    float g = 0.f;
+#pragma unroll
+    for (int k = 0; k < kSumSlices; k++) g += reinterpret_cast<const float*>(sh[k])[threadIdx.x];
     grads[p] = g;
     if (adam.lr > 0.f) {
         const float mi = adam.b1 * adam.m[p] + (1.f - adam.b1) * g;
@@ -774,42 +828,6 @@ __global__ void __launch_bounds__(4 * kSumParams) k_sum_partials(const float* __
 // ---------------------------------------------------------------------------
 // Backward and optimiser helpers
 // ---------------------------------------------------------------------------
-
-// dY = 2 (y - t) / batch (the gradient of the mean over the batch of the
-// squared output error), bf16, row-major [batch][16] and transposed [16][ld];
-// per-block partial sums of the squared error.
-__global__ void k_out_grad(const float4* __restrict__ y, const float4* __restrict__ t, int batch, int ld,
-                           bf16* __restrict__ dy, bf16* __restrict__ dyt, float* __restrict__ loss_part) {
-    __shared__ float red[256 / 32];
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    float se = 0.f;
-    if (i < batch) {
-        const float4 a = y[i], b = t[i];
-        const float d[4] = {a.x - b.x, a.y - b.y, a.z - b.z, a.w - b.w};
-        const float s = 2.f / (float)batch;
-        uint4 lo, hi = make_uint4(0u, 0u, 0u, 0u);
-        lo.x = pack2(s * d[0], s * d[1]);
-        lo.y = pack2(s * d[2], s * d[3]);
-        lo.z = 0u;
-        lo.w = 0u;
-        reinterpret_cast<uint4*>(dy + (size_t)i * kOutPad)[0] = lo;
-        reinterpret_cast<uint4*>(dy + (size_t)i * kOutPad)[1] = hi;
-#pragma unroll
-        for (int o = 0; o < 4; o++) {
-            if (dyt) dyt[(size_t)o * ld + i] = __float2bfloat16_rn(s * d[o]);
-            se += d[o] * d[o];
-        }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) se += __shfl_xor_sync(0xffffffffu, se, o);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = se;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        float s = 0.f;
-        for (int w = 0; w < (int)(blockDim.x >> 5); w++) s += red[w];
-        loss_part[blockIdx.x] = s;
-    }
-}
 
 // loss = sum of the partials / batch (one block, fixed order)
 __global__ void k_loss_sum(const float* __restrict__ part, int nparts, int batch, float* __restrict__ loss) {
@@ -837,18 +855,13 @@ __global__ void k_pack(const float* __restrict__ p, PackedMut W) {
         const int o = i / kInPad, k = i % kInPad;
         W.w1[i] = __float2bfloat16_rn(k < kFeatures ? w1[o * kFeatures + k] : 0.f);
     }
-    if (i < kHidden * kHidden) {  // w2, w3 and their transposes
-        const int o = i / kHidden, k = i % kHidden;
+    if (i < kHidden * kHidden) {
         W.w2[i] = __float2bfloat16_rn(w2[i]);
         W.w3[i] = __float2bfloat16_rn(w3[i]);
-        W.w2t[k * kHidden + o] = __float2bfloat16_rn(w2[i]);
-        W.w3t[k * kHidden + o] = __float2bfloat16_rn(w3[i]);
     }
-    if (i < kOutPad * kHidden) {  // w4 [16][128], w4t [128][16]
+    if (i < kOutPad * kHidden) {  // w4 [16][128]
         const int o = i / kHidden, k = i % kHidden;
-        const float v = o < kOutputs ? w4[o * kHidden + k] : 0.f;
-        W.w4[i] = __float2bfloat16_rn(v);
-        W.w4t[k * kOutPad + o] = __float2bfloat16_rn(v);
+        W.w4[i] = __float2bfloat16_rn(o < kOutputs ? w4[o * kHidden + k] : 0.f);
     }
     if (i < 3 * kHidden + kOutPad) {
         float b;
@@ -866,16 +879,15 @@ __global__ void k_pack(const float* __restrict__ p, PackedMut W) {
 // launchers
 // ---------------------------------------------------------------------------
 
-cudaError_t launch_forward(const float* x, int n, const Packed& W, const Saves& S, float* y, uint32_t* err,
-                           int num_sms, cudaStream_t s) {
+cudaError_t launch_forward(const float* x, int n, const Packed& W, float* y, uint32_t* err, int num_sms,
+                           cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
+    const int tiles = (n + kTile - 1) / kTile;
     // per call (a host-side attribute of the current device): threads and devices stay independent
     cudaError_t e = cudaFuncSetAttribute(k_mlp_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, kFwdSmem);
     if (e != cudaSuccess) return e;
-    const int tiles = (n + kTile - 1) / kTile;
-    const int pairs = (tiles + kGroups - 1) / kGroups;
-    const int grid = pairs < num_sms ? pairs : num_sms;
-    k_mlp_forward<<<grid, kFwdThreads, kFwdSmem, s>>>(x, n, W, S, y, err);
+    const int grid = tiles < num_sms ? tiles : num_sms;
+    k_mlp_forward<<<grid, kFwdThreads, kFwdSmem, s>>>(x, n, W, y, err);
     return cudaGetLastError();
 }
 
@@ -894,27 +906,17 @@ cudaError_t launch_gemm_tn(const bf16* A, int lda, const bf16* B, int ldb, float
     return cudaGetLastError();
 }
 
-cudaError_t launch_out_grad(const float* y, const float* t, int batch, int ld, bf16* dy, bf16* dyt, float* loss_part,
-                            float* loss, cudaStream_t s) {
-    const int blocks = (batch + 255) / 256;
-    k_out_grad<<<blocks, 256, 0, s>>>(reinterpret_cast<const float4*>(y), reinterpret_cast<const float4*>(t), batch,
-                                      ld, dy, dyt, loss_part);
-    if (loss) k_loss_sum<<<1, 256, 0, s>>>(loss_part, blocks, batch, loss);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_backward(const bf16* dy, const Saves& S, const PackedMut& W, int batch, float* part,
-                            float* grads, const AdamStep& adam, uint32_t* err, int num_sms, cudaStream_t s) {
-    // the saved inputs are copied 16 bytes at a time: their row stride must keep that alignment
-    if (batch <= 0 || batch % kTile != 0 || !S.z1 || !S.h0t || S.ldh % 8 != 0 || S.ldh < batch)
-        return cudaErrorInvalidValue;
-    cudaError_t e = cudaFuncSetAttribute(k_mlp_backward, cudaFuncAttributeMaxDynamicSharedMemorySize, kBwdSmem);
+cudaError_t launch_train(const float* x, const float* t, int batch, const Packed& W, float* part, float* loss_part,
+                         float* grads, const AdamStep& adam, float* loss, uint32_t* err, int num_sms, cudaStream_t s) {
+    if (batch <= 0 || batch % kTile != 0) return cudaErrorInvalidValue;
+    cudaError_t e = cudaFuncSetAttribute(k_mlp_train, cudaFuncAttributeMaxDynamicSharedMemorySize, kTrnSmem);
     if (e != cudaSuccess) return e;
     const int tiles = batch / kTile;
     const int grid = tiles < num_sms ? tiles : num_sms;
-    k_mlp_backward<<<grid, kBwdThreads, kBwdSmem, s>>>(dy, S, W.w2t, W.w3t, W.w4t, batch, part, err);
+    k_mlp_train<<<grid, kTrnThreads, kTrnSmem, s>>>(x, t, batch, W, part, loss_part, err);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    k_sum_partials<<<(kParams + kSumParams - 1) / kSumParams, 4 * kSumParams, 0, s>>>(part, grid, grads, adam);
+    if (loss) k_loss_sum<<<1, 256, 0, s>>>(loss_part, batch / 32, batch, loss);
+    k_sum_partials<<<(kParams + kSumParams - 1) / kSumParams, kSumSlices * kSumParams / 4, 0, s>>>(part, grid, grads, adam);
     return cudaGetLastError();
 }
 

@@ -45,21 +45,12 @@ struct Packed {
 
 struct PackedMut {
     __nv_bfloat16 *w1, *w2, *w3, *w4;
-    __nv_bfloat16 *w2t, *w3t, *w4t;  // transposes for the backward pass: [128][128], [128][128], [128][16]
     float* bias;
 };
 
-// Training saves of the forward pass (all null for inference): the hidden
-// layers' pre-activations z in FP16 and the bf16 layer inputs, all transposed
-// ([width][ldh], feature-major).
-struct Saves {
-    __half *z1, *z2, *z3;
-    __nv_bfloat16 *h0t, *h1t, *h2t, *h3t;  // h0t [64][ldh] (rows 48..63 zero), the others [128][ldh]
-    int ldh;
-};
-
-cudaError_t launch_forward(const float* x, int n, const Packed& W, const Saves& S, float* y, uint32_t* err,
-                           int num_sms, cudaStream_t s);
+// y [n][4]
+cudaError_t launch_forward(const float* x, int n, const Packed& W, float* y, uint32_t* err, int num_sms,
+                           cudaStream_t s);
 // D[split][M][N] = A[M][K] B[N][K]^T over the split's K range; N a multiple of 16, <= 128
 cudaError_t launch_gemm_tn(const __nv_bfloat16* A, int lda, const __nv_bfloat16* B, int ldb, float* D, int M, int N,
                            int K, int splits, uint32_t* err, cudaStream_t s);
@@ -74,16 +65,13 @@ struct AdamStep {
 AdamStep adam_step(float* p, float* m, float* v, float lr, float b1, float b2, float eps, int step,
                    const PackedMut& w);
 
-// The whole backward pass after launch_out_grad (fused, one persistent CTA per
-// SM): gradients of every parameter into grads (flat layout), then the Adam
-// step if adam.lr > 0. batch a multiple of 128; part: scratch of num_sms *
-// kParams floats.
-cudaError_t launch_backward(const __nv_bfloat16* dy, const Saves& S, const PackedMut& W, int batch, float* part,
-                            float* grads, const AdamStep& adam, uint32_t* err, int num_sms, cudaStream_t s);
-// dY (bf16 [batch][16], zero padded; transposed into dyt [4][ld] unless null) and
-// the loss into *loss (unless null)
-cudaError_t launch_out_grad(const float* y, const float* t, int batch, int ld, __nv_bfloat16* dy,
-                            __nv_bfloat16* dyt, float* loss_part, float* loss, cudaStream_t s);
+// Forward and backward pass of a batch in one kernel (one persistent CTA per SM):
+// the gradients of the mean over the batch of the squared output error (targets t
+// [batch][4]) by every parameter into grads (flat layout), then the Adam step if
+// adam.lr > 0; that mean into *loss unless null. batch a multiple of 128; scratch:
+// part num_sms * kParams floats, loss_part batch / 32 floats.
+cudaError_t launch_train(const float* x, const float* t, int batch, const Packed& W, float* part, float* loss_part,
+                         float* grads, const AdamStep& adam, float* loss, uint32_t* err, int num_sms, cudaStream_t s);
 cudaError_t launch_pack(const float* p, const PackedMut& W, cudaStream_t s);
 
 }  // namespace mlp

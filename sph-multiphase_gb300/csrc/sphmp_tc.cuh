@@ -43,11 +43,22 @@ __device__ __forceinline__ uint64_t kmajor_desc(uint32_t tile_addr, int kc, int 
     return smem_desc(tile_addr + (uint32_t)kstep * 256u, 128u, (uint32_t)kc * 16u);
 }
 
+// The same core matrices read the other way: an operand whose M (or N) index runs
+// along the 16 contiguous bytes and whose K index runs down the 8 rows (MN-major).
+// A tile [r][c] of kc columns stored for K-major use thus also serves as the operand
+// of its transpose: the stride between core matrices along M / N (128 bytes) goes
+// into the stride-dimension offset, the one along K (a group of 8 rows) into the
+// leading-dimension offset. One MMA consumes two core matrices along K.
+__device__ __forceinline__ uint64_t mnmajor_desc(uint32_t tile_addr, int kc, int kstep) {
+    return smem_desc(tile_addr + (uint32_t)kstep * (uint32_t)kc * 32u, (uint32_t)kc * 16u, 128u);
+}
+
 // Instruction descriptor of kind::f16: D FP32 (bits 4-5 = 1), A and B bf16
-// (bits 7-9 = 1, 10-12 = 1), both K-major (bits 15, 16 = 0), N / 8 in bits
+// (bits 7-9 = 1, 10-12 = 1), K-major or MN-major (bits 15, 16 = 0 or 1), N / 8 in bits
 // 17-22, M / 16 in bits 24-28.
-__host__ __device__ constexpr uint32_t idesc_bf16_f32(int m, int n) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
+__host__ __device__ constexpr uint32_t idesc_bf16_f32(int m, int n, bool a_mn = false, bool b_mn = false) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)a_mn << 15) | ((uint32_t)b_mn << 16) |
+           ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 
 // ---- TMEM (one full warp executes alloc / dealloc) ----
@@ -133,6 +144,24 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
     for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
+}
+
+// 16 consecutive columns of this thread's lane, queued: r holds them after
+// tmem_wait16 (which takes r, so that no use of it moves before the wait).
+__device__ __forceinline__ void tmem_issue16(uint32_t taddr, uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, "
+        "[%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_wait16(uint32_t (&r)[16]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+        : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
+          "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
+        :
+        : "memory");
 }
 
 // TMEM address of column `col` in the lane quadrant of warp `warp`
