@@ -282,9 +282,11 @@ void launch_apply_correction(const DevParams& P, const DevBuffers& B, const int*
 void launch_compare(const DevParams& Pa, const DevBuffers& Ba, const int* cur_a, const DevParams& Pb,
                     const DevBuffers& Bb, const int* cur_b, int32_t* map, int map_size, double* out, cudaStream_t s);
 
-// transfers (staging buffers hold reference records)
+// transfers (staging buffers hold reference records; the calculation records of an
+// upload calc_bytes apart, at least their first kCalcUsed bytes: all that the upload reads)
+constexpr int kCalcUsed = 64;
 void launch_unpack_aos(const DevParams& P, const DevBuffers& B, const int* cur, const sphmp_display_pack* d,
-                       const sphmp_calc_pack* c, int start, int end, cudaStream_t s);
+                       const void* c, int calc_bytes, int start, int end, cudaStream_t s);
 void launch_pack_aos(const DevParams& P, const DevBuffers& B, const int* cur, sphmp_display_pack* d,
                      sphmp_calc_pack* c, int n, cudaStream_t s);
 // field pack/unpack through a float/uint32 staging array; `aux` = alpha_pre buffer selector

@@ -1587,14 +1587,15 @@ __global__ void __launch_bounds__(kThreads) k_unpack_aos(const __grid_constant__
                                                          const __grid_constant__ DevBuffers B,
                                                          const __grid_constant__ F4Set S,
                                                          const sphmp_display_pack* __restrict__ disp,
-                                                         const sphmp_calc_pack* __restrict__ calc, int start,
+                                                         const float4* __restrict__ calc, int calc_words, int start,
                                                          int end) {
     const int i = start + blockIdx.x * kThreads + threadIdx.x;
     if (i >= end) return;
     // the records as 16-byte words: two of the display record, the first four of the
-    // calculation record's 14 (the others are the solid fields, not used here)
+    // calculation record's 14 (the others are the solid fields: not used, and not always
+    // uploaded, so that the records are 4 or 14 words apart)
     const float4* __restrict__ dq = reinterpret_cast<const float4*>(disp + (i - start));
-    const float4* __restrict__ cq = reinterpret_cast<const float4*>(calc + (i - start));
+    const float4* __restrict__ cq = calc + (size_t)(i - start) * calc_words;
     const float4 d0 = __ldcs(dq), d1 = __ldcs(dq + 1);
     const float4 c0 = __ldcs(cq), c1 = __ldcs(cq + 1), c2 = __ldcs(cq + 2), c3 = __ldcs(cq + 3);
     const sphmp_display_pack d = {{d0.x, d0.y, d0.z}, {d0.w, d1.x, d1.y, d1.z}, __float_as_int(d1.w)};
@@ -2004,9 +2005,10 @@ void launch_emit(const DevParams& P, const DevBuffers& B, const int* cur, const 
 }
 
 void launch_unpack_aos(const DevParams& P, const DevBuffers& B, const int* cur, const sphmp_display_pack* d,
-                       const sphmp_calc_pack* c, int start, int end, cudaStream_t s) {
+                       const void* c, int calc_bytes, int start, int end, cudaStream_t s) {
     if (end <= start) return;
-    k_unpack_aos<<<blocks_for(end - start), kThreads, 0, s>>>(P, B, make_set(B, cur, false), d, c, start, end);
+    k_unpack_aos<<<blocks_for(end - start), kThreads, 0, s>>>(P, B, make_set(B, cur, false), d,
+                                                             static_cast<const float4*>(c), calc_bytes / 16, start, end);
 }
 
 void launch_pack_aos(const DevParams& P, const DevBuffers& B, const int* cur, sphmp_display_pack* d,

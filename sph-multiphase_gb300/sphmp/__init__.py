@@ -273,7 +273,7 @@ class Context:
         else:
             n = self.n if n is None else n
         dt = FIELD_DTYPES.get(field, np.float32)
-        a = np.zeros((n,) + FIELD_SHAPES.get(field, ()), dt)
+        a = np.empty((n,) + FIELD_SHAPES.get(field, ()), dt)  # the call writes every element
         check(self._lib.sphmp_download_field(self._ptr, int(field), a.ctypes.data, int(n)))
         return a
 

@@ -3,6 +3,7 @@ back byte for byte (a copy), the volumes against the FP64 oracle with at most fo
 (or 2e-7, three roundings of the result)."""
 import numpy as np
 import pytest
+import torch
 
 import sphmp
 from helpers import device_ctx, oracle_state
@@ -42,6 +43,30 @@ def test_round_trip(n):
             assert (a[n:].view(np.uint8) == 0xA5).all()
         only = ctx.download_aos(n, calc=False)
         assert only.tobytes() == d.tobytes()
+
+
+@pytest.mark.parametrize("pinned", [False, True])
+@pytest.mark.parametrize("n", [1, 33, 1000])
+def test_upload_reads_no_solid_fields(n, pinned):
+    """Only the first 64 bytes of a calculation record go up; what the others hold does not matter, for an upload,
+    an append and a state copy (whole records on the device) alike."""
+    sc = scenes.small_block(seed=73, n=(16, 16, 16), nphase=3, walls=False, velocity_scale=0.5)
+    rng = np.random.default_rng(n)
+    d, c = sc.disp[:2 * n].copy(), sc.calc[:2 * n].copy()
+    want = c.copy()
+    c.view(np.uint8).reshape(2 * n, 224)[:, 60:] = rng.integers(0, 256, (2 * n, 164), dtype=np.uint8)
+    if pinned:
+        d, c = (torch.from_numpy(a.view(np.uint8)).pin_memory().numpy().view(a.dtype) for a in (d, c))
+    with sphmp.Context(sc.params) as ctx, sphmp.Context(sc.params) as other:
+        ctx.upload_aos(d[:n], c[:n])
+        ctx.emit_aos(d[n:], c[n:], n, 2 * n)
+        ctx.sync()
+        other.copy_state_from(ctx)
+        for x in (ctx, other):
+            out = x.download_aos()
+            assert out[0].tobytes() == d.tobytes()
+            for k in ("vel", "veleval", "pressure", "dens", "restdens", "mass", "visc", "bornid", "accel"):
+                assert np.array_equal(out[1][k], want[k]), k
 
 
 @pytest.mark.parametrize("kind", [(1, 1, 1), (3, 2, 5), (9, 7, 6)])
