@@ -514,7 +514,7 @@ sphmp_status enqueue_step(sphmp_ctx* c, int schedule, StageTimer* T = nullptr, c
         if (PL.multiphase) {
             run_force_drift(c, false, true, !reuse, s);
             mark("drift");
-            launch_alpha_advance(PL, c->B, c->cur, s);
+            launch_alpha_advance(PL, c->B, c->cur, true, !reuse, s);
             mark("alpha_advance");
             c->cur[ALPHA] ^= 1;
             c->alpha_advanced = true;
@@ -522,7 +522,7 @@ sphmp_status enqueue_step(sphmp_ctx* c, int schedule, StageTimer* T = nullptr, c
             mark("correction");
         }
         if (schedule == SPHMP_SCHEDULE_PROJECTU) {
-            launch_force_projectu(PL, c->B, c->cur, c->cur[ALPHA] ^ 1, s);
+            launch_force_projectu(PL, c->B, c->cur, c->cur[ALPHA] ^ 1, true, !reuse, s);
             mark("force_projectu");
         } else {
             run_force_drift(c, true, false, !reuse, s);
@@ -1055,7 +1055,7 @@ sphmp_status sphmp_compute_alpha_advance(sphmp_ctx* c) {
     if (sphmp_status st = need_grid(c)) return st;
     if (c->alpha_advanced)
         return fail(SPHMP_ERR_STATE, "volume fractions already advanced in this step (re-sort first)");
-    launch_alpha_advance(dev_params(c), c->B, c->cur, c->stream);
+    launch_alpha_advance(dev_params(c), c->B, c->cur, false, false, c->stream);
     CHECK_LAUNCH("MfComputeAlphaAdvance");
     c->cur[ALPHA] ^= 1;
     c->alpha_advanced = true;
@@ -1085,7 +1085,7 @@ sphmp_status sphmp_compute_force_projectu(sphmp_ctx* c) {
     if (sphmp_status st = need_grid(c)) return st;
     const DevParams P = dev_params(c);
     const int pre = c->alpha_advanced ? c->cur[ALPHA] ^ 1 : c->cur[ALPHA];
-    launch_force_projectu(P, c->B, c->cur, pre, c->stream);
+    launch_force_projectu(P, c->B, c->cur, pre, false, false, c->stream);
     if (P.st_on) launch_surface_tension(P, c->B, c->cur, c->stream);
     CHECK_LAUNCH("ComputeForce_projectu");
     return SPHMP_OK;

@@ -310,11 +310,12 @@ __device__ __forceinline__ float2 density_result(const DevParams& P, float wsum,
 // Force + drift velocity (MfComputeForceCUDA, MfComputeDriftVelCUDA)
 // ---------------------------------------------------------------------------
 
-// Neighbour record of particle s for the alpha pass, 80 contiguous bytes:
+// Neighbour record of particle s for the alpha and project-U passes, 80 contiguous bytes:
 //   {x, y, z, md}, {veleval xyz, alpha_0}, {alpha_1, alpha_2, u_0x, u_0y},
-//   {u_0z, u_1xyz}, {u_2xyz, 0}
+//   {u_0z, u_1xyz}, {u_2xyz, w}
 // with md = mass * (1/rho) for fluid particles and -1 for boundary particles
-// (which exchange no volume fraction), u_k the drift velocities. (A 96-byte
+// (which exchange no volume fraction), u_k the drift velocities, w that of pos4
+// (the mass, or minus the volume of a boundary particle). (A 96-byte
 // record read with three 32-byte loads measured slower: 0.314 against
 // 0.295 ms per alpha pass, from the larger records missing L2.)
 __device__ __forceinline__ void write_nrec(const DevBuffers& B, int s, const float4 p, float md, const float4 ve,
@@ -324,7 +325,7 @@ __device__ __forceinline__ void write_nrec(const DevBuffers& B, int s, const flo
     r[1] = make_float4(ve.x, ve.y, ve.z, a[0]);
     r[2] = make_float4(a[1], a[2], u[0], u[1]);
     r[3] = make_float4(u[2], u[3], u[4], u[5]);
-    r[4] = make_float4(u[6], u[7], u[8], 0.f);
+    r[4] = make_float4(u[6], u[7], u[8], p.w);
 }
 
 // The five float4 of neighbour j's record (the fifth only with three phases).
@@ -485,16 +486,14 @@ struct ForceDrift {
                 out[k].z -= cs * (st[k].z - ssum.z);
                 B.drift4[(size_t)k * P.cap + s] = make_float4(out[k].x, out[k].y, out[k].z, 0.f);
             }
-            if (FORCE) {
-                float u[9] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+            float u[9] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-                for (int k = 0; k < NP; k++) {
-                    u[3 * k] = out[k].x;
-                    u[3 * k + 1] = out[k].y;
-                    u[3 * k + 2] = out[k].z;
-                }
-                write_nrec(B, s, pi, pi.w * idens, vev, ia, u);
+            for (int k = 0; k < NP; k++) {
+                u[3 * k] = out[k].x;
+                u[3 * k + 1] = out[k].y;
+                u[3 * k + 2] = out[k].z;
             }
+            write_nrec(B, s, pi, pi.w * idens, vev, ia, u);
         }
     }
 };
@@ -582,6 +581,17 @@ struct ProjectU {
         const float ave = 2.f / (1.f / dj + 1.f / idens);
         const float xt = cx * cx * cx * mj * ave * P.kpoly6 * 0.5f;
         xx -= vx * xt; xy -= vy * xt; xz -= vz * xt;
+    }
+
+    // Sum the partial sums of the L lanes that share a particle.
+    template <int L>
+    __device__ __forceinline__ void reduce() {
+        fx = group_sum<L>(fx);
+        fy = group_sum<L>(fy);
+        fz = group_sum<L>(fz);
+        xx = group_sum<L>(xx);
+        xy = group_sum<L>(xy);
+        xz = group_sum<L>(xz);
     }
 };
 

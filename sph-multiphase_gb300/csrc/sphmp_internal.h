@@ -43,7 +43,7 @@ constexpr int kWarpSortMax = 256;     // cells up to this size are sorted by one
 constexpr int kCtaSortMax = 8192;     // larger cells up to this size are sorted by one CTA
 constexpr int kNumFloat4Fields = 5;   // pos4, vel4, vev4, alpha4, aprev4
 constexpr int kMaxNbr = 256;          // index-list capacity per particle (more: the passes rescan)
-constexpr int kNrecFloat4 = 5;        // float4 per neighbour record of the alpha pass
+constexpr int kNrecFloat4 = 5;        // float4 per neighbour record of the alpha and project-U passes
 // Bucket neighbour lists: a bitmask over the bucket's candidate sequence (the 27
 // h-subcells around it as 18 index ranges), one word per 32 candidates.
 constexpr int kMaskWords = 64;        // mask words per particle (more candidates: the passes rescan)
@@ -154,7 +154,7 @@ struct DevBuffers {
     uint32_t* wq_n;     // [1] entries in wq (filled by the cell sort)
     uint32_t* hq;       // [cap] heavy particles (internal index), filled by the density pass
     uint32_t* hq_n;     // [1] entries in hq
-    uint32_t* hctr;     // [3] work counters over hq of the drift (or force + drift), force and alpha passes
+    uint32_t* hctr;     // [3] work counters over hq of the drift (or force + drift), force (or project-U) and alpha passes
     // IISPH step (sphmp_iisph.cu): d_ii, sum_j d_ij p_j, d_ii p_l + sum_j d_ij p_j (float4,
     // w unused), a_ii, the predicted density, the pressure iterate p_l, p_l m / rho^2
     float4* iis_dii;
@@ -167,7 +167,7 @@ struct DevBuffers {
     uint32_t* iis_ctl;  // [4] finished blocks of the running iteration, 1 when the solve has ended, iterations,
                         // particles in iis_list
     uint32_t* iis_list; // [cap] in-grid fluid particles with IISPH lists (any order)
-    float4* nrec;       // [kNrecFloat4 * cap] neighbour records of the alpha pass (written by force + drift)
+    float4* nrec;       // [kNrecFloat4 * cap] neighbour records of the alpha and project-U passes (written by the drift pass)
     // Internal order: inside every 2h cell, members grouped by the h-subcell
     // (octant) they occupy, octant index (oy * 2 + oz) * 2 + ox.
     uint32_t* opos;     // [cap] internal index of each reference slot
@@ -241,9 +241,11 @@ void launch_force_drift(const DevParams& P, const DevBuffers& B, const int* cur,
                         cudaStream_t s);
 void launch_surface_tension(const DevParams& P, const DevBuffers& B, const int* cur, cudaStream_t s);
 // project-U force: start-of-step fractions in alpha4[pre], rest densities in alpha4[cur[ALPHA]]
-void launch_force_projectu(const DevParams& P, const DevBuffers& B, const int* cur, int pre, cudaStream_t s);
+// in_step: the drift pass of this step has just written the neighbour records, which are read instead of the fields
+void launch_force_projectu(const DevParams& P, const DevBuffers& B, const int* cur, int pre, bool in_step, bool fresh,
+                           cudaStream_t s);
 // alpha advance: reads alpha4[cur], writes alpha4[cur^1] (new fractions, same restdens)
-void launch_alpha_advance(const DevParams& P, const DevBuffers& B, const int* cur, cudaStream_t s);
+void launch_alpha_advance(const DevParams& P, const DevBuffers& B, const int* cur, bool in_step, bool fresh, cudaStream_t s);
 // correction: fractions in alpha4[cur[ALPHA]], start-of-step fractions in alpha4[pre]; in place
 void launch_correction(const DevParams& P, const DevBuffers& B, const int* cur, int pre, cudaStream_t s);
 // advance in place on the cur buffers

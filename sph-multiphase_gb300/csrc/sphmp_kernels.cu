@@ -1009,7 +1009,7 @@ __device__ __forceinline__ void force_drift_one(const DevParams& P, const DevBuf
         acc.pair(P, pj, dpj, vj, aj);
     });
     acc.finish(P, B, s, DRIFT ? aprev4[s] : make_float4(0.f, 0.f, 0.f, 0.f),
-               FORCE && DRIFT ? vev4[s] : make_float4(0.f, 0.f, 0.f, 0.f));
+               DRIFT ? vev4[s] : make_float4(0.f, 0.f, 0.f, 0.f));
 }
 
 // Force + drift of heavy particle s by the whole warp (every lane calls with
@@ -1033,13 +1033,13 @@ __device__ __forceinline__ void force_drift_warp(const DevParams& P, const DevBu
     acc.template reduce<32>();
     if (lane_id() == 0)
         acc.finish(P, B, s, DRIFT ? aprev4[s] : make_float4(0.f, 0.f, 0.f, 0.f),
-                   FORCE && DRIFT ? vev4[s] : make_float4(0.f, 0.f, 0.f, 0.f));
+                   DRIFT ? vev4[s] : make_float4(0.f, 0.f, 0.f, 0.f));
 }
 
 // Force + drift, L lanes per particle (walk_lanes); every warp first takes heavy
-// particles from the queue (whole warp per particle) while any are left. With
-// both, it also writes every in-grid particle's neighbour record for the fused
-// alpha pass.
+// particles from the queue (whole warp per particle) while any are left. With the
+// drift it also writes every in-grid particle's neighbour record for the alpha and
+// project-U passes of the step.
 // The work counter (hctr) of each pass over the queue of heavy particles.
 template <bool FORCE, bool DRIFT>
 constexpr int kHeavyCounter = FORCE && !DRIFT ? 1 : 0;
@@ -1067,7 +1067,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_force_drift(const __grid_consta
     const float4 pi = in ? pos4[s] : make_float4(0.f, 0.f, 0.f, -1.f);
     if (in && g == 0 && pi.w < 0.f) {
         if (FORCE) B.accel4[s] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (FORCE && DRIFT) {
+        if (DRIFT) {
             const float a0[3] = {0.f, 0.f, 0.f};
             const float u0[9] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
             write_nrec(B, s, pi, -1.f, make_float4(0.f, 0.f, 0.f, 0.f), a0, u0);
@@ -1094,7 +1094,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_force_drift(const __grid_consta
     acc.template reduce<L>();
     if (walk && g == 0)
         acc.finish(P, B, s, DRIFT ? aprev4[s] : make_float4(0.f, 0.f, 0.f, 0.f),
-                   FORCE && DRIFT ? vev4[s] : make_float4(0.f, 0.f, 0.f, 0.f));
+                   DRIFT ? vev4[s] : make_float4(0.f, 0.f, 0.f, 0.f));
 }
 
 // Force + drift of a corrected large step: the same pass, also filling the
@@ -1228,6 +1228,87 @@ __global__ void __launch_bounds__(kThreads) k_force_projectu(const __grid_consta
     B.velxcor[s] = make_float4(acc.xx, acc.xy, acc.xz, 0.f);
 }
 
+// The same force in a step, the neighbours' positions, velocities, start-of-step
+// fractions and drift velocities from the records that the drift pass of this step
+// wrote; L lanes a particle (walk_lanes), the heavy ones from the queue. Bound by its
+// loads as well (seven a neighbour, eight with the gathers): 14, 31, 82, 141 and 413 us
+// at 12 K, 63 K, 244 K, 421 K and 1.3 M slots against 39, 45, 92, 145 and 438.
+template <int NP, int L>
+__global__ void __launch_bounds__(kThreads, 3) k_force_projectu_rec(const __grid_constant__ DevParams P,
+                                                                    const __grid_constant__ DevBuffers B,
+                                                                    const float4* __restrict__ pos4,
+                                                                    const float4* __restrict__ vel4,
+                                                                    const float4* __restrict__ vev4,
+                                                                    const float4* __restrict__ alpha_cur,
+                                                                    const float4* __restrict__ alpha_pre,
+                                                                    const float4* __restrict__ aprev4) {
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    ProjectU<NP> acc;
+    auto init = [&](int i, const float4 pi) {
+        float3 um[NP];
+#pragma unroll
+        for (int k = 0; k < NP; k++) {
+            const float4 u = B.drift4[(size_t)k * P.cap + i];
+            um[k] = make_float3(u.x, u.y, u.z);
+        }
+        acc.init(pi, vev4[i], B.densp[i], vel4[i].w, alpha_cur[i].w, alpha_pre[i], um);
+    };
+    auto pair = [&](uint32_t j) {
+        const float4* __restrict__ r = B.nrec + (size_t)j * kNrecFloat4;
+        const float4 r0 = __ldg(r), r1 = __ldg(r + 1), r2 = __ldg(r + 2), r3 = __ldg(r + 3), r4 = __ldg(r + 4);
+        const float2 dpj = __ldg(&B.densp[j]);
+        const float viscj = __ldg(&vel4[j].w);
+        float4 uj[NP];
+        uj[0] = make_float4(r2.z, r2.w, r3.x, 0.f);
+        if (NP > 1) uj[NP > 1 ? 1 : 0] = make_float4(r3.y, r3.z, r3.w, 0.f);
+        if (NP > 2) uj[NP > 2 ? 2 : 0] = make_float4(r4.x, r4.y, r4.z, 0.f);
+        float mj = r4.w, rho0j = 1.f;
+        if (r4.w < 0.f) {  // boundary: raw mass (per origin) and rest density
+            mj = __ldg(&B.mass_raw[__float_as_uint(__ldg(&aprev4[j].w))]);
+            rho0j = __ldg(&alpha_cur[j].w);
+        }
+        acc.pair(P, make_float4(r0.x, r0.y, r0.z, r4.w), dpj, make_float4(r1.x, r1.y, r1.z, 0.f), viscj, rho0j, mj,
+                 make_float4(r1.w, r2.x, r2.y, 0.f), uj);
+    };
+    auto store = [&](int i) {
+        B.accel4[i] = make_float4(acc.fx, acc.fy, acc.fz, 0.f);
+        B.velxcor[i] = make_float4(acc.xx, acc.xy, acc.xz, 0.f);
+    };
+    if (P.list_mode != 0) {
+        const unsigned lane = lane_id();
+        const uint32_t nh = *B.hq_n;
+        uint32_t* ctr = &B.hctr[kHeavyCounter<true, false>];
+        for (uint32_t h = next_item(ctr, nh, lane); h < nh; h = next_item(ctr, nh, lane)) {
+            const int sh = (int)B.hq[h];
+            const float4 pi = pos4[sh];
+            init(sh, pi);
+            warp_for_slot_list(P, B, sh, pi.x, pi.y, pi.z, pair);
+            acc.template reduce<32>();
+            if (lane == 0) store(sh);
+        }
+    }
+    const int s = (int)((blockIdx.x * (unsigned)kThreads + threadIdx.x) / L);
+    const unsigned g = threadIdx.x % L;
+    const bool in = s < active_n(B);
+    const int si = in ? s : 0;
+    const float4 pi = pos4[si];
+    const bool grid = B.mgcell[si] != kUndef, fluid = grid && !(pi.w < 0.f);
+    if (in && g == 0 && !fluid) {
+        if (grid) B.accel4[s] = zero;
+        B.velxcor[s] = zero;
+    }
+    const bool walk = in && fluid && !is_heavy(P, B.nbr_cnt[si]);
+    if (!__any_sync(0xffffffffu, walk)) return;
+    init(si, pi);
+    if (walk) {
+        if (L == 1) for_slot_list(P, B, s, pi.x, pi.y, pi.z, pair);
+        else group_for_slot_list<L>(P, B, s, g, pi.x, pi.y, pi.z, pair);
+    }
+    __syncwarp();
+    if (L > 1) acc.template reduce<L>();
+    if (walk && g == 0) store(s);
+}
+
 // ---------------------------------------------------------------------------
 // Volume-fraction advance, correction, advection
 // ---------------------------------------------------------------------------
@@ -1274,6 +1355,99 @@ __global__ void __launch_bounds__(kThreads) k_alpha_advance(const __grid_constan
     float na[3] = {ai.x, ai.y, ai.z};
     alpha_change_slot<NP>(P, B, pos4, vev4, alpha_in, s, pi, vev4[s], ai, na);
     alpha_out[s] = make_float4(na[0], na[1], na[2], ai.w);
+}
+
+// The pair of a particle and its neighbour j in the alpha change, j's data from
+// the neighbour record that the drift (or force + drift) pass of this step wrote
+// (five 16-byte loads per neighbour instead of seven separate gathers).
+template <int NP>
+__device__ __forceinline__ void nrec_pair(const DevParams& P, const DevBuffers& B, uint32_t j, AlphaChange<NP>& acc) {
+    float4 q[5];
+    read_nrec<NP>(B, j, q);
+    const float4 r0 = q[0], r1 = q[1], r2 = q[2], r3 = q[3], r4 = q[4];
+    float4 uj[NP];
+    uj[0] = make_float4(r2.z, r2.w, r3.x, 0.f);
+    if (NP > 1) uj[NP > 1 ? 1 : 0] = make_float4(r3.y, r3.z, r3.w, 0.f);
+    if (NP > 2) uj[NP > 2 ? 2 : 0] = make_float4(r4.x, r4.y, r4.z, 0.f);
+    acc.pair(P, r0, r0.w, make_float4(r1.x, r1.y, r1.z, 0.f), make_float4(r1.w, r2.x, r2.y, 0.f), uj);
+}
+
+// Alpha change of in-grid particle s, by one thread.
+template <int NP>
+__device__ __forceinline__ void alpha_change_nrec(const DevParams& P, const DevBuffers& B, int s, const float4 pi,
+                                                  const float4 vei, const float4 ai, float (&out)[3]) {
+    AlphaChange<NP> acc;
+    acc.init(pi, vei, ai, B.drift4 + s, (size_t)P.cap);
+    for_slot_list(P, B, s, pi.x, pi.y, pi.z, [&](uint32_t j) { nrec_pair<NP>(P, B, j, acc); });
+    acc.result(P, out);
+}
+
+// Alpha change of heavy particle s by the whole warp (every lane calls with the
+// same s and gets the result).
+template <int NP>
+__device__ __forceinline__ void alpha_change_nrec_warp(const DevParams& P, const DevBuffers& B, int s, const float4 pi,
+                                                       const float4 vei, const float4 ai, float (&out)[3]) {
+    AlphaChange<NP> acc;
+    acc.init(pi, vei, ai, B.drift4 + s, (size_t)P.cap);
+    warp_for_slot_list(P, B, s, pi.x, pi.y, pi.z, [&](uint32_t j) { nrec_pair<NP>(P, B, j, acc); });
+    acc.template reduce<32>();
+    acc.result(P, out);
+}
+
+// Alpha change of in-grid particle s shared out over the L lanes of its group (g this
+// lane; every lane of the warp calls, `walk` where there is something to do).
+template <int NP, int L>
+__device__ __forceinline__ void alpha_change_nrec_group(const DevParams& P, const DevBuffers& B, int s, unsigned g,
+                                                        bool walk, const float4 pi, const float4 vei, const float4 ai,
+                                                        float (&out)[3]) {
+    AlphaChange<NP> acc;
+    acc.init(pi, vei, ai, B.drift4 + s, (size_t)P.cap);
+    if (walk) group_for_slot_list<L>(P, B, s, g, pi.x, pi.y, pi.z, [&](uint32_t j) { nrec_pair<NP>(P, B, j, acc); });
+    __syncwarp();
+    acc.template reduce<L>();
+    if (walk) acc.result(P, out);
+}
+
+// The same alpha advance in a step, where the drift pass has just written the neighbour
+// records: those instead of seven gathers a neighbour (that pass's load units were
+// 91 % busy with them), L lanes a particle (walk_lanes), the heavy ones from the
+// queue. Bound by the records' loads (L1). 12, 53, 94 and 264 us at 12 K, 244 K,
+// 421 K and 1.3 M slots against 27, 86, 129 and 356 with the gathers; the drift pass
+// pays up to 9 us for writing the records.
+template <int NP, int L>
+__global__ void __launch_bounds__(kThreads, 4) k_alpha_advance_rec(const __grid_constant__ DevParams P,
+                                                                   const __grid_constant__ DevBuffers B,
+                                                                   const float4* __restrict__ pos4,
+                                                                   const float4* __restrict__ vev4,
+                                                                   const float4* __restrict__ alpha_in,
+                                                                   float4* __restrict__ alpha_out) {
+    if (P.list_mode != 0) {
+        const unsigned lane = lane_id();
+        const uint32_t nh = *B.hq_n;
+        uint32_t* ctr = &B.hctr[kHeavyCounterAlpha];
+        for (uint32_t h = next_item(ctr, nh, lane); h < nh; h = next_item(ctr, nh, lane)) {
+            const int sh = (int)B.hq[h];
+            const float4 ai = alpha_in[sh];
+            float na[3] = {ai.x, ai.y, ai.z};
+            alpha_change_nrec_warp<NP>(P, B, sh, pos4[sh], vev4[sh], ai, na);
+            if (lane == 0) alpha_out[sh] = make_float4(na[0], na[1], na[2], ai.w);
+        }
+    }
+    const int s = (int)((blockIdx.x * (unsigned)kThreads + threadIdx.x) / L);
+    const unsigned g = threadIdx.x % L;
+    const bool in = s < active_n(B);
+    const int si = in ? s : 0;
+    const float4 pi = pos4[si], ai = alpha_in[si];
+    const bool sum = in && B.mgcell[si] != kUndef && !(pi.w < 0.f);
+    const bool heavy = sum && is_heavy(P, B.nbr_cnt[si]);  // taken from the queue
+    const bool walk = sum && !heavy;
+    float na[3] = {ai.x, ai.y, ai.z};
+    if (L == 1) {
+        if (walk) alpha_change_nrec<NP>(P, B, s, pi, vev4[s], ai, na);
+    } else if (__any_sync(0xffffffffu, walk)) {
+        alpha_change_nrec_group<NP, L>(P, B, si, g, walk, pi, vev4[si], ai, na);
+    }
+    if (in && g == 0 && !heavy) alpha_out[s] = make_float4(na[0], na[1], na[2], ai.w);
 }
 
 // Separate correction, in place: fractions in alpha_cur, start-of-step in alpha_pre.
@@ -1323,44 +1497,6 @@ __global__ void __launch_bounds__(kThreads) k_advance(const __grid_constant__ De
     aprev4[s] = ap;
 }
 
-// The pair of a particle and its neighbour j in the alpha change, j's data from
-// the neighbour record the force + drift pass of this step wrote (five 16-byte
-// loads per neighbour instead of seven separate gathers).
-template <int NP>
-__device__ __forceinline__ void nrec_pair(const DevParams& P, const DevBuffers& B, uint32_t j, AlphaChange<NP>& acc) {
-    float4 q[5];
-    read_nrec<NP>(B, j, q);
-    const float4 r0 = q[0], r1 = q[1], r2 = q[2], r3 = q[3], r4 = q[4];
-    float4 uj[NP];
-    uj[0] = make_float4(r2.z, r2.w, r3.x, 0.f);
-    if (NP > 1) uj[NP > 1 ? 1 : 0] = make_float4(r3.y, r3.z, r3.w, 0.f);
-    if (NP > 2) uj[NP > 2 ? 2 : 0] = make_float4(r4.x, r4.y, r4.z, 0.f);
-    acc.pair(P, r0, r0.w, make_float4(r1.x, r1.y, r1.z, 0.f), make_float4(r1.w, r2.x, r2.y, 0.f), uj);
-}
-
-// Alpha change of in-grid particle s, by one thread.
-template <int NP>
-__device__ __forceinline__ void alpha_change_nrec(const DevParams& P, const DevBuffers& B, int s, const float4 pi,
-                                                  const float4 vei, const float4 ai, float (&out)[3]) {
-    AlphaChange<NP> acc;
-    acc.init(pi, vei, ai, B.drift4 + s, (size_t)P.cap);
-    for_slot_list(P, B, s, pi.x, pi.y, pi.z, [&](uint32_t j) { nrec_pair<NP>(P, B, j, acc); });
-    acc.result(P, out);
-}
-
-// Alpha change of heavy particle s by the whole warp (every lane calls with the
-// same s and gets the result).
-template <int NP>
-__device__ __forceinline__ void alpha_change_nrec_warp(const DevParams& P, const DevBuffers& B, const F4Set& S, int s,
-                                                       float (&out)[3]) {
-    const float4 pi = S.in[POS][s], vei = S.in[VEV][s], ai = S.in[ALPHA][s];
-    AlphaChange<NP> acc;
-    acc.init(pi, vei, ai, B.drift4 + s, (size_t)P.cap);
-    warp_for_slot_list(P, B, s, pi.x, pi.y, pi.z, [&](uint32_t j) { nrec_pair<NP>(P, B, j, acc); });
-    acc.template reduce<32>();
-    acc.result(P, out);
-}
-
 // Alpha + correction + advance of one slot whose alpha sum (in-grid fluid
 // particles) is `anew`; writes the five float4 fields to the other buffer.
 template <int NP, bool MP>
@@ -1394,8 +1530,9 @@ __global__ void __launch_bounds__(kThreads, 4) k_pass_c(const __grid_constant__ 
         for (uint32_t h = next_item(ctr, nh, lane); h < nh; h = next_item(ctr, nh, lane)) {
             const int sh = (int)B.hq[h];
             float a[3];
-            alpha_change_nrec_warp<NP>(P, B, S, sh, a);
-            if (lane == 0) pass_c_finish<NP, MP>(P, B, S, sh, false, S.in[POS][sh], S.in[VEV][sh], S.in[ALPHA][sh], a);
+            const float4 p = S.in[POS][sh], ve = S.in[VEV][sh], al = S.in[ALPHA][sh];
+            alpha_change_nrec_warp<NP>(P, B, sh, p, ve, al, a);
+            if (lane == 0) pass_c_finish<NP, MP>(P, B, S, sh, false, p, ve, al, a);
         }
     }
     const int s = (int)((blockIdx.x * (unsigned)kThreads + threadIdx.x) / L);
@@ -1414,12 +1551,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_pass_c(const __grid_constant__ 
         if (heavy) return;
         if (walk) alpha_change_nrec<NP>(P, B, s, p, ve, al, anew);
     } else if (__any_sync(0xffffffffu, walk)) {
-        AlphaChange<NP> acc;
-        acc.init(p, ve, al, B.drift4 + si, (size_t)P.cap);
-        if (walk) group_for_slot_list<L>(P, B, s, g, p.x, p.y, p.z, [&](uint32_t j) { nrec_pair<NP>(P, B, j, acc); });
-        __syncwarp();
-        acc.template reduce<L>();
-        if (walk) acc.result(P, anew);
+        alpha_change_nrec_group<NP, L>(P, B, si, g, walk, p, ve, al, anew);
     }
     if (L == 1 || (in && g == 0 && !heavy)) pass_c_finish<NP, MP>(P, B, S, s, undef, p, ve, al, anew);
 }
@@ -1859,9 +1991,11 @@ void launch_density_oct(const DevParams& P, const DevBuffers& B, const int* cur,
 // one, two, four and eight lanes: 51, 33, 25, 21 at 22 K slots; 54, 38, 30, 38 at
 // 49 K; 60, 57, 59, 69 at 106 K; 127, 107, 123, 165 at 244 K; 199, 186, 222, 299
 // at 421 K; 322, 338, 420, 585 at 778 K; 518, 580, 720, 1012 at 1.3 M.
-static int walk_lanes(int n) {
-    constexpr int kResident = 152 * 4 * kThreads;
-    return n <= kResident / 6 ? 8 : n <= kResident / 2 ? 4 : n <= 3 * kResident ? 2 : 1;
+// (The project-U force keeps three blocks an SM: 43, 29, 29, 31 us at 63 K; 86, 84,
+// 88, 107 at 244 K; 141, 150, 166, 201 at 421 K.)
+static int walk_lanes(int n, int blocks = 4) {
+    const int resident = 152 * blocks * kThreads;
+    return n <= resident / 6 ? 8 : n <= resident / 2 ? 4 : n <= 3 * resident ? 2 : 1;
 }
 
 template <bool F, bool D, int NP>
@@ -1922,8 +2056,28 @@ void launch_surface_tension(const DevParams& P, const DevBuffers& B, const int* 
     k_surface_tension<<<blocks_for(P.n), kThreads, 0, s>>>(P, B, B.f4[POS][cur[POS]]);
 }
 
-void launch_force_projectu(const DevParams& P, const DevBuffers& B, const int* cur, int pre, cudaStream_t s) {
+template <int NP>
+static void projectu_lanes(const DevParams& P, const DevBuffers& B, const int* cur, int pre, cudaStream_t s) {
+    const float4 *pos = B.f4[POS][cur[POS]], *vel = B.f4[VEL][cur[VEL]], *vev = B.f4[VEV][cur[VEV]],
+                 *ac = B.f4[ALPHA][cur[ALPHA]], *ap = B.f4[ALPHA][pre], *apv = B.f4[APREV][cur[APREV]];
+    switch (walk_lanes(P.n, 3)) {
+        case 8: k_force_projectu_rec<NP, 8><<<walk_blocks(P.n, 8), kThreads, 0, s>>>(P, B, pos, vel, vev, ac, ap, apv); break;
+        case 4: k_force_projectu_rec<NP, 4><<<walk_blocks(P.n, 4), kThreads, 0, s>>>(P, B, pos, vel, vev, ac, ap, apv); break;
+        case 2: k_force_projectu_rec<NP, 2><<<walk_blocks(P.n, 2), kThreads, 0, s>>>(P, B, pos, vel, vev, ac, ap, apv); break;
+        default: k_force_projectu_rec<NP, 1><<<walk_blocks(P.n, 1), kThreads, 0, s>>>(P, B, pos, vel, vev, ac, ap, apv); break;
+    }
+}
+
+void launch_force_projectu(const DevParams& P, const DevBuffers& B, const int* cur, int pre, bool in_step, bool fresh,
+                           cudaStream_t s) {
     if (P.n <= 0) return;
+    if (in_step) {
+        if (!fresh) cudaMemsetAsync(&B.hctr[kHeavyCounter<true, false>], 0, sizeof(uint32_t), s);
+        if (P.nphase == 1) projectu_lanes<1>(P, B, cur, pre, s);
+        else if (P.nphase == 2) projectu_lanes<2>(P, B, cur, pre, s);
+        else projectu_lanes<3>(P, B, cur, pre, s);
+        return;
+    }
     const float4* pos = B.f4[POS][cur[POS]];
     const float4* vel = B.f4[VEL][cur[VEL]];
     const float4* vev = B.f4[VEV][cur[VEV]];
@@ -1938,12 +2092,31 @@ void launch_force_projectu(const DevParams& P, const DevBuffers& B, const int* c
     }
 }
 
-void launch_alpha_advance(const DevParams& P, const DevBuffers& B, const int* cur, cudaStream_t s) {
+template <int NP>
+static void alpha_lanes(const DevParams& P, const DevBuffers& B, const float4* pos, const float4* vev, const float4* ain,
+                        float4* aout, cudaStream_t s) {
+    switch (walk_lanes(P.n)) {
+        case 8: k_alpha_advance_rec<NP, 8><<<walk_blocks(P.n, 8), kThreads, 0, s>>>(P, B, pos, vev, ain, aout); break;
+        case 4: k_alpha_advance_rec<NP, 4><<<walk_blocks(P.n, 4), kThreads, 0, s>>>(P, B, pos, vev, ain, aout); break;
+        case 2: k_alpha_advance_rec<NP, 2><<<walk_blocks(P.n, 2), kThreads, 0, s>>>(P, B, pos, vev, ain, aout); break;
+        default: k_alpha_advance_rec<NP, 1><<<walk_blocks(P.n, 1), kThreads, 0, s>>>(P, B, pos, vev, ain, aout); break;
+    }
+}
+
+void launch_alpha_advance(const DevParams& P, const DevBuffers& B, const int* cur, bool in_step, bool fresh,
+                          cudaStream_t s) {
     if (P.n <= 0) return;
     const float4* pos = B.f4[POS][cur[POS]];
     const float4* vev = B.f4[VEV][cur[VEV]];
     const float4* ain = B.f4[ALPHA][cur[ALPHA]];
     float4* aout = B.f4[ALPHA][cur[ALPHA] ^ 1];
+    if (in_step) {
+        if (!fresh) cudaMemsetAsync(&B.hctr[kHeavyCounterAlpha], 0, sizeof(uint32_t), s);
+        if (P.nphase == 1) alpha_lanes<1>(P, B, pos, vev, ain, aout, s);
+        else if (P.nphase == 2) alpha_lanes<2>(P, B, pos, vev, ain, aout, s);
+        else alpha_lanes<3>(P, B, pos, vev, ain, aout, s);
+        return;
+    }
     const int g = blocks_for(P.n);
     switch (P.nphase) {
         case 1: k_alpha_advance<1><<<g, kThreads, 0, s>>>(P, B, pos, vev, ain, aout); break;
