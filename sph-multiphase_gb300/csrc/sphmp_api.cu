@@ -175,6 +175,8 @@ DevParams dev_params(const sphmp_ctx* c) {
     P.ss = p.simscale;
     P.h = p.smoothradius;
     P.r2 = p.smoothradius * p.smoothradius;
+    P.ih = 1.f / P.h;
+    P.ir2 = 1.f / P.r2;
     P.r2list = P.r2 * (1.0f + 1.0e-5f);
     P.list_mode = c->nbr_valid ? c->list_mode : 0;
     P.narrow = c->pos_sorted ? 1 : 0;

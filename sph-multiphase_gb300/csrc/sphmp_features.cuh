@@ -30,33 +30,30 @@ namespace dev {
 
 constexpr int kLearnedFeatures = 48;
 
+// Only what the neighbour walk needs stays in registers: the particle's own features
+// (0 .. 10) go to memory before it, and the sums take their scale in store().
 struct LearnedFeatures {
-    float f[kLearnedFeatures];
+    float f[kLearnedFeatures];  // 11 .. 47: the sums
     float4 pi, vi, ai;
-    float pres_i, reli, ivs, ips, ih, ih2, ir2;
+    float pres_i, reli;
 
-    // own features; pi, vi, ai, di, gi: this particle's pos4, vel4, alpha4,
-    // (1/rho, p), aprev4
-    __device__ __forceinline__ void init(const DevParams& P, float4 pi_, float4 vi_, float4 ai_, float2 di, float4 gi,
-                                         float vs, float dt_large) {
+    __device__ __forceinline__ static float pressure_scale(float4 ai, float vs) { return 1.f / (ai.w * vs * vs); }
+
+    // pi, vi, ai, di: this particle's pos4, vel4, alpha4, (1/rho, p); features 0 .. 7 into row
+    __device__ __forceinline__ void init(const DevParams& P, float4 pi_, float4 vi_, float4 ai_, float2 di, float vs,
+                                         float* row) {
         pi = pi_;
         vi = vi_;
         ai = ai_;
         pres_i = di.y;
         const float rhoi = 1.f / di.x;
         reli = rhoi / ai.w;
-        ivs = 1.f / vs;
-        ips = 1.f / (ai.w * vs * vs);
-        ih = 1.f / P.h;
-        ih2 = ih * ih;
-        ir2 = 1.f / P.r2;
+        const float ivs = 1.f / vs;
 #pragma unroll
-        for (int k = 0; k < kLearnedFeatures; k++) f[k] = 0.f;
-        f[0] = vi.x * ivs; f[1] = vi.y * ivs; f[2] = vi.z * ivs;
-        f[3] = reli - 1.f;
-        f[4] = di.y * ips;
-        f[5] = ai.x; f[6] = P.nphase > 1 ? ai.y : 0.f; f[7] = P.nphase > 2 ? ai.z : 0.f;
-        f[8] = gi.x * dt_large * ivs; f[9] = gi.y * dt_large * ivs; f[10] = gi.z * dt_large * ivs;
+        for (int k = 11; k < kLearnedFeatures; k++) f[k] = 0.f;
+        float4* out = reinterpret_cast<float4*>(row);
+        out[0] = make_float4(vi.x * ivs, vi.y * ivs, vi.z * ivs, reli - 1.f);
+        out[1] = make_float4(di.y * pressure_scale(ai, vs), ai.x, P.nphase > 1 ? ai.y : 0.f, P.nphase > 2 ? ai.z : 0.f);
     }
 
     // neighbour j: pos4, (1/rho, p), vel4, alpha4
@@ -66,44 +63,57 @@ struct LearnedFeatures {
         const float dsq = dx * dx + dy * dy + dz * dz;
         if (!(dsq < P.r2 && dsq > 0.f)) return;
         const float rinv = rsqrtf(dsq);
-        const float q2 = dsq * ir2, q = dsq * rinv * ih;
-        const float w = (1.f - q2) * (1.f - q2) * (1.f - q2);
-        const float g = (1.f - q) * (1.f - q);
-        const float ux = dx * rinv, uy = dy * rinv, uz = dz * rinv;
+        const float q1 = 1.f - dsq * P.ir2, q = 1.f - dsq * rinv * P.ih;
+        const float w = q1 * q1 * q1, g = q * q;
+        const float wx = w * dx, wy = w * dy, wz = w * dz;
         if (pj.w < 0.f) {  // boundary
             f[40] += w;
-            f[41] += w * dx * ih; f[42] += w * dy * ih; f[43] += w * dz * ih;
+            f[41] += wx; f[42] += wy; f[43] += wz;
             f[44] += 1.f / 32.f;
             return;
         }
         const float dvx = vj.x - vi.x, dvy = vj.y - vi.y, dvz = vj.z - vi.z;
         f[11] += w;
-        f[12] += w * dx * ih; f[13] += w * dy * ih; f[14] += w * dz * ih;
-        f[15] += w * dvx * ivs; f[16] += w * dvy * ivs; f[17] += w * dvz * ivs;
+        f[12] += wx; f[13] += wy; f[14] += wz;
+        f[15] += w * dvx; f[16] += w * dvy; f[17] += w * dvz;
         f[18] += w * (__fdividef(1.f, dj.x * aj.w) - reli);
-        f[19] += w * (dj.y - pres_i) * ips;
+        f[19] += w * (dj.y - pres_i);
         f[20] += w * (aj.x - ai.x);
         f[21] += w * (P.nphase > 1 ? aj.y - ai.y : 0.f);
         f[22] += w * (P.nphase > 2 ? aj.z - ai.z : 0.f);
-        const float wh2 = w * ih2;
-        f[23] += wh2 * dx * dx; f[24] += wh2 * dy * dy; f[25] += wh2 * dz * dz;
-        f[26] += wh2 * dx * dy; f[27] += wh2 * dx * dz; f[28] += wh2 * dy * dz;
-        f[29] += g * ux; f[30] += g * uy; f[31] += g * uz;
-        f[32] += g * (dvx * ux + dvy * uy + dvz * uz) * ivs;
-        f[33] += g * (dvy * uz - dvz * uy) * ivs;
-        f[34] += g * (dvz * ux - dvx * uz) * ivs;
-        f[35] += g * (dvx * uy - dvy * ux) * ivs;
-        const float pp = g * (pres_i + dj.y) * ips;
-        f[36] += pp * ux; f[37] += pp * uy; f[38] += pp * uz;
+        f[23] += wx * dx; f[24] += wy * dy; f[25] += wz * dz;
+        f[26] += wx * dy; f[27] += wx * dz; f[28] += wy * dz;
+        const float gr = g * rinv, gx = gr * dx, gy = gr * dy, gz = gr * dz;
+        f[29] += gx; f[30] += gy; f[31] += gz;
+        f[32] += dvx * gx + dvy * gy + dvz * gz;
+        f[33] += dvy * gz - dvz * gy;
+        f[34] += dvz * gx - dvx * gz;
+        f[35] += dvx * gy - dvy * gx;
+        const float pp = pres_i + dj.y;
+        f[36] += pp * gx; f[37] += pp * gy; f[38] += pp * gz;
         f[39] += 1.f / 32.f;
-        const float da = g * (aj.x - ai.x);
-        f[45] += da * ux; f[46] += da * uy; f[47] += da * uz;
+        const float da = aj.x - ai.x;
+        f[45] += da * gx; f[46] += da * gy; f[47] += da * gz;
     }
 
-    __device__ __forceinline__ void store(float* row) const {
+    // Features 8 .. 47 into row; gi: this particle's aprev4.
+    __device__ __forceinline__ void store(const DevParams& P, float4 gi, float vs, float dt_large, float* row) {
+        const float ivs = 1.f / vs, ih = P.ih, ih2 = ih * ih, ips = pressure_scale(ai, vs);
+        auto scale = [&](int from, int to, float k) {
+#pragma unroll
+            for (int i = from; i <= to; i++) f[i] *= k;
+        };
+        f[8] = gi.x * dt_large * ivs; f[9] = gi.y * dt_large * ivs; f[10] = gi.z * dt_large * ivs;
+        scale(12, 14, ih);
+        scale(15, 17, ivs);
+        scale(19, 19, ips);
+        scale(23, 28, ih2);
+        scale(32, 35, ivs);
+        scale(36, 38, ips);
+        scale(41, 43, ih);
         float4* out = reinterpret_cast<float4*>(row);
 #pragma unroll
-        for (int i = 0; i < kLearnedFeatures / 4; i++)
+        for (int i = 2; i < kLearnedFeatures / 4; i++)
             out[i] = make_float4(f[4 * i], f[4 * i + 1], f[4 * i + 2], f[4 * i + 3]);
     }
 };

@@ -77,6 +77,7 @@ struct DevParams {
     float srad[3];   // search radius h/simscale in cell units per axis, plus a rounding margin
     float ss;        // simscale
     float h, r2;     // smoothing radius and its square
+    float ih, ir2;   // their reciprocals
     float r2list;    // squared radius of the neighbour list (r2 plus a rounding margin)
     int list_mode;   // 0: no list, 1: index lists in nbr (written by the last density pass)
     int narrow;      // 1: positions are the ones the cell lists were built from (the cell

@@ -999,7 +999,7 @@ __device__ __forceinline__ void force_drift_one(const DevParams& P, const DevBuf
                                                 const float4* __restrict__ vev4, int s, const float4 pi) {
     ForceDrift<FORCE, DRIFT, NP> acc;
     acc.init(P, pi, vel4[s], B.densp[s], alpha4[s]);
-    for_slot_list(P, B, s, pi.x, pi.y, pi.z, [&](uint32_t j) {
+    for_slot_list<false>(P, B, s, pi.x, pi.y, pi.z, [&](uint32_t j) {
         // every load first (list entries are almost always neighbours), so that
         // consecutive neighbours' gathers overlap
         const float4 pj = __ldg(&pos4[j]);
@@ -1036,15 +1036,15 @@ __device__ __forceinline__ void force_drift_warp(const DevParams& P, const DevBu
                    DRIFT ? vev4[s] : make_float4(0.f, 0.f, 0.f, 0.f));
 }
 
-// Force + drift, L lanes per particle (walk_lanes); every warp first takes heavy
-// particles from the queue (whole warp per particle) while any are left. With the
-// drift it also writes every in-grid particle's neighbour record for the alpha and
-// project-U passes of the step.
 // The work counter (hctr) of each pass over the queue of heavy particles.
 template <bool FORCE, bool DRIFT>
 constexpr int kHeavyCounter = FORCE && !DRIFT ? 1 : 0;
 constexpr int kHeavyCounterAlpha = 2;
 
+// Force + drift, L lanes per particle (walk_lanes); every warp first takes heavy
+// particles from the queue (whole warp per particle) while any are left. With the
+// drift it also writes every in-grid particle's neighbour record for the alpha and
+// project-U passes of the step.
 template <bool FORCE, bool DRIFT, int NP, int L>
 __global__ void __launch_bounds__(kThreads, 4) k_force_drift(const __grid_constant__ DevParams P,
                                                              const __grid_constant__ DevBuffers B,
@@ -1099,9 +1099,14 @@ __global__ void __launch_bounds__(kThreads, 4) k_force_drift(const __grid_consta
 
 // Force + drift of a corrected large step: the same pass, also filling the
 // corrector's features from the neighbours it gathers (alpha4 is gathered
-// even without drift). Features and ids cover every particle; 128 registers.
+// even without drift). Features and ids cover every particle. Bound by the latency of
+// its gathers with 16 warps an SM: 52 sums and the neighbours in flight take 126
+// registers (96 spill: 320 us). What the walk does not need stays out of them:
+// the own features are stored before it, the sums scaled after it. 895 K slots, two
+// phases: 264 us (306 with the own features and scales held and applied to every pair).
+constexpr int kFeatThreads = 128;
 template <bool DRIFT, int NP>
-__global__ void __launch_bounds__(kThreads, 2) k_force_drift_feat(const __grid_constant__ DevParams P,
+__global__ void __launch_bounds__(kFeatThreads, 4) k_force_drift_feat(const __grid_constant__ DevParams P,
                                                                   const __grid_constant__ DevBuffers B,
                                                                   const float4* __restrict__ pos4,
                                                                   const float4* __restrict__ vel4,
@@ -1109,7 +1114,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_force_drift_feat(const __grid_c
                                                                   const float4* __restrict__ aprev4,
                                                                   const float4* __restrict__ vev4, float* feat,
                                                                   int32_t* ids, float vs, float dt_large) {
-    const int s = blockIdx.x * kThreads + threadIdx.x;
+    const int s = blockIdx.x * kFeatThreads + threadIdx.x;
     if (s >= active_n(B)) return;
     float* row = feat + (size_t)s * kLearnedFeatures;
     if (B.mgcell[s] == kUndef) {
@@ -1127,12 +1132,12 @@ __global__ void __launch_bounds__(kThreads, 2) k_force_drift_feat(const __grid_c
         store_no_features(row, &ids[s]);
         return;
     }
-    const float4 vi = vel4[s], ai = alpha4[s], gi = aprev4[s];
+    const float4 vi = vel4[s], ai = alpha4[s];
     const float2 di = B.densp[s];
     ForceDrift<true, DRIFT, NP> acc;
     acc.init(P, pi, vi, di, ai);
     LearnedFeatures lf;
-    lf.init(P, pi, vi, ai, di, gi, vs, dt_large);
+    lf.init(P, pi, vi, ai, di, vs, row);
     for_slot_list(P, B, s, pi.x, pi.y, pi.z, [&](uint32_t j) {
         const float4 pj = __ldg(&pos4[j]);
         const float2 dpj = __ldg(&B.densp[j]);
@@ -1141,8 +1146,9 @@ __global__ void __launch_bounds__(kThreads, 2) k_force_drift_feat(const __grid_c
         acc.pair(P, pj, dpj, vj, aj);
         lf.pair(P, pj, dpj, vj, aj);
     });
+    const float4 gi = aprev4[s];
+    lf.store(P, gi, vs, dt_large, row);
     acc.finish(P, B, s, DRIFT ? gi : make_float4(0.f, 0.f, 0.f, 0.f), DRIFT ? vev4[s] : make_float4(0.f, 0.f, 0.f, 0.f));
-    lf.store(row);
     ids[s] = B.bornid[__float_as_uint(gi.w)];
 }
 
@@ -2039,15 +2045,15 @@ void launch_force_drift_features(const DevParams& P, const DevBuffers& B, const 
     const float4* al = B.f4[ALPHA][cur[ALPHA]];
     const float4* ap = B.f4[APREV][cur[APREV]];
     const float4* ve = B.f4[VEV][cur[VEV]];
-    const int g = blocks_for(P.n);
+    const int g = blocks_for(P.n, kFeatThreads);
     if (!P.multiphase) {
-        k_force_drift_feat<false, 0><<<g, kThreads, 0, s>>>(P, B, pos, vel, al, ap, ve, feat, ids, vs, dt_large);
+        k_force_drift_feat<false, 0><<<g, kFeatThreads, 0, s>>>(P, B, pos, vel, al, ap, ve, feat, ids, vs, dt_large);
         return;
     }
     switch (P.nphase) {
-        case 1: k_force_drift_feat<true, 1><<<g, kThreads, 0, s>>>(P, B, pos, vel, al, ap, ve, feat, ids, vs, dt_large); break;
-        case 2: k_force_drift_feat<true, 2><<<g, kThreads, 0, s>>>(P, B, pos, vel, al, ap, ve, feat, ids, vs, dt_large); break;
-        default: k_force_drift_feat<true, 3><<<g, kThreads, 0, s>>>(P, B, pos, vel, al, ap, ve, feat, ids, vs, dt_large); break;
+        case 1: k_force_drift_feat<true, 1><<<g, kFeatThreads, 0, s>>>(P, B, pos, vel, al, ap, ve, feat, ids, vs, dt_large); break;
+        case 2: k_force_drift_feat<true, 2><<<g, kFeatThreads, 0, s>>>(P, B, pos, vel, al, ap, ve, feat, ids, vs, dt_large); break;
+        default: k_force_drift_feat<true, 3><<<g, kFeatThreads, 0, s>>>(P, B, pos, vel, al, ap, ve, feat, ids, vs, dt_large); break;
     }
 }
 
