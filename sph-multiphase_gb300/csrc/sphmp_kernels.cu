@@ -67,16 +67,33 @@ __global__ void __launch_bounds__(kHashBlock) k_hash(const __grid_constant__ Dev
         base = __shfl_sync(peers, base, leader);
         B.arank[i] = base + __popc(peers & lanemask_lt());
     }
-    // The Morton order scans the cells in another sequence (k_scan_reduce). Slots are
-    // nearly in cell order, so a block mostly counts into one sum, with one atomic
-    // (one per warp took 20 us at 1.3 M slots: they all go to the same few words).
+    // The Morton order scans the cells in another sequence (k_scan_reduce). All go to the
+    // same few words, so a block adds up what it counts into one sum and adds that with
+    // one atomic, for up to four sums, one after the other (slots are nearly in cell
+    // order after a sort: one or two sums); the rest by warps. (One atomic a warp: 40
+    // instead of 20 us at 1.3 M sorted slots; one sum a block and the rest one by one:
+    // 127 us instead of 14.5 for 913 K slots as uploaded.)
     if (!P.morton) {
-        __shared__ uint32_t first;
-        if (threadIdx.x == 0) first = in ? key / kScanPer : 0u;
-        __syncthreads();
-        const int same = __syncthreads_count((int)(in && key / kScanPer == first));
-        if (threadIdx.x == 0 && same) atomicAdd(&B.bsum[first], (uint32_t)same);
-        if (in && key / kScanPer != first) atomicAdd(&B.bsum[key / kScanPer], 1u);
+        __shared__ volatile uint32_t shared_sum;
+        const uint32_t sum = key / kScanPer;
+        bool open = in;
+        int left = __syncthreads_count((int)open);
+        for (int round = 0; round < 4 && left > 0; round++) {
+            if (open) shared_sum = sum;  // any of the open ones
+            __syncthreads();
+            const uint32_t f = shared_sum;
+            const int same = __syncthreads_count((int)(open && sum == f));
+            if (threadIdx.x == 0) atomicAdd(&B.bsum[f], (uint32_t)same);
+            open = open && sum != f;
+            left -= same;
+        }
+        if (left > 0) {
+            const unsigned om = __ballot_sync(0xffffffffu, open);
+            if (open) {
+                const unsigned peers = __match_any_sync(om, sum);
+                if ((int)lane == __ffs(peers) - 1) atomicAdd(&B.bsum[sum], (uint32_t)__popc(peers));
+            }
+        }
     }
     const bool und = valid && key == kUndef;
     const unsigned ub = __ballot_sync(0xffffffffu, und);
@@ -186,19 +203,20 @@ __global__ void __launch_bounds__(kScanBlock) k_scan_reduce(const __grid_constan
 // the list of cells too large for the warp sort, in one pass: every block adds up
 // the sums of the blocks before it (a few dozen words) and scans its kScanPer
 // counts together with their occupied flags (counts in the low 40 bits, flags
-// above). `clear`: the counts are zeroed for the next hash. (Three kernels, one
-// of them a single block over the block sums and the chunks' out-of-grid counts,
-// took 13 us at 11 K particles and 21 us at 1.3 M.)
+// above). `clear`: the counts are zeroed for the next hash. Bound by its chain: counts,
+// two block scans, the stores, which take 16 bytes a thread and array (7 to 9 us at 11 K
+// to 1.3 M particles; 10 to 13 with 4-byte stores and the counts read behind the first
+// scan; three kernels, one of them a single block over the block sums and the chunks'
+// out-of-grid counts, took 13 to 21).
 __global__ void __launch_bounds__(kScanBlock) k_scan(const __grid_constant__ DevParams P,
                                                      const __grid_constant__ DevBuffers B, int clear) {
     __shared__ uint32_t act_base;
-    uint32_t before = 0;
-    for (unsigned k = threadIdx.x; k < blockIdx.x; k += kScanBlock) before += B.bsum[k];
-    uint32_t run;
-    block_excl_scan(before, &run);
     const int idx = (blockIdx.x * kScanBlock + threadIdx.x) * kScanItems;
     uint32_t v[4];
-    load4_cells(P, B, idx, v);
+    load4_cells(P, B, idx, v);  // beside the sums before, which the first block does not need
+    uint32_t before = 0, run = 0;
+    for (unsigned k = threadIdx.x; k < blockIdx.x; k += kScanBlock) before += B.bsum[k];
+    if (blockIdx.x > 0) block_excl_scan(before, &run);
     uint64_t sum = 0;
 #pragma unroll
     for (int k = 0; k < 4; k++) sum += (uint64_t)v[k] + (v[k] ? 1ull << 40 : 0ull);
@@ -212,15 +230,26 @@ __global__ void __launch_bounds__(kScanBlock) k_scan(const __grid_constant__ Dev
         B.cstart[P.G + 1] = (uint32_t)active_n(B);
     }
     run += (uint32_t)excl;
+    const bool four = !P.morton && idx + 3 < P.G;  // this thread's cells as 16-byte words
+    if (four) {
+        const uint32_t e0 = run + v[0], e1 = e0 + v[1], e2 = e1 + v[2], e3 = e2 + v[3];
+        reinterpret_cast<uint4*>(B.cstart + idx)[0] = make_uint4(run, e0, e1, e2);
+        reinterpret_cast<uint4*>(B.cend + idx)[0] = make_uint4(e0, e1, e2, e3);
+        reinterpret_cast<uint4*>(B.mgridoff + idx)[0] = make_uint4(v[0] ? run : 0u, v[1] ? e0 : 0u, v[2] ? e1 : 0u, v[3] ? e2 : 0u);
+        reinterpret_cast<uint4*>(B.mgridcnt + idx)[0] = make_uint4(v[0], v[1], v[2], v[3]);
+        if (clear) reinterpret_cast<uint4*>(B.ccount + idx)[0] = make_uint4(0u, 0u, 0u, 0u);
+    }
 #pragma unroll
     for (int k = 0; k < 4; k++) {
         if (idx + k < P.G) {
             const int c = P.morton ? (int)B.corder[idx + k] : idx + k;
-            B.cstart[c] = run;
-            B.cend[c] = run + v[k];
-            B.mgridoff[c] = v[k] ? (int32_t)run : 0;
-            B.mgridcnt[c] = (int32_t)v[k];
-            if (clear) B.ccount[c] = 0u;
+            if (!four) {
+                B.cstart[c] = run;
+                B.cend[c] = run + v[k];
+                B.mgridoff[c] = v[k] ? (int32_t)run : 0;
+                B.mgridcnt[c] = (int32_t)v[k];
+                if (clear) B.ccount[c] = 0u;
+            }
             if (v[k]) B.act[at++] = (uint32_t)c;
             if (v[k] > (uint32_t)kWarpSortMax) {
                 if (v[k] > (uint32_t)kCtaSortMax) {
@@ -310,14 +339,14 @@ __device__ __forceinline__ void warp_bitonic(uint32_t (&v)[E]) {
 
 // Write the internal order of cell c from the key (octant << shift | member index)
 // held at sorted position q (cellstart + q is its internal index): the member's
-// previous internal index (osrc), its slot (oidx) and the bucket starts.
+// previous internal index src (osrc), its slot (oidx) and the bucket starts.
 __device__ __forceinline__ void emit_octant(const DevBuffers& B, uint32_t c, uint32_t start, uint32_t cnt, uint32_t q,
-                                            uint32_t key, uint32_t prev_oct, int shift, uint32_t pre_slot,
+                                            uint32_t key, uint32_t prev_oct, int shift, uint32_t src,
                                             uint32_t* bst = nullptr) {
     const uint32_t oct = key >> shift;
     const uint32_t idx = key & ((1u << shift) - 1u);
     if (q < cnt) {
-        B.osrc[start + q] = B.opos[pre_slot];
+        B.osrc[start + q] = src;
         B.oidx[start + q] = start + idx;
     }
     // bucket starts: every bucket in (prev_oct, oct] begins at q (8 marks past the end)
@@ -360,13 +389,13 @@ __device__ __forceinline__ void warp_sort_cell(const DevParams& P, const DevBuff
 #pragma unroll
     for (int r = 0; r < E; r++) {
         const uint32_t idx = lane * E + r;
-        wsm[idx] = v[r];
         key[r] = 0xFFFFFFFFu;
         if (idx < cnt) {
+            key[r] = ((uint32_t)B.octk[v[r]] << 8) | idx;
+            wsm[idx] = B.opos[v[r]];  // beside the octants, not behind their sort
             B.midsort[start + idx] = v[r];
             B.mgcell[start + idx] = c;
             B.mgndx[start + idx] = idx;
-            key[r] = ((uint32_t)B.octk[v[r]] << 8) | idx;
         }
     }
     // octant order: sort (octant, member index)
@@ -380,8 +409,8 @@ __device__ __forceinline__ void warp_sort_cell(const DevParams& P, const DevBuff
         const uint32_t prev_oct = (q == 0) ? 0xFFFFFFFFu : (pk == 0xFFFFFFFFu ? 8u : pk >> 8);
         if (q <= cnt) {
             const uint32_t k = key[r];
-            const uint32_t pre = q < cnt ? wsm[k & 255u] : 0u;
-            emit_octant(B, c, start, cnt, q, q < cnt ? k : (8u << 8), prev_oct, 8, pre, bst);
+            const uint32_t src = q < cnt ? wsm[k & 255u] : 0u;
+            emit_octant(B, c, start, cnt, q, q < cnt ? k : (8u << 8), prev_oct, 8, src, bst);
         }
     }
     __syncwarp();  // the bucket starts in bst are visible to the whole warp
@@ -463,8 +492,8 @@ __global__ void __launch_bounds__(1024) k_big_cell_sort(const __grid_constant__ 
             const uint32_t k = q < cnt ? sm[q] : (8u << 13);
             const uint32_t pk = q == 0 ? 0xFFFFFFFFu : sm[q - 1];
             const uint32_t prev_oct = q == 0 ? 0xFFFFFFFFu : (pk >> 13);
-            const uint32_t pre = q < cnt ? B.midsort[start + (k & 0x1FFFu)] : 0u;
-            emit_octant(B, c, start, cnt, q, k, prev_oct, 13, pre);
+            const uint32_t src = q < cnt ? B.opos[B.midsort[start + (k & 0x1FFFu)]] : 0u;
+            emit_octant(B, c, start, cnt, q, k, prev_oct, 13, src);
         }
         __syncthreads();
         if (threadIdx.x < 8) {
@@ -607,7 +636,8 @@ __global__ void __launch_bounds__(kThreads) k_boundary_volume_store(const __grid
 // cost the force and alpha passes 27 us of cache misses.) A lane adds at most 16
 // pairs of terms before they go to its Kahan-compensated sum, and the lanes of a
 // member are added pairwise (a scan). Warps take work items from a shared counter (their
-// costs differ by orders of magnitude): the first window of every bucket, then
+// costs differ by orders of magnitude), each its first one without it (14 instead of
+// 12.5 us at 11 K particles when every warp began and ended at the counter): the first window of every bucket, then
 // the further windows of large buckets, which the cell sort queued in wq, so that
 // no bucket serialises on one warp. Members whose lists overflow their kMaxNbr
 // entries get mask lists instead (overflow_masks) or, where the sequence is too
@@ -735,7 +765,9 @@ __global__ void __launch_bounds__(kDensThreads, 7) k_density_bucket(const __grid
     const size_t cap = (size_t)P.cap;
     const float r2 = P.r2, r2list = P.r2list;
     const float kFar = __int_as_float(0x7f800000);  // +inf: never within range
-    for (uint32_t it = next_bucket(B.dctr, lane); it < nitems; it = next_bucket(B.dctr, lane)) {
+    const uint32_t nwarps = gridDim.x * (kDensThreads / 32);
+    for (uint32_t it = (blockIdx.x * kDensThreads + threadIdx.x) >> 5; it < nitems;
+         it = nitems > nwarps ? nwarps + next_bucket(B.dctr, lane) : nitems) {
         uint32_t c, q, w0;
         if (it < nb) {
             c = __ldg(&B.act[it >> 3]);

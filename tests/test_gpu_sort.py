@@ -75,6 +75,30 @@ def test_sort_equals_a_stable_sort(n, out, order):
             assert np.array_equal(again[k], got[k]), k
 
 
+@pytest.mark.parametrize("runs", [1, 3, 7, 256])
+def test_blocks_that_count_into_many_sums(runs):
+    """A block of 256 slots whose particles fall into about `runs` of the grid's ten groups of 4,096 cells: added up
+    group by group for four of them, by warps for the rest."""
+    n, side = 64000, 40
+    sc = scenes.small_block(seed=5, n=(side, side, side), d=0.01, h=0.006, nphase=1, dens=(1000.0,), walls=False)
+    p, d, c = sc.params, sc.disp[:n].copy(), sc.calc[:n].copy()
+    assert p.gridtotal > 8 * 4096
+    rng = np.random.default_rng(runs)
+    piece = max(1, 256 // runs)  # stretches of the sorted order, shuffled
+    y = np.argsort(d["pos"][:, 1], kind="stable")
+    d["pos"] = d["pos"][np.concatenate([y[k * piece:(k + 1) * piece] for k in rng.permutation(-(-n // piece))])]
+    with sphmp.Context(p) as ctx:
+        ctx.upload_aos(d, c)
+        ctx.get_particle_index()
+        key = ctx.download_field(abi.F_MGCELL).astype(np.int64)
+        ctx.get_grid_list()
+        got = _lists(ctx)
+    assert (key != abi.GRID_UNDEF).all()
+    assert np.array_equal(got["midsort"], np.argsort(key, kind="stable").astype(np.uint32))
+    assert np.array_equal(got["mgridcnt"], np.bincount(key, minlength=p.gridtotal).astype(np.int32))
+    assert np.array_equal(got["mgcell"], np.sort(key).astype(np.uint32))
+
+
 @pytest.mark.parametrize("order", [abi.CELL_ORDER_LINEAR, abi.CELL_ORDER_MORTON])
 @pytest.mark.parametrize("graph", [False, True])
 def test_list_after_a_step(graph, order):
