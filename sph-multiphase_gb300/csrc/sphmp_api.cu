@@ -469,7 +469,7 @@ sphmp_status enqueue_step(sphmp_ctx* c, int schedule, StageTimer* T = nullptr, c
         c->hash_n = c->emit_on ? -1 : c->n;  // with an emitter the count is only known on the device
         launch_cell_starts(P, c->B, true, true, s);
         mark("cell_starts");
-        launch_cell_order(P, c->B, c->cur, s);
+        launch_cell_order(P, c->B, s);
         mark("cell_order");
         launch_rearrange(P, c->B, c->cur, false, true, s);
         mark("rearrange");
@@ -1005,7 +1005,7 @@ sphmp_status sphmp_get_grid_list(sphmp_ctx* c) {
     if (c->counts_clear) launch_recount(dev_params(c), c->B, c->stream);  // a step's sort has cleared them
     c->counts_clear = false;
     launch_cell_starts(dev_params(c), c->B, true, false, c->stream);
-    launch_cell_order(dev_params(c), c->B, c->cur, c->stream);
+    launch_cell_order(dev_params(c), c->B, c->stream);
     CHECK_LAUNCH("GetGridList");
     c->oct_built = true;
     return SPHMP_OK;

@@ -225,7 +225,7 @@ void launch_recount(const DevParams& P, const DevBuffers& B, cudaStream_t s);
 // per-cell stable ordering and the per-cell octant order (which reads the
 // pre-sort positions pos4[cur[POS]] to build the next internal order)
 void launch_cell_starts(const DevParams& P, const DevBuffers& B, bool hashed, bool clear, cudaStream_t s);
-void launch_cell_order(const DevParams& P, const DevBuffers& B, const int* cur, cudaStream_t s);
+void launch_cell_order(const DevParams& P, const DevBuffers& B, cudaStream_t s);
 // move every particle to its new internal index (osrc) and update opos; with
 // `slot_order`, the new internal order is the reference's sorted slot order
 // (for a rearrange that did not follow this library's grid list); with `clear`

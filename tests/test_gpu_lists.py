@@ -75,6 +75,13 @@ def test_sequence_lengths(around):
     _step_matches(_cluster(6, around, 200 + around))
 
 
+@pytest.mark.parametrize("members,around", [(4, 4), (5, 4), (8, 8), (9, 8), (16, 16), (17, 16), (32, 32), (33, 32)])
+def test_cell_sort_sizes(members, around):
+    """A cell of members + 7 around particles: 32, 33, 64, 65, 128, 129, 256 and 257, where a lane of the cell sort
+    holds one, two, four or eight of them, or a block sorts the cell."""
+    _step_matches(_cluster(members, around, 500 + members))
+
+
 @pytest.mark.parametrize("window", [8, 16, 32])
 def test_window_parameter(window):
     _step_matches(_cluster(40, 12, 300), window)
