@@ -10,9 +10,9 @@
 // sort) are scanned once a step, by warps that share their candidates among 8
 // particles, for the density (cubic spline of support 2h); the scan also writes
 // every particle's fluid neighbours within h and boundary neighbours within 2h as
-// index lists, which every other sum walks, several lanes per particle. The kernels, cut-offs and formulas are the
-// reference's (the advection viscosity within 2h, every other gradient sum
-// within h). As in the reference, `dens` (densp.x) holds the density itself
+// index lists, which every other sum walks, several lanes per particle. The
+// kernels, cut-offs and formulas are the reference's (the advection viscosity
+// within 2h, every other gradient sum within h). As in the reference, `dens` (densp.x) holds the density itself
 // after the IISPH density pass, not its inverse. The per-particle IISPH arrays
 // (d_ii, a_ii, predicted density, the pressure iterate and the terms its
 // neighbours gather) live in DevBuffers.

@@ -146,8 +146,8 @@ struct DevBuffers {
     double* red;        // [16] FP64 reduction results
     float* vtmp;        // [cap + 64] scratch (boundary volumes; block sums of the IISPH residue)
     uint32_t* nbr;      // [kMaxNbr * cap] neighbour indices, groups of 4 column-major: entry k of s at ((k / 4) * cap + s) * 4 + k % 4
-    uint32_t* nbr_cnt;  // [cap] list of particle s: kMaskList | bucket, index count (<= kMaxNbr) or kRescan
-    uint32_t* nmask;    // [kMaskWords * cap] bucket mask lists, column-major: word k of particle s at k * cap + s
+    uint32_t* nbr_cnt;  // [cap] list of particle s: index count (<= kMaxNbr), with kHeavyFlag if heavy; overflowed: kMaskList | bucket or kRescan
+    uint32_t* nmask;    // [kMaskWords * cap] bucket mask lists (of overflowed index lists), column-major: word k of particle s at k * cap + s
     uint32_t* btab;     // [8 * G * kTabStride] candidate ranges of each bucket with a mask list
     uint32_t* dctr;     // [1] work counter of the bucket density kernel
     uint2* wq;          // [cap / kBucketWindowMin + 16] member windows after the first of large buckets:

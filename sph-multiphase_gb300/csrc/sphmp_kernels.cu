@@ -632,11 +632,11 @@ __global__ void __launch_bounds__(kThreads) k_boundary_volume_store(const __grid
 // that interleave measured 338 us, but put the lists out of sequence order, which
 // cost the force and alpha passes 27 us of cache misses.) A lane adds at most 16
 // pairs of terms before they go to its Kahan-compensated sum, and the lanes of a
-// member are added pairwise (a scan). Warps take work items from a shared counter (their
-// costs differ by orders of magnitude), each its first one without it (14 instead of
-// 12.5 us at 11 K particles when every warp began and ended at the counter): the first window of every bucket, then
-// the further windows of large buckets, which the cell sort queued in wq, so that
-// no bucket serialises on one warp. Members whose lists overflow their kMaxNbr
+// member are added pairwise (a scan). Warps take work items from a shared counter
+// (their costs differ by orders of magnitude), each its first one without it (12.5
+// instead of 14.3 us at 11 K particles): the first window of every bucket, then the
+// further windows of large buckets, which the cell sort queued in wq, so that no
+// bucket serialises on one warp. Members whose lists overflow their kMaxNbr
 // entries get mask lists instead (overflow_masks) or, where the sequence is too
 // long for those, are left to the cell search; they and members with more than
 // P.heavy neighbours are queued in hq for the force and alpha passes.
