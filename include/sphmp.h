@@ -178,7 +178,7 @@ typedef struct sphmp_params {
     float mf_omega;              /* simData.omega: boundary pressure factor of the project-U force */
     float mf_visc_factor;        /* simData.visc_factor: boundary viscosity factor of the project-U force */
     int32_t cell_order;          /* sphmp_cell_order: order of the cells in the sorted arrays */
-    int32_t bucket_window;       /* members of one h-subcell per work item of the density pass, 8..32 (0: 32) */
+    int32_t bucket_window;       /* members of one h-subcell per work item of the density pass, 8..32 (0: 16) */
     int32_t heavy_list;          /* neighbour lists longer than this are walked by a whole warp, 32..256 (0: 128) */
 } sphmp_params;
 

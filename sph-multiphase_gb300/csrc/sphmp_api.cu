@@ -206,7 +206,7 @@ DevParams dev_params(const sphmp_ctx* c) {
     P.st_C = p.surfaceTensionFluidC;
     for (int k = 0; k < 27; k++) P.neighborid[k] = p.neighborid[k];
     P.morton = p.cell_order == SPHMP_CELL_ORDER_MORTON;
-    P.bwin = p.bucket_window > 0 ? p.bucket_window : (int)kBucketWindow;
+    P.bwin = p.bucket_window > 0 ? p.bucket_window : (int)kBucketWindowDefault;
     P.heavy = p.heavy_list > 0 ? (uint32_t)p.heavy_list : kHeavyList;
     const double h = (double)P.h;
     P.ii_c1 = 2.25 / h;
@@ -1180,7 +1180,7 @@ sphmp_status sphmp_autotune(sphmp_ctx* c, int32_t trial_steps, int32_t allow_reo
         for (int w : {16, 32})
             for (int h : {64, 128, 256}) cands.push_back({orders[o], w, h});
     // the context's own configuration first: its time is ms_before
-    const Cand cur = {c->prm.cell_order, c->prm.bucket_window ? c->prm.bucket_window : (int)kBucketWindow,
+    const Cand cur = {c->prm.cell_order, c->prm.bucket_window ? c->prm.bucket_window : (int)kBucketWindowDefault,
                       c->prm.heavy_list ? c->prm.heavy_list : (int)kHeavyList};
     cands.insert(cands.begin(), cur);
     float best = 0.f;

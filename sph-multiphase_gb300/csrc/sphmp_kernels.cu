@@ -616,7 +616,7 @@ __global__ void __launch_bounds__(kThreads) k_boundary_volume_store(const __grid
 // gradients vanish to below 1e-7 of a typical term). The 27 subcells form 18
 // contiguous index ranges (per (y, z) row: the x-neighbour bucket in the adjacent
 // cell and the two buckets of the same cell); their concatenation is the bucket's
-// candidate sequence. A warp takes one window of up to P.bwin (<= 32) members of a
+// candidate sequence. A warp takes one window of up to P.bwin (16, at most 32) members of a
 // bucket and stages the bucket's candidates in shared memory, 256 at a time. The
 // window's n fluid members share the lanes out: 32 / n lanes a member, each
 // testing its share of the sequence two candidates at a time in packed FP32

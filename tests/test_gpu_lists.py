@@ -70,6 +70,12 @@ def test_window_sizes(members):
     _step_matches(_cluster(members, 4, 80 + members))
 
 
+@pytest.mark.parametrize("members", [17, 25, 31, 32])
+def test_one_lane_a_member(members):
+    """Windows of more than 16 members (not the default)."""
+    _step_matches(_cluster(members, 4, 700 + members), 32)
+
+
 @pytest.mark.parametrize("around", [0, 1, 9, 10, 19, 20, 40])
 def test_sequence_lengths(around):
     _step_matches(_cluster(6, around, 200 + around))
