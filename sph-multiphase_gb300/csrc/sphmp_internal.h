@@ -59,7 +59,7 @@ constexpr uint32_t kBucketWindowDefault = 16;
 constexpr uint32_t kMaskList = 0x80000000u;  // nbr_cnt flag: bucket mask list, low bits = bucket (cell * 8 + octant)
 constexpr uint32_t kRescan = 0x7fffffffu;    // nbr_cnt value: no list, search the cells
 // Heavy particles (long lists, overflowed lists, cell searches) are queued in hq by
-// the list expansion and taken by whole warps in the force and alpha passes; an
+// the density pass and taken by whole warps in the force and alpha passes; an
 // index list of a heavy particle carries this flag over its length.
 constexpr uint32_t kHeavyFlag = 0x40000000u;
 constexpr uint32_t kHeavyList = 128;         // default: index lists longer than this are heavy
