@@ -234,7 +234,7 @@ void free_buffers(sphmp_ctx* c) {
         for (int b = 0; b < 2; b++) cudaFree(B.f4[f][b]);
     void* ptrs[] = {B.densp, B.accel4, B.drift4, B.velxcor, B.pmod, B.mgcell, B.midsort, B.mgndx, B.mgridoff, B.mgridcnt,
                     B.key, B.octk, B.arank, B.sidx, B.ccount, B.cstart, B.cend, B.corder, B.uchunk, B.big, B.ctl, B.color, B.bornid,
-                    B.mass_raw, B.err, B.red, B.vtmp, B.nbr, B.nbr_cnt, B.nmask, B.btab, B.wq, B.hq, B.iis_dii, B.iis_dijpj, B.iis_aii, B.iis_rho_adv, B.iis_pl, B.iis_dsum, B.iis_pm, B.iis_ctl, B.iis_list, B.nrec, B.opos, B.oidx, B.osrc, B.oct_start,
+                    B.mass_raw, B.err, B.red, B.vtmp, B.nbr, B.nbr_cnt, B.nmask, B.btab, B.wq, B.hq, B.iis_dii, B.nrec, B.opos, B.oidx, B.osrc, B.oct_start,
                     B.act, B.nact, B.frame, c->stage};
     for (void* q : ptrs) cudaFree(q);
     memset(&c->B, 0, sizeof(c->B));
@@ -297,15 +297,16 @@ sphmp_status alloc_buffers(sphmp_ctx* c) {
     B.dctr = B.ctl + 3;
     B.big_n = B.ctl + 4;
     B.hctr = B.ctl + 5;
-    CK(dalloc(&B.iis_dii, N));
-    CK(dalloc(&B.iis_dijpj, N));
-    CK(dalloc(&B.iis_aii, N));
-    CK(dalloc(&B.iis_rho_adv, N));
-    CK(dalloc(&B.iis_pl, N));
-    CK(dalloc(&B.iis_dsum, N));
-    CK(dalloc(&B.iis_pm, N));
-    CK(dalloc(&B.iis_ctl, 4));
-    CK(dalloc(&B.iis_list, N));
+    // the IISPH arrays in one allocation (creating a context is mostly its allocations)
+    CK(dalloc(&B.iis_dii, 3 * N + (5 * N + 4 + 3) / 4));
+    B.iis_dijpj = B.iis_dii + N;
+    B.iis_dsum = B.iis_dii + 2 * N;
+    B.iis_aii = reinterpret_cast<float*>(B.iis_dii + 3 * N);
+    B.iis_rho_adv = B.iis_aii + N;
+    B.iis_pl = B.iis_aii + 2 * N;
+    B.iis_pm = B.iis_aii + 3 * N;
+    B.iis_list = reinterpret_cast<uint32_t*>(B.iis_aii + 4 * N);
+    B.iis_ctl = B.iis_list + N;
     CK(cudaMemset(B.iis_dii, 0, sizeof(float4) * N));
     CK(cudaMemset(B.iis_dijpj, 0, sizeof(float4) * N));
     CK(cudaMemset(B.iis_pl, 0, sizeof(float) * N));

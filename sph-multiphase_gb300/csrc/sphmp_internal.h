@@ -162,7 +162,7 @@ struct DevBuffers {
     uint32_t* hq;       // [cap] heavy particles (internal index), filled by the density pass
     uint32_t* hq_n;     // [1] entries in hq
     uint32_t* hctr;     // [3] work counters over hq of the drift (or force + drift), force (or project-U) and alpha passes
-    // IISPH step (sphmp_iisph.cu): d_ii, sum_j d_ij p_j, d_ii p_l + sum_j d_ij p_j (float4,
+    // IISPH step (sphmp_iisph.cu; one allocation, at iis_dii): d_ii, sum_j d_ij p_j, d_ii p_l + sum_j d_ij p_j (float4,
     // w unused), a_ii, the predicted density, the pressure iterate p_l, p_l m / rho^2
     float4* iis_dii;
     float4* iis_dijpj;
