@@ -324,7 +324,9 @@ __device__ __forceinline__ float2 density_result(const DevParams& P, float wsum,
 //   {u_0z, u_1xyz}, {u_2xyz, w}
 // with md = mass * (1/rho) for fluid particles and -1 for boundary particles
 // (which exchange no volume fraction), u_k the drift velocities, w that of pos4
-// (the mass, or minus the volume of a boundary particle). (A 96-byte
+// (the mass, or minus the volume of a boundary particle). A boundary particle's
+// record holds its veleval too (walls may move), with zero fractions and drift
+// velocities, which no pass reads of it. (A 96-byte
 // record read with three 32-byte loads measured slower: 0.314 against
 // 0.295 ms per alpha pass, from the larger records missing L2.)
 __device__ __forceinline__ void write_nrec(const DevBuffers& B, int s, const float4 p, float md, const float4 ve,
@@ -443,9 +445,8 @@ struct ForceDrift {
     }
 
     // mfComputeDriftVel's closing terms (multiphase.cu:131-163) and the stores.
-    // `vev` (the particle's veleval) is only read when FORCE and DRIFT run
-    // together: that pass also writes the particle's neighbour record for the
-    // alpha pass (write_nrec).
+    // `vev` (the particle's veleval) is only read with DRIFT: that pass also writes
+    // the particle's neighbour record for the alpha and project-U passes (write_nrec).
     __device__ __forceinline__ void finish(const DevParams& P, const DevBuffers& B, int s, const float4 ap,
                                            const float4 vev = make_float4(0.f, 0.f, 0.f, 0.f)) {
         if (FORCE) B.accel4[s] = make_float4(fx, fy, fz, 0.f);

@@ -1099,7 +1099,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_force_drift(const __grid_consta
         if (DRIFT) {
             const float a0[3] = {0.f, 0.f, 0.f};
             const float u0[9] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-            write_nrec(B, s, pi, -1.f, make_float4(0.f, 0.f, 0.f, 0.f), a0, u0);
+            write_nrec(B, s, pi, -1.f, vev4[s], a0, u0);
         }
     }
     const bool walk = !(pi.w < 0.f) && !is_heavy(P, B.nbr_cnt[s]);  // heavy: taken from the queue
@@ -1156,7 +1156,7 @@ __global__ void __launch_bounds__(kFeatThreads, 4) k_force_drift_feat(const __gr
         if (DRIFT) {
             const float a0[3] = {0.f, 0.f, 0.f};
             const float u0[9] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-            write_nrec(B, s, pi, -1.f, make_float4(0.f, 0.f, 0.f, 0.f), a0, u0);
+            write_nrec(B, s, pi, -1.f, vev4[s], a0, u0);
         }
         store_no_features(row, &ids[s]);
         return;
