@@ -465,7 +465,7 @@ sphmp_status enqueue_step(sphmp_ctx* c, int schedule, StageTimer* T = nullptr, c
             mark("emit");
         }
         if (!c->counts_clear) launch_clear_counts(c->B, s);
-        launch_hash(P, c->B, c->cur, s);
+        launch_hash(P, c->B, c->cur, true, s);
         mark("hash");
         c->hash_n = c->emit_on ? -1 : c->n;  // with an emitter the count is only known on the device
         launch_cell_starts(P, c->B, true, true, s);
@@ -958,7 +958,7 @@ sphmp_status sphmp_upload_field(sphmp_ctx* c, int32_t field, const void* host, i
             const int saved = P.n;
             P.n = 0;  // scan only: no scatter / cell sort
             c->counts_clear = false;
-            launch_hash(P, c->B, c->cur, c->stream);  // nothing to hash: clears the control words
+            launch_hash(P, c->B, c->cur, false, c->stream);  // nothing to hash: clears the control words
             launch_cell_starts(P, c->B, false, false, c->stream);
             P.n = saved;
             // cstart[G+1] must still be n
@@ -983,7 +983,7 @@ sphmp_status sphmp_get_particle_index(sphmp_ctx* c) {
     if (sphmp_status st = refresh_n(c)) return st;
     if (!c->counts_clear) launch_clear_counts(c->B, c->stream);
     c->counts_clear = false;
-    launch_hash(dev_params(c), c->B, c->cur, c->stream);
+    launch_hash(dev_params(c), c->B, c->cur, false, c->stream);
     CHECK_LAUNCH("GetParticleIndex");
     c->hash_n = c->n;
     c->listed = false;
@@ -1005,7 +1005,7 @@ sphmp_status sphmp_get_grid_list(sphmp_ctx* c) {
     c->listed = true;
     if (c->counts_clear) launch_recount(dev_params(c), c->B, c->stream);  // a step's sort has cleared them
     c->counts_clear = false;
-    launch_cell_starts(dev_params(c), c->B, true, false, c->stream);
+    launch_cell_starts(dev_params(c), c->B, false, false, c->stream);
     launch_cell_order(dev_params(c), c->B, c->stream);
     CHECK_LAUNCH("GetGridList");
     c->oct_built = true;

@@ -222,15 +222,15 @@ sphmp_status record_error(sphmp_status st, const char* msg);
 // All take the current double-buffer selectors in `cur` (one per Field4).
 // zero the counts the hash adds to (DevBuffers::ccount)
 void launch_clear_counts(const DevBuffers& B, cudaStream_t s);
-// cell keys, ranks and counts (the counts zero before), control words cleared
-void launch_hash(const DevParams& P, const DevBuffers& B, const int* cur, cudaStream_t s);
+// cell keys, ranks and counts (the counts zero before), control words cleared; with
+// `sums` also the sums of the counts in the linear order
+void launch_hash(const DevParams& P, const DevBuffers& B, const int* cur, bool sums, cudaStream_t s);
 // the counts again from the last hash's keys, after they were cleared
 void launch_recount(const DevParams& P, const DevBuffers& B, cudaStream_t s);
-// GetGridList in two halves: cell starts (a scan of the counts, which the hash
-// left with `hashed`; with `clear` the counts are zeroed), then the scatter, the
-// per-cell stable ordering and the per-cell octant order (which reads the
-// pre-sort positions pos4[cur[POS]] to build the next internal order)
-void launch_cell_starts(const DevParams& P, const DevBuffers& B, bool hashed, bool clear, cudaStream_t s);
+// GetGridList in two halves: cell starts (a scan of the counts, whose sums the hash
+// of the same step left with `sums`; with `clear` the counts are zeroed), then the
+// scatter, the per-cell stable ordering and the per-cell octant order
+void launch_cell_starts(const DevParams& P, const DevBuffers& B, bool sums, bool clear, cudaStream_t s);
 void launch_cell_order(const DevParams& P, const DevBuffers& B, cudaStream_t s);
 // move every particle to its new internal index (osrc) and update opos; with
 // `slot_order`, the new internal order is the reference's sorted slot order

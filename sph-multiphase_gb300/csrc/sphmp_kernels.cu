@@ -36,14 +36,15 @@ using namespace dev;
 
 // One block = one chunk of kHashBlock slots. In-grid slots take a rank inside
 // their cell from a warp-aggregated atomic (the order is fixed later by the
-// cell sort) and are counted per kScanPer cells as well, so that the scan of the
-// cell counts needs no pass of its own for its blocks' sums; out-of-grid slots
+// cell sort) and, with `sums` (the linear order only), are counted per kScanPer
+// cells as well, so that the scan that follows at once in a step needs no pass of
+// its own for its blocks' sums; out-of-grid slots
 // get their exact rank inside the chunk, and the chunk totals, also summed per
 // kHashBlock chunks, place them in slot order. The first block clears the
 // control words of the sort and the passes after it.
 __global__ void __launch_bounds__(kHashBlock) k_hash(const __grid_constant__ DevParams P,
                                                      const __grid_constant__ DevBuffers B,
-                                                     const float4* __restrict__ pos4) {
+                                                     const float4* __restrict__ pos4, int sums) {
     __shared__ uint32_t wcount[kHashBlock / 32];
     const int i = blockIdx.x * kHashBlock + threadIdx.x;
     if (i < kCtlWords) B.ctl[i] = 0u;
@@ -67,13 +68,12 @@ __global__ void __launch_bounds__(kHashBlock) k_hash(const __grid_constant__ Dev
         base = __shfl_sync(peers, base, leader);
         B.arank[i] = base + __popc(peers & lanemask_lt());
     }
-    // The Morton order scans the cells in another sequence (k_scan_reduce). All go to the
-    // same few words, so a block adds up what it counts into one sum and adds that with
+    // All go to the same few words, so a block adds up what it counts into one sum and adds that with
     // one atomic, for up to four sums, one after the other (slots are nearly in cell
     // order after a sort: one or two sums); the rest by warps. (One atomic a warp: 40
     // instead of 20 us at 1.3 M sorted slots; one sum a block and the rest one by one:
     // 127 us instead of 14.5 for 913 K slots as uploaded.)
-    if (!P.morton) {
+    if (sums) {
         __shared__ volatile uint32_t shared_sum;
         const uint32_t sum = key / kScanPer;
         bool open = in;
@@ -130,7 +130,6 @@ __global__ void __launch_bounds__(kHashBlock) k_recount(const __grid_constant__ 
     if (threadIdx.x == 0 && B.uchunk[blockIdx.x]) atomicAdd(&B.usum[blockIdx.x / kHashBlock], B.uchunk[blockIdx.x]);
     if (i >= active_n(B) || B.key[i] == kUndef) return;
     atomicAdd(&B.ccount[B.key[i]], 1u);
-    if (!P.morton) atomicAdd(&B.bsum[B.key[i] / kScanPer], 1u);
 }
 
 // ---------------------------------------------------------------------------
@@ -187,8 +186,9 @@ __device__ __forceinline__ void load4_cells(const DevParams& P, const DevBuffers
     for (int k = 0; k < 4; k++) v[k] = idx + k < P.G ? B.ccount[B.corder[idx + k]] : 0u;
 }
 
-// Block sums of the cell counts in scan order, where the hash has not left them
-// (the Morton order; counts uploaded by the caller).
+// Block sums of the cell counts in scan order, where the hash of the same step has not
+// left them: the Morton order, and a cell list made by its own call, whose counts may
+// be the caller's and whose order may have been changed since the hash.
 __global__ void __launch_bounds__(kScanBlock) k_scan_reduce(const __grid_constant__ DevParams P,
                                                             const __grid_constant__ DevBuffers B) {
     const int idx = (blockIdx.x * kScanBlock + threadIdx.x) * kScanItems;
@@ -1955,21 +1955,21 @@ F4Set make_set(const DevBuffers& B, const int* cur, bool to_alt) {
 
 void launch_clear_counts(const DevBuffers& B, cudaStream_t s) { cudaMemsetAsync(B.ccount, 0, B.count_bytes, s); }
 
-void launch_hash(const DevParams& P, const DevBuffers& B, const int* cur, cudaStream_t s) {
+void launch_hash(const DevParams& P, const DevBuffers& B, const int* cur, bool sums, cudaStream_t s) {
     if (P.n <= 0) {
         cudaMemsetAsync(B.ctl, 0, sizeof(uint32_t) * kCtlWords, s);
         return;
     }
-    k_hash<<<blocks_for(P.n, kHashBlock), kHashBlock, 0, s>>>(P, B, B.f4[POS][cur[POS]]);
+    k_hash<<<blocks_for(P.n, kHashBlock), kHashBlock, 0, s>>>(P, B, B.f4[POS][cur[POS]], sums && !P.morton ? 1 : 0);
 }
 
 void launch_recount(const DevParams& P, const DevBuffers& B, cudaStream_t s) {
     if (P.n > 0) k_recount<<<blocks_for(P.n, kHashBlock), kHashBlock, 0, s>>>(P, B);
 }
 
-void launch_cell_starts(const DevParams& P, const DevBuffers& B, bool hashed, bool clear, cudaStream_t s) {
+void launch_cell_starts(const DevParams& P, const DevBuffers& B, bool sums, bool clear, cudaStream_t s) {
     const int nb = (P.G + (int)kScanPer - 1) / (int)kScanPer;
-    if (P.morton || !hashed) k_scan_reduce<<<nb, kScanBlock, 0, s>>>(P, B);
+    if (P.morton || !sums) k_scan_reduce<<<nb, kScanBlock, 0, s>>>(P, B);
     k_scan<<<nb, kScanBlock, 0, s>>>(P, B, clear ? 1 : 0);
 }
 
