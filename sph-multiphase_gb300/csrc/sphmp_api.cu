@@ -36,7 +36,6 @@ struct sphmp_ctx {
     bool oct_valid = false;       // the internal order is octant-grouped for the current cell list
     bool pos_sorted = false;      // positions unchanged since the cell list was built from them
     int hash_n = -1;              // particle count the cell keys were computed for (-1: none)
-    bool listed = false;          // GetGridList has run since the last hash
     bool counts_clear = true;     // the hash's counts (B.ccount ...) are zero: a step's sort leaves them so
     int list_mode = 0;            // kind of list the last density pass wrote (DevParams::list_mode)
     int device = 0;
@@ -293,10 +292,10 @@ sphmp_status alloc_buffers(sphmp_ctx* c) {
     CK(cudaMemset(B.ctl, 0, sizeof(uint32_t) * kCtlWords));
     B.act_n = B.ctl;
     B.wq_n = B.ctl + 1;
-    B.hq_n = B.ctl + 2;
-    B.dctr = B.ctl + 3;
-    B.big_n = B.ctl + 4;
-    B.hctr = B.ctl + 5;
+    B.big_n = B.ctl + 2;
+    B.hq_n = B.ctl + kListWords;
+    B.dctr = B.ctl + kListWords + 1;
+    B.hctr = B.ctl + kListWords + 2;
     // the IISPH arrays in one allocation (creating a context is mostly its allocations)
     CK(dalloc(&B.iis_dii, 3 * N + (5 * N + 4 + 3) / 4));
     B.iis_dijpj = B.iis_dii + N;
@@ -474,7 +473,7 @@ sphmp_status enqueue_step(sphmp_ctx* c, int schedule, StageTimer* T = nullptr, c
         mark("cell_order");
         launch_rearrange(P, c->B, c->cur, false, true, s);
         mark("rearrange");
-        c->counts_clear = c->listed = true;
+        c->counts_clear = true;
         swap_all(c);
         c->alpha_advanced = false;
         c->grid_valid = true;
@@ -954,16 +953,8 @@ sphmp_status sphmp_upload_field(sphmp_ctx* c, int32_t field, const void* host, i
             // rebuild the cell starts (and mgridoff) from the uploaded counts
             CK(cudaMemcpyAsync(c->B.ccount, c->B.mgridcnt, sizeof(uint32_t) * (size_t)c->prm.gridtotal,
                                cudaMemcpyDeviceToDevice, c->stream));
-            DevParams P = dev_params(c);
-            const int saved = P.n;
-            P.n = 0;  // scan only: no scatter / cell sort
             c->counts_clear = false;
-            launch_hash(P, c->B, c->cur, false, c->stream);  // nothing to hash: clears the control words
-            launch_cell_starts(P, c->B, false, false, c->stream);
-            P.n = saved;
-            // cstart[G+1] must still be n
-            const uint32_t nn = (uint32_t)c->n;
-            CK(cudaMemcpyAsync(c->B.cstart + c->prm.gridtotal + 1, &nn, sizeof(uint32_t), cudaMemcpyHostToDevice, c->stream));
+            launch_cell_starts(dev_params(c), c->B, false, false, c->stream);  // scan only: no scatter / cell sort
             CHECK_LAUNCH("rebuild cell starts");
             c->grid_valid = true;
         }
@@ -986,7 +977,6 @@ sphmp_status sphmp_get_particle_index(sphmp_ctx* c) {
     launch_hash(dev_params(c), c->B, c->cur, false, c->stream);
     CHECK_LAUNCH("GetParticleIndex");
     c->hash_n = c->n;
-    c->listed = false;
     c->grid_valid = false;
     c->nbr_valid = c->ii_valid = false;
     c->oct_valid = false;
@@ -1000,9 +990,6 @@ sphmp_status sphmp_get_grid_list(sphmp_ctx* c) {
     // the scatter places every slot by its cell key and rank: both must exist for the current count
     if (c->hash_n != c->n)
         return fail(SPHMP_ERR_STATE, "no cell keys for the current %d particles (run GetParticleIndex first)", c->n);
-    // called again without a new hash, the words that the first call counted with are cleared here
-    if (c->listed) CK(cudaMemsetAsync(c->B.ctl, 0, sizeof(uint32_t) * kCtlWords, c->stream));
-    c->listed = true;
     if (c->counts_clear) launch_recount(dev_params(c), c->B, c->stream);  // a step's sort has cleared them
     c->counts_clear = false;
     launch_cell_starts(dev_params(c), c->B, false, false, c->stream);
@@ -1399,7 +1386,7 @@ sphmp_status sphmp_step(sphmp_ctx* c, int32_t nsteps, int32_t schedule, int32_t 
             memcpy(c->graph_cur, c->cur, sizeof(c->graph_cur));
         }
         if (!c->counts_clear) launch_clear_counts(c->B, c->stream);
-        c->counts_clear = c->listed = true;
+        c->counts_clear = true;
         for (int t = 0; t + per <= nsteps; t += per) CK(cudaGraphLaunch(c->graph, c->stream));
         if (c->emit_on) c->n_stale = true;
         // the state a step leaves behind (as enqueue_step sets it)
@@ -1607,7 +1594,6 @@ static sphmp_status clone_state(sphmp_ctx* dst, sphmp_ctx* src) {
     dst->oct_built = src->oct_built;
     dst->pos_sorted = src->pos_sorted;
     dst->hash_n = src->hash_n;
-    dst->listed = src->listed;
     dst->counts_clear = src->counts_clear;
     dst->list_mode = src->list_mode;
     dst->nbr_valid = dst->ii_valid = false;

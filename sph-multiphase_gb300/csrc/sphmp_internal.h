@@ -39,6 +39,7 @@ constexpr int kScanBlock = 1024;      // threads per scan block
 constexpr int kScanItems = 4;         // items per thread in the scan
 constexpr uint32_t kScanPer = kScanBlock * kScanItems;  // cells per scan block
 constexpr int kCtlWords = 16;         // control words of the sort and the passes (DevBuffers::ctl)
+constexpr int kListWords = 3;         // the first of them: those a cell list counts with (act_n, wq_n, big_n)
 constexpr int kWarpSortMax = 256;     // cells up to this size are sorted by one warp
 constexpr int kCtaSortMax = 8192;     // larger cells up to this size are sorted by one CTA
 constexpr int kNumFloat4Fields = 5;   // pos4, vel4, vev4, alpha4, aprev4
@@ -141,8 +142,9 @@ struct DevBuffers {
     uint32_t* corder;   // [G] cells in Z-order (the scan order of the Morton mode)
     uint32_t* uchunk;   // [cap / kHashBlock + 2] out-of-grid count per hash chunk
     uint32_t* big;      // [cap / (kWarpSortMax+1) + 2] cells above the warp sort's size
-    // Control words, one allocation of kCtlWords cleared by the hash: the pointers to
-    // single words below (act_n, wq_n, hq_n, dctr, hctr, big_n) point into it
+    // Control words, one allocation of kCtlWords cleared by the hash (the first kListWords
+    // also by a cell list of its own call): the pointers to single words below (act_n,
+    // wq_n, big_n, hq_n, dctr, hctr) point into it
     uint32_t* ctl;
     uint32_t* big_n;    // [1] entries in big
     float4* color;      // [cap] per origin

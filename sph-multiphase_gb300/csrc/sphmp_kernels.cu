@@ -188,10 +188,13 @@ __device__ __forceinline__ void load4_cells(const DevParams& P, const DevBuffers
 
 // Block sums of the cell counts in scan order, where the hash of the same step has not
 // left them: the Morton order, and a cell list made by its own call, whose counts may
-// be the caller's and whose order may have been changed since the hash.
+// be the caller's and whose order may have been changed since the hash. Such a list may
+// be made twice from one hash, so the words that it counts with start from zero here
+// (the queue of heavy particles is not among them: lists of neighbours may hold it).
 __global__ void __launch_bounds__(kScanBlock) k_scan_reduce(const __grid_constant__ DevParams P,
                                                             const __grid_constant__ DevBuffers B) {
     const int idx = (blockIdx.x * kScanBlock + threadIdx.x) * kScanItems;
+    if (idx < kListWords * kScanItems) B.ctl[idx / kScanItems] = 0u;
     uint32_t v[4];
     load4_cells(P, B, idx, v);
     uint32_t total;

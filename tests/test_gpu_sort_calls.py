@@ -4,7 +4,8 @@ import numpy as np
 import pytest
 
 import sphmp
-from sphmp import abi
+from helpers import bits_equal, device_ctx
+from sphmp import abi, scenes
 from test_gpu_sort import _lists, _morton, _scene
 
 pytestmark = pytest.mark.gpu
@@ -67,3 +68,65 @@ def test_cell_order_changes_between_the_calls(first, steps):
                 ctx.set_params(q)
         ctx.rearrange_data()
         assert np.array_equal(np.sort(ctx.download_field(abi.F_BORNID)), np.arange(p.num))
+
+
+def _dense(per):
+    """`per` particles in each h-subcell of four cells along every axis, in a grid with no room to spare."""
+    h, sub = 0.02, 8
+    sc = scenes.small_block(seed=per, n=(16, 16, 16), d=h / 2, h=h, nphase=2, walls=False, eos=abi.EOS_LINEAR,
+                            box=(sub * h, sub * h, sub * h), dens=(1000.0, 900.0), velocity_scale=0.1)
+    p, n = sc.params, per * sub ** 3
+    rng = np.random.default_rng(per)
+    d, c = sphmp.record_arrays(n)
+    src = rng.integers(0, len(sc.disp), n)
+    d[:], c[:] = sc.disp[src], sc.calc[src]
+    cell = np.repeat(np.stack(np.meshgrid(*[np.arange(sub)] * 3, indexing="ij"), -1).reshape(-1, 3), per, axis=0)
+    at = np.array(p.gridmin[:3]) + 2 * h / p.simscale  # the first inner cell
+    d["pos"] = (at + (cell + rng.uniform(0.02, 0.98, (n, 3))) * h / p.simscale)[rng.permutation(n)]
+    c["mass"] *= np.float32(8.0 / per)
+    p.num = p.maxNum = n
+    return scenes.Scene(p, d, c, n, 0)
+
+
+def _state(ctx):
+    return {f: ctx.download_field(f) for f in (abi.F_MIDSORT, abi.F_POS, abi.F_DENS, abi.F_PRESSURE, abi.F_ACCEL)}
+
+
+@pytest.mark.parametrize("twice", ["counts", "list"])
+def test_cells_listed_twice_from_one_hash(twice):
+    """The cells scanned for uploaded counts (the same ones) or listed, and listed again: occupied cells, large cells
+    and member windows are counted once. A cell holds 320 particles, a particle has about 170 neighbours."""
+    sc = _dense(40)
+    got = []
+    for again in (False, True):
+        with device_ctx(sc) as ctx:
+            ctx.before_first_step()
+            ctx.get_particle_index()
+            if again and twice == "counts":
+                ctx.upload_field(abi.F_MGRIDCNT, ctx.download_field(abi.F_MGRIDCNT))
+            elif again:
+                ctx.get_grid_list()
+            ctx.get_grid_list()
+            ctx.rearrange_data()
+            ctx.compute_pressure()
+            ctx.compute_force()
+            got.append(_state(ctx))
+    for f, v in got[0].items():
+        assert bits_equal(got[1][f], v), f
+
+
+def test_list_between_density_and_force():
+    """The queue of particles with many neighbours outlives a cell list made between the passes."""
+    sc = _dense(40)
+    got = []
+    for again in (False, True):
+        with device_ctx(sc) as ctx:
+            ctx.before_first_step()
+            ctx.sort()
+            ctx.compute_pressure()
+            if again:
+                ctx.get_grid_list()
+            ctx.compute_force()
+            got.append(_state(ctx))
+    assert bits_equal(got[1][abi.F_ACCEL], got[0][abi.F_ACCEL])
+    assert np.abs(got[0][abi.F_ACCEL]).max() > 0
