@@ -36,7 +36,6 @@ struct sphmp_ctx {
     bool oct_valid = false;       // the internal order is octant-grouped for the current cell list
     bool pos_sorted = false;      // positions unchanged since the cell list was built from them
     int hash_n = -1;              // particle count the cell keys were computed for (-1: none)
-    bool counts_clear = true;     // the hash's counts (B.ccount ...) are zero: a step's sort leaves them so
     int list_mode = 0;            // kind of list the last density pass wrote (DevParams::list_mode)
     int device = 0;
     cudaStream_t own_stream = nullptr;
@@ -267,10 +266,11 @@ sphmp_status alloc_buffers(sphmp_ctx* c) {
     CK(dalloc(&B.sidx, N));
     const size_t nb = G / kScanPer + 2, nu = N / ((size_t)kHashBlock * kHashBlock) + 2;
     const size_t nc = (G + 4) / 4 * 4;  // the sums behind the counts start on 16 bytes
-    B.count_bytes = sizeof(uint32_t) * (nc + nb + nu);
-    CK(dalloc(&B.ccount, nc + nb + nu));
+    B.count_bytes = sizeof(uint32_t) * (nc + nb + nu + 1);
+    CK(dalloc(&B.ccount, nc + nb + nu + 1));
     B.bsum = B.ccount + nc;
     B.usum = B.bsum + nb;
+    B.counted = B.usum + nu;
     CK(dalloc(&B.cstart, G + 2));
     CK(dalloc(&B.cend, G));
     CK(dalloc(&B.corder, G));
@@ -446,9 +446,13 @@ struct LargeStep {
 
 // Queue one full step on the context stream (no host synchronisation). With
 // `L` (fused schedule only), the features are taken after the density pass and
-// the network's correction is applied to the step's result.
+// the network's correction is applied to the step's result. A step of the library's
+// own captured graph (`in_graph`) finds the counts of the sort clear, as sphmp_step and
+// the step before leave them, and clears what it has read; any other clears them
+// itself: what is queued must not depend on what has run before it, since a
+// caller may capture the calls on its own stream and replay them later.
 sphmp_status enqueue_step(sphmp_ctx* c, int schedule, StageTimer* T = nullptr, const LargeStep* L = nullptr,
-                          bool reuse_sorted = false) {
+                          bool reuse_sorted = false, bool in_graph = false) {
     const DevParams P = dev_params(c);
     const cudaStream_t s = c->stream;
     auto mark = [&](const char* nm) {
@@ -463,17 +467,16 @@ sphmp_status enqueue_step(sphmp_ctx* c, int schedule, StageTimer* T = nullptr, c
             c->n_stale = true;
             mark("emit");
         }
-        if (!c->counts_clear) launch_clear_counts(c->B, s);
+        if (!in_graph) launch_clear_counts(c->B, s);
         launch_hash(P, c->B, c->cur, true, s);
         mark("hash");
         c->hash_n = c->emit_on ? -1 : c->n;  // with an emitter the count is only known on the device
-        launch_cell_starts(P, c->B, true, true, s);
+        launch_cell_starts(P, c->B, true, in_graph, s);
         mark("cell_starts");
         launch_cell_order(P, c->B, s);
         mark("cell_order");
-        launch_rearrange(P, c->B, c->cur, false, true, s);
+        launch_rearrange(P, c->B, c->cur, false, in_graph, s);
         mark("rearrange");
-        c->counts_clear = true;
         swap_all(c);
         c->alpha_advanced = false;
         c->grid_valid = true;
@@ -953,8 +956,8 @@ sphmp_status sphmp_upload_field(sphmp_ctx* c, int32_t field, const void* host, i
             // rebuild the cell starts (and mgridoff) from the uploaded counts
             CK(cudaMemcpyAsync(c->B.ccount, c->B.mgridcnt, sizeof(uint32_t) * (size_t)c->prm.gridtotal,
                                cudaMemcpyDeviceToDevice, c->stream));
-            c->counts_clear = false;
-            launch_cell_starts(dev_params(c), c->B, false, false, c->stream);  // scan only: no scatter / cell sort
+            // scan only: no scatter / cell sort; a list made after it counts the keys again
+            launch_cell_starts(dev_params(c), c->B, false, true, c->stream);
             CHECK_LAUNCH("rebuild cell starts");
             c->grid_valid = true;
         }
@@ -972,8 +975,7 @@ sphmp_status sphmp_upload_field(sphmp_ctx* c, int32_t field, const void* host, i
 sphmp_status sphmp_get_particle_index(sphmp_ctx* c) {
     if (sphmp_status st = need_ctx(c)) return st;
     if (sphmp_status st = refresh_n(c)) return st;
-    if (!c->counts_clear) launch_clear_counts(c->B, c->stream);
-    c->counts_clear = false;
+    launch_clear_counts(c->B, c->stream);
     launch_hash(dev_params(c), c->B, c->cur, false, c->stream);
     CHECK_LAUNCH("GetParticleIndex");
     c->hash_n = c->n;
@@ -990,8 +992,7 @@ sphmp_status sphmp_get_grid_list(sphmp_ctx* c) {
     // the scatter places every slot by its cell key and rank: both must exist for the current count
     if (c->hash_n != c->n)
         return fail(SPHMP_ERR_STATE, "no cell keys for the current %d particles (run GetParticleIndex first)", c->n);
-    if (c->counts_clear) launch_recount(dev_params(c), c->B, c->stream);  // a step's sort has cleared them
-    c->counts_clear = false;
+    launch_recount(dev_params(c), c->B, c->stream);  // where a captured step's sort has cleared the counts
     launch_cell_starts(dev_params(c), c->B, false, false, c->stream);
     launch_cell_order(dev_params(c), c->B, c->stream);
     CHECK_LAUNCH("GetGridList");
@@ -1356,14 +1357,12 @@ sphmp_status sphmp_step(sphmp_ctx* c, int32_t nsteps, int32_t schedule, int32_t 
         if (!c->graph || c->graph_n != key || c->graph_schedule != schedule ||
             memcmp(c->graph_cur, c->cur, sizeof(c->graph_cur)) != 0) {
             drop_graph(c);
-            if (!c->counts_clear) launch_clear_counts(c->B, c->stream);  // before the capture: a captured step leaves them clear
-            c->counts_clear = true;
             cudaStream_t cap = c->stream;
             CK(cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal));
             int saved[kNumFloat4Fields];
             memcpy(saved, c->cur, sizeof(saved));
             sphmp_status st = SPHMP_OK;
-            for (int k = 0; k < per && !st; k++) st = enqueue_step(c, schedule);
+            for (int k = 0; k < per && !st; k++) st = enqueue_step(c, schedule, nullptr, nullptr, false, true);
             cudaGraph_t g = nullptr;
             cudaError_t e = cudaStreamEndCapture(cap, &g);
             if (st) {
@@ -1385,8 +1384,7 @@ sphmp_status sphmp_step(sphmp_ctx* c, int32_t nsteps, int32_t schedule, int32_t 
             c->graph_schedule = schedule;
             memcpy(c->graph_cur, c->cur, sizeof(c->graph_cur));
         }
-        if (!c->counts_clear) launch_clear_counts(c->B, c->stream);
-        c->counts_clear = true;
+        launch_clear_counts(c->B, c->stream);
         for (int t = 0; t + per <= nsteps; t += per) CK(cudaGraphLaunch(c->graph, c->stream));
         if (c->emit_on) c->n_stale = true;
         // the state a step leaves behind (as enqueue_step sets it)
@@ -1594,7 +1592,6 @@ static sphmp_status clone_state(sphmp_ctx* dst, sphmp_ctx* src) {
     dst->oct_built = src->oct_built;
     dst->pos_sorted = src->pos_sorted;
     dst->hash_n = src->hash_n;
-    dst->counts_clear = src->counts_clear;
     dst->list_mode = src->list_mode;
     dst->nbr_valid = dst->ii_valid = false;
     dst->n_stale = false;

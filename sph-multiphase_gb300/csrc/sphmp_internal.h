@@ -130,11 +130,12 @@ struct DevBuffers {
     uint8_t* octk;      // [cap] octant (h-subcell inside the cell) per slot, in-grid slots only
     uint32_t* arank;    // [cap] rank inside the bin (atomic order; exact for out-of-grid)
     uint32_t* sidx;     // [cap] scatter target (pre-sort slots grouped by cell)
-    // One allocation of count_bytes, all zero between a step's sort and the next hash (the
-    // steps' sorts clear what they have read; other calls leave it to a memset before the next hash):
+    // One allocation of count_bytes, all zero before a hash: a memset queued with it, but in the
+    // library's captured steps, whose sorts clear what they have read
     uint32_t* ccount;   // [G + 4] particles per cell
     uint32_t* bsum;     // [G / kScanPer + 2] particles per kScanPer cells (linear order)
     uint32_t* usum;     // [cap / kHashBlock^2 + 2] out-of-grid slots per kHashBlock hash chunks
+    uint32_t* counted;  // [1] 1: ccount and usum hold what the last hash's keys count to, 0: cleared since
     size_t count_bytes;
     uint32_t* cstart;   // [G + 2] exclusive scan of ccount in the cell order; cstart[G] = in-grid count,
                         // cstart[G+1] = n
@@ -227,7 +228,7 @@ void launch_clear_counts(const DevBuffers& B, cudaStream_t s);
 // cell keys, ranks and counts (the counts zero before), control words cleared; with
 // `sums` also the sums of the counts in the linear order
 void launch_hash(const DevParams& P, const DevBuffers& B, const int* cur, bool sums, cudaStream_t s);
-// the counts again from the last hash's keys, after they were cleared
+// the counts again from the last hash's keys, if they have been cleared since (decided on the device)
 void launch_recount(const DevParams& P, const DevBuffers& B, cudaStream_t s);
 // GetGridList in two halves: cell starts (a scan of the counts, whose sums the hash
 // of the same step left with `sums`; with `clear` the counts are zeroed), then the

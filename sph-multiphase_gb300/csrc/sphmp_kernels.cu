@@ -48,6 +48,7 @@ __global__ void __launch_bounds__(kHashBlock) k_hash(const __grid_constant__ Dev
     __shared__ uint32_t wcount[kHashBlock / 32];
     const int i = blockIdx.x * kHashBlock + threadIdx.x;
     if (i < kCtlWords) B.ctl[i] = 0u;
+    if (i == 0) *B.counted = 1u;
     const bool valid = i < active_n(B);
     uint32_t key = kUndef;
     if (valid) {
@@ -122,14 +123,30 @@ __global__ void __launch_bounds__(kHashBlock) k_hash(const __grid_constant__ Dev
     if (und) B.arank[i] = wcount[warp] + __popc(ub & lanemask_lt());
 }
 
-// The counts again from the keys of the last hash, for a GetGridList after a step's
-// sort has cleared them.
+// The counts again from the keys of the last hash, for a GetGridList after they were
+// cleared: by the sort of a captured step, or with counts that the caller uploaded.
+// Whether they were is known on the device alone (steps and calls may be replayed from
+// a caller's graph), so every list queues this, and it usually ends here.
 __global__ void __launch_bounds__(kHashBlock) k_recount(const __grid_constant__ DevParams P,
                                                         const __grid_constant__ DevBuffers B) {
-    const int i = blockIdx.x * kHashBlock + threadIdx.x;
-    if (threadIdx.x == 0 && B.uchunk[blockIdx.x]) atomicAdd(&B.usum[blockIdx.x / kHashBlock], B.uchunk[blockIdx.x]);
-    if (i >= active_n(B) || B.key[i] == kUndef) return;
-    atomicAdd(&B.ccount[B.key[i]], 1u);
+    if (*B.counted) return;
+    const int n = active_n(B);
+    const int chunks = (n + kHashBlock - 1) / kHashBlock;
+    for (int g = blockIdx.x; g * kHashBlock < chunks; g += (int)gridDim.x) {
+        const int k = g * kHashBlock + (int)threadIdx.x;
+        __shared__ uint32_t part[kHashBlock / 32];
+        const uint32_t v = __reduce_add_sync(0xffffffffu, k < chunks ? B.uchunk[k] : 0u);
+        if (lane_id() == 0) part[threadIdx.x >> 5] = v;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            uint32_t t = 0;
+            for (int w = 0; w < kHashBlock / 32; w++) t += part[w];
+            B.usum[g] = t;
+        }
+        __syncthreads();
+    }
+    for (int i = blockIdx.x * kHashBlock + (int)threadIdx.x; i < n; i += (int)gridDim.x * kHashBlock)
+        if (B.key[i] != kUndef) atomicAdd(&B.ccount[B.key[i]], 1u);
 }
 
 // ---------------------------------------------------------------------------
@@ -206,7 +223,7 @@ __global__ void __launch_bounds__(kScanBlock) k_scan_reduce(const __grid_constan
 // the list of cells too large for the warp sort, in one pass: every block adds up
 // the sums of the blocks before it (a few dozen words) and scans its kScanPer
 // counts together with their occupied flags (counts in the low 40 bits, flags
-// above). `clear`: the counts are zeroed for the next hash. Bound by its chain: counts,
+// above). `clear`: the counts are zeroed, for the next hash of captured steps. Bound by its chain: counts,
 // two block scans, the stores, which take 16 bytes a thread and array (7 to 9 us at 11 K
 // to 1.3 M particles; 10 to 13 with 4-byte stores and the counts read behind the first
 // scan; three kernels, one of them a single block over the block sums and the chunks'
@@ -231,6 +248,7 @@ __global__ void __launch_bounds__(kScanBlock) k_scan(const __grid_constant__ Dev
     if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) {
         B.cstart[P.G] = run + (uint32_t)total;
         B.cstart[P.G + 1] = (uint32_t)active_n(B);
+        *B.counted = clear ? 0u : 1u;
     }
     run += (uint32_t)excl;
     const bool four = !P.morton && idx + 3 < P.G;  // this thread's cells as 16-byte words
@@ -1967,7 +1985,7 @@ void launch_hash(const DevParams& P, const DevBuffers& B, const int* cur, bool s
 }
 
 void launch_recount(const DevParams& P, const DevBuffers& B, cudaStream_t s) {
-    if (P.n > 0) k_recount<<<blocks_for(P.n, kHashBlock), kHashBlock, 0, s>>>(P, B);
+    if (P.n > 0) k_recount<<<min(blocks_for(P.n, kHashBlock), 152 * 4), kHashBlock, 0, s>>>(P, B);
 }
 
 void launch_cell_starts(const DevParams& P, const DevBuffers& B, bool sums, bool clear, cudaStream_t s) {

@@ -130,3 +130,113 @@ def test_list_between_density_and_force():
             got.append(_state(ctx))
     assert bits_equal(got[1][abi.F_ACCEL], got[0][abi.F_ACCEL])
     assert np.abs(got[0][abi.F_ACCEL]).max() > 0
+
+
+def _captured(ctx, calls):
+    """`calls` on the context's stream as a caller's own graph; nothing of it has run yet."""
+    torch = pytest.importorskip("torch")
+    stream = torch.cuda.Stream()
+    ctx.set_stream(stream.cuda_stream)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.stream(stream):
+        graph.capture_begin()
+        calls()
+        graph.capture_end()
+
+    def replay():
+        with torch.cuda.stream(stream):
+            graph.replay()
+    return replay
+
+
+@pytest.mark.parametrize("before", ["calls", "step", "replayed steps"])
+@pytest.mark.parametrize("order", [LINEAR, MORTON])
+def test_a_callers_capture_of_the_sort(order, before):
+    """Two sorts captured by the caller and replayed, with the library's own sorts, steps and lists in between: what a
+    replay counts does not depend on what ran before it."""
+    p, d, c = _scene(70000, 0.3, order, 6)
+    c["bornid"] = np.arange(p.num)
+    with sphmp.Context(p) as ctx:
+        ctx.upload_aos(d, c)
+        if before == "calls":
+            ctx.sort()
+        else:
+            ctx.step(2, abi.SCHEDULE_FUSED, use_graph=before != "step")
+        replay = _captured(ctx, lambda: (ctx.sort(), ctx.sort()))
+        for k in range(4):
+            replay()
+            if k:  # the first replays follow one another
+                ctx.sync()
+                key = ctx.download_field(abi.F_MGCELL)  # sorted: the next sort leaves the order
+                _check(ctx, p, key, order)
+                assert np.array_equal(np.sort(ctx.download_field(abi.F_BORNID)), np.arange(p.num))
+            if k == 1:
+                ctx.get_particle_index()
+            elif k == 2:
+                ctx.step(2, abi.SCHEDULE_FUSED)
+        ctx.get_grid_list()
+        _check(ctx, p, key, order)
+        ctx.sync()
+
+
+def test_a_callers_capture_of_a_step():
+    p, d, c = _scene(70000, 0.3, LINEAR, 7)
+    c["bornid"] = np.arange(p.num)
+    fields = (abi.F_BORNID, abi.F_POS, abi.F_VEL, abi.F_ACCEL, abi.F_MGRIDCNT)
+    with sphmp.Context(p) as ctx:
+        ctx.upload_aos(d, c)
+        ctx.step(1, abi.SCHEDULE_FUSED, use_graph=False)
+        replay = _captured(ctx, lambda: ctx.step(1, abi.SCHEDULE_FUSED, use_graph=False))
+        replay()
+        ctx.get_particle_index()
+        replay()
+        ctx.step(2, abi.SCHEDULE_FUSED, use_graph=True)
+        replay()
+        ctx.sync()
+        got = [ctx.download_field(f) for f in fields]
+    with sphmp.Context(p) as ctx:
+        ctx.upload_aos(d, c)
+        ctx.step(6, abi.SCHEDULE_FUSED)
+        ctx.sync()
+        want = [ctx.download_field(f) for f in fields]
+    for f, a, b in zip(fields, got, want):
+        assert bits_equal(a, b), f
+
+
+@pytest.mark.parametrize("order", [LINEAR, MORTON])
+def test_a_callers_capture_of_the_list(order):
+    """The list alone, replayed after steps that have cleared the counts and after ones that have not."""
+    p, d, c = _scene(70000, 0.3, order, 8)
+    with sphmp.Context(p) as ctx:
+        ctx.upload_aos(d, c)
+        ctx.sort()
+        ctx.get_particle_index()
+        replay = _captured(ctx, ctx.get_grid_list)
+        for use_graph in (None, True, False, True, True):
+            if use_graph is not None:
+                ctx.step(1, abi.SCHEDULE_FUSED, use_graph=use_graph)
+                want = _lists(ctx)
+            replay()
+            ctx.sync()
+            if use_graph is not None:
+                got = _lists(ctx)
+                for k in want:
+                    assert np.array_equal(got[k], want[k]), (k, use_graph)
+
+
+def test_list_after_uploaded_counts():
+    """A list is made from the keys, whatever counts the caller has put in."""
+    p, d, c = _scene(70000, 0.3, LINEAR, 9)
+    with sphmp.Context(p) as ctx:
+        ctx.upload_aos(d, c)
+        ctx.get_particle_index()
+        key = ctx.download_field(abi.F_MGCELL)
+        cnt = np.zeros(p.gridtotal, np.int32)
+        cnt[100:200] = 7
+        ctx.upload_field(abi.F_MGRIDCNT, cnt)
+        ctx.get_grid_list()
+        _check(ctx, p, key, LINEAR)
+        ctx.step(1, abi.SCHEDULE_FUSED)
+        ctx.upload_field(abi.F_MGRIDCNT, cnt)
+        ctx.get_grid_list()
+        _check(ctx, p, key, LINEAR)
