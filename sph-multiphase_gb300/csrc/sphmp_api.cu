@@ -1574,7 +1574,8 @@ static sphmp_status clone_state(sphmp_ctx* dst, sphmp_ctx* src) {
     CK(cp(b.osrc, a.osrc, sizeof(uint32_t) * N));
     CK(cp(b.oct_start, a.oct_start, sizeof(uint32_t) * 8 * G));
     CK(cp(b.act, a.act, sizeof(uint32_t) * G));
-    CK(cp(b.ctl, a.ctl, sizeof(uint32_t) * kCtlWords));
+    CK(cudaMemsetAsync(b.ctl, 0, sizeof(uint32_t) * kCtlWords, s));  // no lists, so no queue of heavy particles either
+    CK(cp(b.ctl, a.ctl, sizeof(uint32_t) * kListWords));
     CK(cp(b.wq, a.wq, sizeof(uint2) * (N / kBucketWindowMin + 16)));
     CK(cp(b.nact, a.nact, sizeof(int32_t)));
     CK(cp(b.frame, a.frame, sizeof(int32_t)));

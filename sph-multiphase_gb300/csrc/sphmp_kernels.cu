@@ -2019,6 +2019,7 @@ void launch_boundary_volume(const DevParams& P, const DevBuffers& B, const int* 
 
 void launch_density(const DevParams& P, const DevBuffers& B, const int* cur, cudaStream_t s) {
     if (P.n <= 0) return;
+    cudaMemsetAsync(B.hq_n, 0, sizeof(uint32_t), s);  // its lists queue nobody: what the queue holds is of other lists
     k_density<<<blocks_for(P.n), kThreads, 0, s>>>(P, B, B.f4[POS][cur[POS]], B.f4[ALPHA][cur[ALPHA]]);
 }
 
