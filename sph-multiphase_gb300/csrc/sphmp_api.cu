@@ -154,6 +154,12 @@ float sqrt_cut(float r) {
     return x;
 }
 
+// v as an unevaluated sum of two floats.
+void split(double v, float (&part)[2]) {
+    part[0] = (float)v;
+    part[1] = (float)(v - (double)part[0]);
+}
+
 DevParams dev_params(const sphmp_ctx* c) {
     const sphmp_params& p = c->prm;
     DevParams P;
@@ -175,6 +181,13 @@ DevParams dev_params(const sphmp_ctx* c) {
     P.r2 = p.smoothradius * p.smoothradius;
     P.ih = 1.f / P.h;
     P.ir2 = 1.f / P.r2;
+    {
+        const double r = (double)P.h / (double)P.ss;  // in the positions' units
+        const int e = std::min(std::max(-ilogb(r), -126), 126);
+        P.vol_scale = ldexpf(1.f, e);
+        split(ldexp(r * r, 2 * e), P.vol_r2);
+        split(ldexp((double)p.kpoly6 * pow((double)P.ss, 6.0), -6 * e), P.vol_factor);
+    }
     P.r2list = P.r2 * (1.0f + 1.0e-5f);
     P.list_mode = c->nbr_valid ? c->list_mode : 0;
     P.narrow = c->pos_sorted ? 1 : 0;
@@ -209,11 +222,8 @@ DevParams dev_params(const sphmp_ctx* c) {
     const double h = (double)P.h;
     P.ii_c1 = 2.25 / h;
     P.ii_k = (double)P.kspline / (h * h);
-    P.ii_ih[0] = (float)(1.0 / h);
-    P.ii_ih[1] = (float)(1.0 / h - (double)P.ii_ih[0]);
-    const double idt2 = 1.0 / ((double)P.dt * (double)P.dt);
-    P.ii_idt2[0] = (float)idt2;
-    P.ii_idt2[1] = (float)(idt2 - (double)P.ii_idt2[0]);
+    split(1.0 / h, P.ii_ih);
+    split(1.0 / ((double)P.dt * (double)P.dt), P.ii_idt2);
     P.ii_cut[0] = sqrt_cut(P.h);
     P.ii_cut[1] = sqrt_cut(2.0f * P.h);
     return P;

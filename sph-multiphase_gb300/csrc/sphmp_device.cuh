@@ -38,6 +38,13 @@ struct Kahan {
     }
 };
 
+// s += v, and c += what the rounding of that sum leaves.
+__device__ __forceinline__ void add_exact(float& s, float& c, float v) {
+    const float t = __fadd_rn(s, v), b = __fsub_rn(t, s);
+    c = __fadd_rn(c, __fadd_rn(__fsub_rn(s, __fsub_rn(t, b)), __fsub_rn(v, b)));
+    s = t;
+}
+
 // Grid coordinate in cell units, the reference's (pos - gridmin) * gridIdfac.
 __device__ __forceinline__ float grid_t(float p, float gmin, float fac) { return __fmul_rn(__fsub_rn(p, gmin), fac); }
 // int(t) is only defined inside the int range; outside it (and for NaN) the

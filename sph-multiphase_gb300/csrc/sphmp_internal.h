@@ -85,6 +85,9 @@ struct DevParams {
     float ss;        // simscale
     float h, r2;     // smoothing radius and its square
     float ih, ir2;   // their reciprocals
+    float vol_scale;      // boundary volumes (k_boundary_volume): scale of a difference of positions,
+    float vol_r2[2];      // the squared radius at that scale and the sums' factor, in two parts each
+    float vol_factor[2];
     float r2list;    // squared radius of the neighbour list (r2 plus a rounding margin)
     int list_mode;   // 0: no list, 1: index lists in nbr (written by the last density pass)
     int narrow;      // 1: positions are the ones the cell lists were built from (the cell

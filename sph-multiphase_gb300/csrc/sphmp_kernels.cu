@@ -566,11 +566,16 @@ __global__ void __launch_bounds__(kThreads) k_slot_order(const __grid_constant__
 // Boundary volume (ComputeBoundaryDensity)
 // ---------------------------------------------------------------------------
 
-// kVolumeLanes lanes a particle share its candidate rows. Each lane sums with
-// Kahan compensation and the lanes' sums are added with their compensations, so
-// the result is as exact as the one-thread sum this replaces, which was a serial
-// chain of several hundred loads (58 us at 11 K particles, 122 us at 1.3 M; 13 and
-// 104 us with eight lanes, 17 and 100 us with four).
+// kVolumeLanes lanes a particle share its candidate rows (one thread a particle is a
+// serial chain of several hundred loads: 58 us at 11 K particles, 122 us at 1.3 M). A
+// wall is a lattice, whose particles all round alike, and everything near it inherits
+// their error, of one sign: with terms in plain FP32 the volumes were 7e-8 too small on
+// average, which is what the mean residue of an IISPH solve then showed. So a term
+// (h^2 - r^2)^3 carries its rounding errors (the differences of positions are exact but
+// where a coordinate changes sign) and the volume is exact to a few 1e-9 before it is
+// rounded once. In units in which the radius is 1 to 2 (vol_scale, a power of two). A
+// sum costs 12, 133 and 162 us at 11 K, 1.3 M and 913 K particles; with plain terms 11,
+// 103 and 125.
 constexpr int kVolumeLanes = 8;
 
 __global__ void __launch_bounds__(kThreads) k_boundary_volume(const __grid_constant__ DevParams P,
@@ -586,31 +591,46 @@ __global__ void __launch_bounds__(kThreads) k_boundary_volume(const __grid_const
         if (pi.w < 0.f) cell = B.mgcell[s];
     }
     Kahan sum;
+    float low = 0.f;  // the terms' rounding errors
     if (cell != kUndef)
         for_candidate_rows(P, B, cell, pi.x, pi.y, pi.z, [&](uint32_t j0, uint32_t j1) {
+#pragma unroll 2
             for (uint32_t j = j0 + g; j < j1; j += kVolumeLanes) {
                 const float4 pj = __ldg(&pos4[j]);
-                const float dx = (pi.x - pj.x) * P.ss, dy = (pi.y - pj.y) * P.ss, dz = (pi.z - pj.z) * P.ss;
-                const float dsq = dx * dx + dy * dy + dz * dz;
-                if (pj.w < 0.f && dsq < P.r2) {
-                    const float c = P.r2 - dsq;
-                    sum.add(c * c * c);
+                const float x = (pi.x - pj.x) * P.vol_scale, y = (pi.y - pj.y) * P.vol_scale,
+                            z = (pi.z - pj.z) * P.vol_scale;
+                const float xx = __fmul_rn(x, x), yy = __fmul_rn(y, y), zz = __fmul_rn(z, z);
+                if (pj.w < 0.f && xx + yy + zz < P.vol_r2[0]) {
+                    // c = r2 - xx - yy - zz, each difference of two of which the first is the larger
+                    const float c0 = __fsub_rn(P.vol_r2[0], xx), c1 = __fsub_rn(c0, yy), c = __fsub_rn(c1, zz);
+                    float e = __fsub_rn(__fsub_rn(P.vol_r2[0], c0), xx);
+                    e = __fadd_rn(e, __fsub_rn(__fsub_rn(c0, c1), yy));
+                    e = __fadd_rn(e, __fsub_rn(__fsub_rn(c1, c), zz));
+                    e = __fadd_rn(e, P.vol_r2[1]);
+                    e = __fsub_rn(e, __fmaf_rn(x, x, -xx));
+                    e = __fsub_rn(e, __fmaf_rn(y, y, -yy));
+                    e = __fsub_rn(e, __fmaf_rn(z, z, -zz));
+                    // (c + e)^3 = q c + what the two products and e leave
+                    const float q = __fmul_rn(c, c), w = __fmul_rn(q, c);
+                    low += __fmaf_rn(3.f * e, q, __fmaf_rn(__fmaf_rn(c, c, -q), c, __fmaf_rn(q, c, -w)));
+                    sum.add(w);
                 }
             }
         });
     __syncwarp();
 #pragma unroll
-    for (int o = kVolumeLanes / 2; o > 0; o >>= 1) {  // the pairwise sums, their rounding errors in c
-        const float s2 = __shfl_xor_sync(0xffffffffu, sum.s, o), c2 = __shfl_xor_sync(0xffffffffu, sum.c, o);
-        const float a = __fadd_rn(sum.s, s2), b = __fsub_rn(a, sum.s);
-        const float e = __fadd_rn(__fsub_rn(sum.s, __fsub_rn(a, b)), __fsub_rn(s2, b));
-        sum.c = __fsub_rn(__fadd_rn(sum.c, c2), e);
-        sum.s = a;
+    for (int o = kVolumeLanes / 2; o > 0; o >>= 1) {  // the pairwise sums, their rounding errors in low
+        low = __fadd_rn(low, __shfl_xor_sync(0xffffffffu, low, o));
+        sum.c = __fadd_rn(sum.c, __shfl_xor_sync(0xffffffffu, sum.c, o));
+        add_exact(sum.s, low, __shfl_xor_sync(0xffffffffu, sum.s, o));
     }
     if (cell == kUndef || g != 0) return;
-    float v = __fsub_rn(sum.s, sum.c) * P.kpoly6;
-    if (v == 0.f) v = 1.f;
-    B.vtmp[s] = 1.f / v;
+    // the volume 1 / (sum factor), the sum and the factor in two floats each
+    const float v = sum.s * P.vol_factor[0];
+    const float v0 = fmaf(low - sum.c, P.vol_factor[0], fmaf(sum.s, P.vol_factor[1], fmaf(sum.s, P.vol_factor[0], -v)));
+    const float q = v == 0.f ? 1.f : 1.f / v;
+    const float rest = fmaf(-q, v0, fmaf(-q, v, 1.f));  // 1 - q (v + v0)
+    B.vtmp[s] = fabsf(rest) < 1e-6f ? fmaf(q, rest, q) : q;  // (else nothing was summed, or v is no ordinary float)
 }
 
 __global__ void __launch_bounds__(kThreads) k_boundary_volume_store(const __grid_constant__ DevParams P,
