@@ -222,7 +222,7 @@ DevParams dev_params(const sphmp_ctx* c) {
     const double h = (double)P.h;
     P.ii_c1 = 2.25 / h;
     P.ii_k = (double)P.kspline / (h * h);
-    split(1.0 / h, P.ii_ih);
+    split(1.0 / (h * h), P.ii_ir2);
     split(1.0 / ((double)P.dt * (double)P.dt), P.ii_idt2);
     P.ii_cut[0] = sqrt_cut(P.h);
     P.ii_cut[1] = sqrt_cut(2.0f * P.h);
@@ -307,14 +307,15 @@ sphmp_status alloc_buffers(sphmp_ctx* c) {
     B.dctr = B.ctl + kListWords + 1;
     B.hctr = B.ctl + kListWords + 2;
     // the IISPH arrays in one allocation (creating a context is mostly its allocations)
-    CK(dalloc(&B.iis_dii, 3 * N + (5 * N + 4 + 3) / 4));
+    CK(dalloc(&B.iis_dii, 3 * N + (6 * N + 4 + 3) / 4));
     B.iis_dijpj = B.iis_dii + N;
     B.iis_dsum = B.iis_dii + 2 * N;
     B.iis_aii = reinterpret_cast<float*>(B.iis_dii + 3 * N);
     B.iis_rho_adv = B.iis_aii + N;
     B.iis_pl = B.iis_aii + 2 * N;
     B.iis_pm = B.iis_aii + 3 * N;
-    B.iis_list = reinterpret_cast<uint32_t*>(B.iis_aii + 4 * N);
+    B.iis_rho_lo = B.iis_aii + 4 * N;
+    B.iis_list = reinterpret_cast<uint32_t*>(B.iis_aii + 5 * N);
     B.iis_ctl = B.iis_list + N;
     CK(cudaMemset(B.iis_dii, 0, sizeof(float4) * N));
     CK(cudaMemset(B.iis_dijpj, 0, sizeof(float4) * N));

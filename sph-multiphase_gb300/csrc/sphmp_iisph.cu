@@ -57,7 +57,8 @@ struct NablaH {
         c0 = (float)(c - (double)c1);
         k = P.ii_k;
     }
-    __device__ __forceinline__ float operator()(float r) const { return fmaf(c1, r, fmaf(c0, r, -3.f)); }
+    // (the small part last: added to 3 it would vanish, which put 6e-8 of one sign into a_ii)
+    __device__ __forceinline__ float operator()(float r) const { return fmaf(c0, r, fmaf(c1, r, -3.f)); }
     __device__ __forceinline__ float sum(float v) const { return (float)((double)v * k); }
 };
 
@@ -139,12 +140,41 @@ __device__ __forceinline__ void scan_cells(const DevBuffers& B, const float4* __
     }
 }
 
+// The sums over all lanes of each member's v, with their rounding errors: lane i gets
+// member i's as sum + rest. Halves of the members go to halves of the lanes three times,
+// then the four lanes of a member are added.
+__device__ __forceinline__ void sum_members(float (&v)[kScanMembers], float& sum, float& rest) {
+    static_assert(kScanMembers == 8, "three halvings");
+    const unsigned lane = lane_id();
+    float low[kScanMembers] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int o = 16, k = kScanMembers / 2; o > 0; o >>= 1, k >>= 1) {
+        const bool up = (lane & (unsigned)o) != 0;
+#pragma unroll
+        for (int i = 0; i < (k > 0 ? k : 1); i++) {
+            const float keep = k > 0 && up ? v[i + k] : v[i], keep0 = k > 0 && up ? low[i + k] : low[i];
+            const float give = k > 0 && !up ? v[i + k] : v[i], give0 = k > 0 && !up ? low[i + k] : low[i];
+            v[i] = keep;
+            low[i] = keep0 + __shfl_xor_sync(0xffffffffu, give0, o);
+            add_exact(v[i], low[i], __shfl_xor_sync(0xffffffffu, give, o));
+        }
+    }
+    const int at = (int)((lane & 4u) << 2 | (lane & 2u) << 2 | (lane & 1u) << 2);  // where member `lane` ended up
+    sum = __shfl_sync(0xffffffffu, v[0], at);
+    rest = __shfl_sync(0xffffffffu, low[0], at);
+}
+
 // ComputeDensityIISPH (:1067-1115): rho_i = sum over every candidate of kern(x_ij) m_j,
 // m_j = mass_j (fluid) or restdens_i V_j (boundary); also the lists of the fluid
 // neighbours with 0 < r < h (entries 0, 1, ...) and of the boundary neighbours
 // with 0 < r < 2h (entries kMaxNbr - 1, kMaxNbr - 2, ...), their counts in the low
 // and high halves of nbr_cnt (kIiSearch when both do not fit: the walks then
 // search the cells), and the particles that have them in iis_list (any order).
+// The density is held in two parts (iis_rho_lo: what rounding to densp.x left) and its
+// sums over masses and volumes apart (rest density times volume rounds alike for all of
+// a wall's lattice): the residue of a solve is a mean of differences from the rest
+// density, in which 1e-9 of the density of one sign shows as 1e-7 (33 K particles,
+// ten iterations: 6e-7 off without these, 1e-8 with them).
 // DENSITY false: the lists only. Issue-bound: a candidate costs its distance to
 // every member (two at a time in packed FP32) and, within 2h, about 20
 // instructions; the cut-offs compare squared distances with the smallest ones
@@ -158,7 +188,7 @@ __global__ void __launch_bounds__(kScanThreads) k_ii_density(const __grid_consta
                                                              const float4* __restrict__ pos4,
                                                              const float4* __restrict__ alpha4) {
     __shared__ uint32_t tab[kScanWarps][2][28];
-    __shared__ float2 mem[kScanWarps][kScanMembers / 2][4];  // x, y, z, rest density of two members each
+    __shared__ float2 mem[kScanWarps][kScanMembers / 2][3];  // x, y, z of two members each
     const unsigned lane = lane_id();
     const int w = threadIdx.x >> 5;
     const int s0 = (int)(blockIdx.x * kScanWarps + w) * kScanMembers;
@@ -174,17 +204,16 @@ __global__ void __launch_bounds__(kScanThreads) k_ii_density(const __grid_consta
         m[0] = pm.x;
         m[2] = pm.y;
         m[4] = pm.z;
-        m[6] = mine ? alpha4[s].w : 0.f;
     }
     __syncwarp();
     const float2 SS = make_float2(P.ss, P.ss);
     const float cut_h = P.ii_cut[0], cut_2h = P.ii_cut[1];
-    const float ih = P.ii_ih[0], ih0 = P.ii_ih[1];
-    float acc[kScanMembers];
+    const float ir2 = P.ii_ir2[0], ir20 = P.ii_ir2[1];
+    float2 acc[kScanMembers];  // sums over masses, over boundary volumes
     uint32_t cf[kScanMembers], cb[kScanMembers];
 #pragma unroll
     for (int i = 0; i < kScanMembers; i++) {
-        acc[i] = 0.f;
+        acc[i] = make_float2(0.f, 0.f);
         cf[i] = cb[i] = 0;
     }
     scan_cells(B, pos4, mine, cell, tab[w][0], tab[w][1], [&](uint32_t gc, unsigned) { return gc + (uint32_t)P.neighborid[min(lane, 26u)]; },
@@ -203,7 +232,9 @@ __global__ void __launch_bounds__(kScanThreads) k_ii_density(const __grid_consta
             dy = __fmul2_rn(dy, SS);
             dz = __fmul2_rn(dz, SS);
             const float2 d2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
-            const float2 rho0 = mem[w][p][3];
+            // r^2 / h^2, not 0 for the member itself
+            const float2 qq2 = __ffma2_rn(d2, make_float2(ir2, ir2),
+                                          __ffma2_rn(d2, make_float2(ir20, ir20), make_float2(1e-30f, 1e-30f)));
 #pragma unroll
             for (int h = 0; h < 2; h++) {
                 const int i = 2 * p + h;
@@ -211,12 +242,15 @@ __global__ void __launch_bounds__(kScanThreads) k_ii_density(const __grid_consta
                 const float dsq = h ? d2.y : d2.x;
                 if (!__any_sync(0xffffffffu, dsq < cut_2h)) continue;
                 if (DENSITY) {
-                    // the root to its last bit (one Newton step): the density's mean is a small
-                    // part of the residue's terms, so a bias of 1e-8 would show there
-                    const float rs = rsqrtf(fmaxf(dsq, 1e-30f)), r0 = dsq * rs;
-                    const float r = fmaf(0.5f * rs, fmaf(-r0, r0, dsq), r0);
-                    const float q = fminf(fmaf(r, ih, r * ih0), 2.f);
-                    acc[i] = fmaf(ii_kern(q), fmaf(h ? rho0.y : rho0.x, cv, cm), acc[i]);
+                    // q = r / h to its last bit (a Newton step of the root): the density's mean is a
+                    // small part of the residue's terms, so a bias of 1e-9 shows there. (The root
+                    // after the division by h^2: a root times 1 / h = 80 takes few values between
+                    // two floats, and rounds by -4e-9 on average.)
+                    const float qq = h ? qq2.y : qq2.x;
+                    const float rs = rsqrtf(qq), q0 = qq * rs;
+                    const float q = fminf(fmaf(0.5f * rs, fmaf(-q0, q0, qq), q0), 2.f);
+                    const float k = ii_kern(q);
+                    acc[i] = __ffma2_rn(make_float2(k, k), make_float2(cm, cv), acc[i]);
                 }
                 const bool hit = dsq < cutf && dsq > 0.f;
                 const unsigned b = __ballot_sync(0xffffffffu, hit);
@@ -236,13 +270,30 @@ __global__ void __launch_bounds__(kScanThreads) k_ii_density(const __grid_consta
             }
         }
     });
+    float rho = 0.f, lo = 0.f;
+    if (DENSITY) {
+        float sum, rest, sumb, restb, part[kScanMembers];
 #pragma unroll
-    for (int i = 0; i < kScanMembers; i++) {
-        const float sum = DENSITY ? warp_sum_f(acc[i]) : 0.f;
-        if (lane == (unsigned)i && mine) {
-            if (DENSITY) B.densp[s].x = sum * P.kspline;
+        for (int i = 0; i < kScanMembers; i++) part[i] = acc[i].x;
+        sum_members(part, sum, rest);
+#pragma unroll
+        for (int i = 0; i < kScanMembers; i++) part[i] = acc[i].y;
+        sum_members(part, sumb, restb);
+        // (mass sum + rest density times volume sum) kspline
+        const float r0 = mine ? alpha4[s].w : 0.f, b = r0 * sumb;
+        rest += fmaf(r0, sumb, -b) + r0 * restb;
+        add_exact(sum, rest, b);
+        const float p = sum * P.kspline, e = fmaf(sum, P.kspline, -p) + rest * P.kspline;
+        rho = p + e;
+        lo = (p - rho) + e;
+    }
+#pragma unroll
+    for (int i = 0; i < kScanMembers; i++)
+        if (lane == (unsigned)i && mine)
             B.nbr_cnt[s] = cf[i] + cb[i] <= (uint32_t)kMaxNbr ? cf[i] | (cb[i] << 16) : kIiSearch;
-        }
+    if (mine) {
+        if (DENSITY) B.densp[s].x = rho;
+        B.iis_rho_lo[s] = lo;
     }
     uint32_t at = 0;
     if (lane == 0) at = atomicAdd(&B.iis_ctl[3], (uint32_t)__popc(all));
@@ -394,9 +445,11 @@ __global__ void __launch_bounds__(kThreads) k_ii_aii(const __grid_constant__ Dev
     const float rho = dpi.x, mi = pos4[s].w;
     const float dx = -sx / rho / rho * P.dt * P.dt, dy = -sy / rho / rho * P.dt * P.dt,
                 dz = -sz / rho / rho * P.dt * P.dt;
-    B.iis_dii[s] = make_float4(dx, dy, dz, 0.f);
     B.iis_aii[s] = (dx * sx + dy * sy + dz * sz) - mi / rho / rho * P.dt * P.dt * s2;
-    B.iis_rho_adv[s] = rho + N.sum(change) * P.dt;
+    float radv = rho, rest = 0.f;
+    add_exact(radv, rest, fmaf(N.sum(change), P.dt, B.iis_rho_lo[s]));
+    B.iis_rho_adv[s] = radv;
+    B.iis_dii[s] = make_float4(dx, dy, dz, rest);
     B.iis_pl[s] = 0.5f * dpi.y;
 }
 
@@ -481,8 +534,9 @@ __global__ void __launch_bounds__(kThreads) k_ii_iter(const __grid_constant__ De
             const float4 dii = B.iis_dii[s];
             const float omega = 0.1f, aii = B.iis_aii[s], rho0 = alpha4[s].w, radv = B.iis_rho_adv[s];
             ut = N.sum(ut);
-            const float pl1 = fabsf(aii) < 0.00001f ? pli : (1.f - omega) * pli + omega / aii * (rho0 - radv - ut);
-            rv = -rho0 + (radv + ut + aii * pli);
+            const float off = ((radv - rho0) + dii.w) + ut;  // rho_adv - rho0 before it is rounded to rho's size
+            const float pl1 = fabsf(aii) < 0.00001f ? pli : fmaf(omega, -off / aii - pli, pli);
+            rv = fmaf(aii, pli, off);
             B.iis_pl[s] = pl1;
             B.iis_pm[s] = pl1 * mr;
             auto over_dt2 = [&](float v) { return fmaf(v, P.ii_idt2[0], v * P.ii_idt2[1]); };

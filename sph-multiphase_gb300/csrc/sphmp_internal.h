@@ -110,10 +110,10 @@ struct DevParams {
     int morton;      // 1: cells in Z-order in the sorted arrays (corder), 0: the reference's linear order
     int bwin;        // members per work item of the bucket density pass (8..32)
     uint32_t heavy;  // index lists longer than this are heavy (queued in hq)
-    // IISPH: 2.25 / h, kspline / h^2, 1 / h and 1 / dt^2 in two parts each, and the smallest
+    // IISPH: 2.25 / h, kspline / h^2, 1 / h^2 and 1 / dt^2 in two parts each, and the smallest
     // floats whose square root is not below h and 2h (the cut-offs on squared distances)
     double ii_c1, ii_k;
-    float ii_ih[2], ii_idt2[2];
+    float ii_ir2[2], ii_idt2[2];
     float ii_cut[2];
 };
 
@@ -169,7 +169,8 @@ struct DevBuffers {
     uint32_t* hq_n;     // [1] entries in hq
     uint32_t* hctr;     // [3] work counters over hq of the drift (or force + drift), force (or project-U) and alpha passes
     // IISPH step (sphmp_iisph.cu; one allocation, at iis_dii): d_ii, sum_j d_ij p_j, d_ii p_l + sum_j d_ij p_j (float4,
-    // w unused), a_ii, the predicted density, the pressure iterate p_l, p_l m / rho^2
+    // w unused but for d_ii's: what rho_adv's rounding left), a_ii, the predicted density, the pressure iterate p_l,
+    // p_l m / rho^2, what rounding left of the density
     float4* iis_dii;
     float4* iis_dijpj;
     float4* iis_dsum;
@@ -177,6 +178,7 @@ struct DevBuffers {
     float* iis_rho_adv;
     float* iis_pl;
     float* iis_pm;
+    float* iis_rho_lo;
     uint32_t* iis_ctl;  // [4] finished blocks of the running iteration, 1 when the solve has ended, iterations,
                         // particles in iis_list
     uint32_t* iis_list; // [cap] in-grid fluid particles with IISPH lists (any order)
