@@ -189,6 +189,21 @@ DevParams dev_params(const sphmp_ctx* c) {
         split(ldexp((double)p.kpoly6 * pow((double)P.ss, 6.0), -6 * e), P.vol_factor);
     }
     P.r2list = P.r2 * (1.0f + 1.0e-5f);
+    {
+        // a h^2 for the a in 1 .. 1 + 2^-16 for which it is next to a float (to a few 1e-10)
+        double best = INFINITY;
+        P.dens_a = 1.f;
+        P.dens_r2 = P.r2;
+        for (int k = 0; k < 128; k++) {
+            const float a = 1.f + (float)k * 0x1p-23f;
+            const double ar2 = (double)P.h * (double)P.h * (double)a, off = fabs((double)(float)ar2 - ar2);
+            if (off >= best) continue;
+            best = off;
+            P.dens_a = a;
+            P.dens_r2 = (float)ar2;
+        }
+        split((double)p.kpoly6 / ((double)P.dens_a * P.dens_a * P.dens_a), P.dens_k6);
+    }
     P.list_mode = c->nbr_valid ? c->list_mode : 0;
     P.narrow = c->pos_sorted ? 1 : 0;
     P.dt = p.dt;

@@ -313,7 +313,7 @@ __device__ __forceinline__ float group_sum(float v) {
 // products are taken in double (fluid_system_kern.cu:310) and rounded to float
 // once, as here.
 __device__ __forceinline__ float2 density_result(const DevParams& P, float wsum, float rho0) {
-    float rho = wsum * P.kpoly6;
+    float rho = fmaf(wsum, P.dens_k6[0], wsum * P.dens_k6[1]);
     if (rho == 0.f) rho = 1.f;
     float p;
     if (P.eos == SPHMP_EOS_LINEAR) p = P.eos_k * (rho - rho0);

@@ -85,6 +85,8 @@ struct DevParams {
     float ss;        // simscale
     float h, r2;     // smoothing radius and its square
     float ih, ir2;   // their reciprocals
+    float dens_r2, dens_a;  // density terms (a (h^2 - r^2))^3 m: a h^2, and the a just above 1 that makes it a float
+    float dens_k6[2];       // kpoly6 / a^3 in two parts
     float vol_scale;      // boundary volumes (k_boundary_volume): scale of a difference of positions,
     float vol_r2[2];      // the squared radius at that scale and the sums' factor, in two parts each
     float vol_factor[2];

@@ -673,7 +673,10 @@ __global__ void __launch_bounds__(kThreads) k_boundary_volume_store(const __grid
 // that interleave measured 338 us, but put the lists out of sequence order, which
 // cost the force and alpha passes 27 us of cache misses.) A lane adds at most 16
 // pairs of terms before they go to its Kahan-compensated sum, and the lanes of a
-// member are added pairwise (a scan). Warps take work items from a shared counter
+// member are added pairwise (a scan) with their rounding errors. The difference
+// h^2 - r^2 is formed with a squared radius that is exact as a float (dens_r2: both
+// times a factor just above 1); h^2 itself rounds by up to 6e-8, for all terms
+// alike (densities 8e-8 too large at h = 0.01 and 0.02, -5e-9 so). Warps take work items from a shared counter
 // (their costs differ by orders of magnitude), each its first one without it (12.5
 // instead of 14.3 us at 11 K particles): the first window of every bucket, then the
 // further windows of large buckets, which the cell sort queued in wq, so that no
@@ -801,7 +804,7 @@ __global__ void __launch_bounds__(kDensThreads, 7) k_density_bucket(const __grid
     const uint32_t nb = *B.act_n * 8u;
     const uint32_t nitems = nb + *B.wq_n;  // the first window of every bucket, then the queued windows
     const size_t cap = (size_t)P.cap;
-    const float r2 = P.r2, r2list = P.r2list;
+    const float r2list = P.r2list;
     const float kFar = __int_as_float(0x7f800000);  // +inf: never within range
     const uint32_t nwarps = gridDim.x * (kDensThreads / 32);
     for (uint32_t it = (blockIdx.x * kDensThreads + threadIdx.x) >> 5; it < nitems;
@@ -853,7 +856,7 @@ __global__ void __launch_bounds__(kDensThreads, 7) k_density_bucket(const __grid
                     pz = __shfl_sync(0xffffffffu, pm.z, (int)src);
         rho0 = __shfl_sync(0xffffffffu, rho0, (int)src);
         const float2 PX = make_float2(px, px), PY = make_float2(py, py), PZ = make_float2(pz, pz);
-        const float2 SS = make_float2(P.ss, P.ss), R2 = make_float2(r2, r2), NEG1 = make_float2(-1.f, -1.f);
+        const float2 SS = make_float2(P.ss, P.ss), R2 = make_float2(P.dens_r2, P.dens_r2), NEGA = make_float2(-P.dens_a, -P.dens_a), NEG1 = make_float2(-1.f, -1.f);
         const uint32_t T = bucket_rows(P, B, c, q, lane, W.rows);
         Kahan sum;
         uint32_t count = 0;  // the member's neighbours in the blocks so far
@@ -923,7 +926,7 @@ __global__ void __launch_bounds__(kDensThreads, 7) k_density_bucket(const __grid
                     for (; p < end; p++) {
                         const float4 a = W.pxy[p], b = W.pzw[p];
                         const float2 d2 = dist2(a, b);
-                        float2 cc = __ffma2_rn(d2, NEG1, R2);  // r2 - d2, rounded once
+                        float2 cc = __ffma2_rn(d2, NEGA, R2);  // a (r2 - d2), rounded once
                         cc.x = fmaxf(cc.x, 0.f);               // 0 outside h (and for the padding)
                         cc.y = fmaxf(cc.y, 0.f);
                         const float2 c3 = __fmul2_rn(__fmul2_rn(cc, cc), cc);
@@ -996,11 +999,15 @@ __global__ void __launch_bounds__(kDensThreads, 7) k_density_bucket(const __grid
             count += total;
             __syncwarp();  // before the candidates and rows are rewritten
         }
-        float dens = sum.s - sum.c;  // of this lane and the member's lanes before it
+        float dens = sum.s, low = -sum.c;  // of this lane and the member's lanes before it
         for (uint32_t o = 1; o < L; o <<= 1) {
-            const float v = __shfl_up_sync(0xffffffffu, dens, o);
-            if (share >= o) dens += v;
+            const float v = __shfl_up_sync(0xffffffffu, dens, o), v0 = __shfl_up_sync(0xffffffffu, low, o);
+            if (share >= o) {
+                low += v0;
+                add_exact(dens, low, v);
+            }
         }
+        dens += low;
         const bool own = live && share == L - 1u;  // holds the whole sum
         // lists that overflowed: mask lists, or the cell search where the sequence is too long for them
         const bool over = own && count > (uint32_t)kMaxNbr;
@@ -1043,7 +1050,7 @@ __global__ void __launch_bounds__(kThreads) k_density(const __grid_constant__ De
         const float dx = (pi.x - pj.x) * P.ss, dy = (pi.y - pj.y) * P.ss, dz = (pi.z - pj.z) * P.ss;
         const float dsq = dx * dx + dy * dy + dz * dz;
         if (dsq < P.r2) {
-            const float c = P.r2 - dsq;
+            const float c = fmaxf(fmaf(-P.dens_a, dsq, P.dens_r2), 0.f);
             const float m = pj.w > 0.f ? pj.w : rho0 * (-pj.w);
             sum.add(c * c * c * m);
         }
