@@ -36,6 +36,7 @@ struct sphmp_ctx {
     bool oct_valid = false;       // the internal order is octant-grouped for the current cell list
     bool pos_sorted = false;      // positions unchanged since the cell list was built from them
     int hash_n = -1;              // particle count the cell keys were computed for (-1: none)
+    bool counts_cleared = false;  // the hash's counts may be clear again (B.counted says whether they are)
     int list_mode = 0;            // kind of list the last density pass wrote (DevParams::list_mode)
     int device = 0;
     cudaStream_t own_stream = nullptr;
@@ -426,6 +427,14 @@ inline void swap_all(sphmp_ctx* c) {
     for (int f = 0; f < kNumFloat4Fields; f++) c->cur[f] ^= 1;
 }
 
+// Whether what is queued now runs now, and not whenever a caller replays its own capture.
+bool runs_now(const sphmp_ctx* c) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(c->stream, &st) == cudaSuccess) return st == cudaStreamCaptureStatusNone;
+    cudaGetLastError();
+    return false;
+}
+
 // Density pass: the bucket kernel when the internal order of this sort is
 // octant-grouped, otherwise the cell-search kernel; both write neighbour lists.
 void run_density(sphmp_ctx* c, bool fresh, cudaStream_t s) {
@@ -493,7 +502,10 @@ sphmp_status enqueue_step(sphmp_ctx* c, int schedule, StageTimer* T = nullptr, c
             c->n_stale = true;
             mark("emit");
         }
-        if (!in_graph) launch_clear_counts(c->B, s);
+        if (!in_graph) {
+            launch_clear_counts(c->B, s);
+            if (runs_now(c)) c->counts_cleared = false;
+        }
         launch_hash(P, c->B, c->cur, true, s);
         mark("hash");
         c->hash_n = c->emit_on ? -1 : c->n;  // with an emitter the count is only known on the device
@@ -984,6 +996,7 @@ sphmp_status sphmp_upload_field(sphmp_ctx* c, int32_t field, const void* host, i
                                cudaMemcpyDeviceToDevice, c->stream));
             // scan only: no scatter / cell sort; a list made after it counts the keys again
             launch_cell_starts(dev_params(c), c->B, false, true, c->stream);
+            c->counts_cleared = true;
             CHECK_LAUNCH("rebuild cell starts");
             c->grid_valid = true;
         }
@@ -1002,6 +1015,7 @@ sphmp_status sphmp_get_particle_index(sphmp_ctx* c) {
     if (sphmp_status st = need_ctx(c)) return st;
     if (sphmp_status st = refresh_n(c)) return st;
     launch_clear_counts(c->B, c->stream);
+    if (runs_now(c)) c->counts_cleared = false;
     launch_hash(dev_params(c), c->B, c->cur, false, c->stream);
     CHECK_LAUNCH("GetParticleIndex");
     c->hash_n = c->n;
@@ -1018,7 +1032,9 @@ sphmp_status sphmp_get_grid_list(sphmp_ctx* c) {
     // the scatter places every slot by its cell key and rank: both must exist for the current count
     if (c->hash_n != c->n)
         return fail(SPHMP_ERR_STATE, "no cell keys for the current %d particles (run GetParticleIndex first)", c->n);
-    launch_recount(dev_params(c), c->B, c->stream);  // where a captured step's sort has cleared the counts
+    // the counts are there since the hash unless the library's captured steps or the caller's
+    // counts came between (a replay of the caller's own captures leaves them there)
+    if (c->counts_cleared || !runs_now(c)) launch_recount(dev_params(c), c->B, c->stream);
     launch_cell_starts(dev_params(c), c->B, false, false, c->stream);
     launch_cell_order(dev_params(c), c->B, c->stream);
     CHECK_LAUNCH("GetGridList");
@@ -1411,6 +1427,7 @@ sphmp_status sphmp_step(sphmp_ctx* c, int32_t nsteps, int32_t schedule, int32_t 
             memcpy(c->graph_cur, c->cur, sizeof(c->graph_cur));
         }
         launch_clear_counts(c->B, c->stream);
+        c->counts_cleared = true;
         for (int t = 0; t + per <= nsteps; t += per) CK(cudaGraphLaunch(c->graph, c->stream));
         if (c->emit_on) c->n_stale = true;
         // the state a step leaves behind (as enqueue_step sets it)
@@ -1619,6 +1636,7 @@ static sphmp_status clone_state(sphmp_ctx* dst, sphmp_ctx* src) {
     dst->oct_built = src->oct_built;
     dst->pos_sorted = src->pos_sorted;
     dst->hash_n = src->hash_n;
+    dst->counts_cleared = src->counts_cleared;
     dst->list_mode = src->list_mode;
     dst->nbr_valid = dst->ii_valid = false;
     dst->n_stale = false;

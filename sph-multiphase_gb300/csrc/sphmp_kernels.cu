@@ -125,8 +125,8 @@ __global__ void __launch_bounds__(kHashBlock) k_hash(const __grid_constant__ Dev
 
 // The counts again from the keys of the last hash, for a GetGridList after they were
 // cleared: by the sort of a captured step, or with counts that the caller uploaded.
-// Whether they were is known on the device alone (steps and calls may be replayed from
-// a caller's graph), so every list queues this, and it usually ends here.
+// Whether they were is known on the device alone (a list may be replayed from a caller's
+// graph), so this ends here if not.
 __global__ void __launch_bounds__(kHashBlock) k_recount(const __grid_constant__ DevParams P,
                                                         const __grid_constant__ DevBuffers B) {
     if (*B.counted) return;
