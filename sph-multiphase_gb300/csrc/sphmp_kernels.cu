@@ -664,20 +664,20 @@ __global__ void __launch_bounds__(kThreads) k_boundary_volume_store(const __grid
 // arithmetic, adding its density terms and appending the hits to a
 // list of its own in shared memory. The lanes' lists of a member are then joined
 // and written as rows of four indices. Bound by shared-memory accesses (78 % of
-// the L1 data pipe) and the issue slots (64 %): about 14 instructions a candidate
+// the L1 data pipe) and the issue slots (63 %): about 14 instructions a candidate
 // and lane, none of them across lanes. (The kernel this replaces had the lanes
 // hold the candidates and walked the members, with ballots and selects per 32
 // candidates and a shuffle reduction per member, and left mask words that a
 // second kernel expanded: 174 M warp instructions at 442 K fluid particles
-// against 117 M here; 404 against 350 us at 1.05 M, 33 against 16 us at 4 K. Shares
-// that interleave measured 338 us, but put the lists out of sequence order, which
+// against 126 M here; 404 against 373 us at 1.05 M, 33 against 13 us at 4 K. Shares
+// that interleave take 12 us less, but put the lists out of sequence order, which
 // cost the force and alpha passes 27 us of cache misses.) A lane adds at most 16
 // pairs of terms before they go to its Kahan-compensated sum, and the lanes of a
 // member are added pairwise (a scan) with their rounding errors. The difference
 // h^2 - r^2 is formed with a squared radius that is exact as a float (dens_r2: both
 // times a factor just above 1); h^2 itself rounds by up to 6e-8, for all terms
-// alike (densities 8e-8 too large at h = 0.01 and 0.02, -5e-9 so). Warps take work items from a shared counter
-// (their costs differ by orders of magnitude), each its first one without it (12.5
+// alike (densities 8e-8 too large at h = 0.01 and 0.02, -5e-9 so). Warps take work
+// items from a shared counter (their costs differ by orders of magnitude), each its first one without it (12.5
 // instead of 14.3 us at 11 K particles): the first window of every bucket, then the
 // further windows of large buckets, which the cell sort queued in wq, so that no
 // bucket serialises on one warp. Members whose lists overflow their kMaxNbr

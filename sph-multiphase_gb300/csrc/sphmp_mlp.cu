@@ -844,7 +844,7 @@ __global__ void k_loss_sum(const float* __restrict__ part, int nparts, int batch
 }
 
 
-// FP32 master parameters -> padded bf16 operands (and their transposes) + biases
+// FP32 master parameters -> padded bf16 operands + biases
 __global__ void k_pack(const float* __restrict__ p, PackedMut W) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const float* w1 = p + kOffParamW1;
